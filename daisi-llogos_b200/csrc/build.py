@@ -28,7 +28,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 # library name -> sources (first is the .cu that is compiled; the rest are hashed with it)
 SOURCES: Dict[str, List[str]] = {
     "elementwise": ["elementwise.cu", "common.cuh", "kernel_args.h"],
-    "gemm_simt": ["gemm_simt.cu", "common.cuh"],
+    "gemm_simt": ["gemm_simt.cu", "common.cuh", "kernel_args.h"],
     "gemm_tc": ["gemm_tc.cu", "common.cuh", "kernel_args.h"],
     "attention_simt": ["attention_simt.cu", "common.cuh", "kernel_args.h", "attention_noalloc.h", "attention_reduce.cuh"],
     "attention_mix": ["attention_mix.cu", "common.cuh", "kernel_args.h", "attention_reduce.cuh"],

@@ -7,6 +7,10 @@
 #include "common.cuh"
 #include "kernel_args.h"
 
+#include <cooperative_groups.h>
+
+namespace cg = cooperative_groups;
+
 LLG_API const char* llg_last_error() { return g_llg_error; }
 
 namespace {
@@ -72,6 +76,274 @@ __global__ void __launch_bounds__(256) gemm_tn_kernel(const AT* __restrict__ x, 
   }
 }
 
+// ---- float32 operands with 16-byte rows: two kernels by the count of rows ------------------------------------------
+//
+// Few rows (a decode step): a stream of the weights.  A warp keeps F features x NR rows of sums; its lanes take
+// neighbouring float4s of k, the next group of weights is on its way while this one is used, and the WK warps of a
+// feature group share k.  Bound by the weight stream: a float4 of weights is used for NR products of four, and the rows'
+// float4s come from the first-level cache once per F features, so F x NR = 32 keeps the CUDA cores and that cache below
+// half of what the memory's rate asks of them.  The weights of the first group do not wait for the kernel before.
+template <int NR, int F>
+__global__ void __launch_bounds__(256, 2) gemv_rows_kernel(const float* __restrict__ x, const float* __restrict__ w,
+                                                        float* __restrict__ out, int n, int o, int k, int wk, RowScale scale) {
+  constexpr int NV = NR * F;
+  static_assert(NV == 8 || NV == 16 || NV == 32, "the sums of a warp are spread over its lanes");
+  __shared__ float part[8][NV];
+  pdl_launch_dependents();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int groups = 8 / wk, kp = warp % wk, fg = warp / wk;
+  const int chunks = (n + NR - 1) / NR;                  // row chunks of one feature group are neighbours: its weights stay in L2
+  const int r0 = (blockIdx.x % chunks) * NR;
+  const int f0 = ((blockIdx.x / chunks) * groups + fg) * F;
+  const int k4 = k >> 2;
+  const float4* wp[F];
+#pragma unroll
+  for (int f = 0; f < F; ++f) wp[f] = reinterpret_cast<const float4*>(w + (long long)min(f0 + f, o - 1) * k);
+  float4 wc[F];
+  int c = kp * 32 + lane;
+  const int step = wk * 32;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int f = 0; f < F; ++f) wc[f] = c < k4 ? __ldcs(wp[f] + c) : zero;
+  pdl_wait();                                            // x is the kernel's before, and what that kernel reads may be `out`
+  const float4* xp[NR];
+#pragma unroll
+  for (int r = 0; r < NR; ++r) xp[r] = reinterpret_cast<const float4*>(x + (long long)min(r0 + r, n - 1) * k);
+  float acc[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) acc[i] = 0.f;
+  for (; c < k4; c += step) {
+    float4 wn[F];
+    const int cn = c + step;
+#pragma unroll
+    for (int f = 0; f < F; ++f) wn[f] = cn < k4 ? __ldcs(wp[f] + cn) : zero;
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      const float4 xv = xp[r][c];
+#pragma unroll
+      for (int f = 0; f < F; ++f) {
+        float& a = acc[r * F + f];
+        a = fmaf(xv.x, wc[f].x, a);
+        a = fmaf(xv.y, wc[f].y, a);
+        a = fmaf(xv.z, wc[f].z, a);
+        a = fmaf(xv.w, wc[f].w, a);
+      }
+    }
+#pragma unroll
+    for (int f = 0; f < F; ++f) wc[f] = wn[f];
+  }
+  // the sums of 32 lanes: every exchange halves the values a lane keeps, so that NV - 1 exchanges and log2(32 / NV) more
+  // leave value (lane * NV / 32) in the lane
+#pragma unroll
+  for (int h = NV / 2, off = 16; off > 0; off >>= 1, h >>= 1) {
+    if (h >= 1) {
+      const bool up = (lane & off) != 0;
+#pragma unroll
+      for (int i = 0; i < NV / 2; ++i) {
+        if (i < h) {
+          const float give = up ? acc[i] : acc[i + h];
+          const float keep = up ? acc[i + h] : acc[i];
+          acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+        }
+      }
+    } else {
+      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], off);
+    }
+  }
+  constexpr int LANES_PER = 32 / NV;
+  if (lane % LANES_PER == 0) part[warp][lane / LANES_PER] = acc[0];
+  __syncthreads();
+  const int t = threadIdx.x;
+  if (t < groups * NV) {
+    const int g = t / NV, v = t % NV;
+    float sum = 0.f;
+    for (int q = 0; q < wk; ++q) sum += part[g * wk + q][v];
+    const int r = r0 + v / F, col = ((blockIdx.x / chunks) * groups + g) * F + v % F;
+    if (r < n && col < o) out[(long long)r * o + col] = scale.ss ? sum * row_scale_of(scale, r) : sum;
+  }
+}
+
+// More rows (a prompt step): tiles of 64 rows x 128 features, 128 threads with 8 x 8 sums each, so that a k takes 16
+// values from shared memory for 64 products.  Operands lie k-major in shared memory; column c of k-row kk is kept at
+// c ^ 8 ((kk / 4) % 4), which spreads the transposing stores over the banks without padding.  Bound by the multiply-add
+// pipes.  Where a shape has few tiles, the blocks of a cluster share the tile's k and add their sums through distributed
+// shared memory, in the order of the ranks.
+constexpr int TM = 64, TF = 128, TK = 16;
+
+__device__ __forceinline__ int tile_col(int kk, int c) { return c ^ (((kk >> 2) & 3) << 3); }
+
+__global__ void __launch_bounds__(128, 3) gemm_tile_kernel(const float* __restrict__ x, const float* __restrict__ w,
+                                                           float* __restrict__ out, int n, int o, int k, RowScale scale) {
+  __shared__ __align__(16) float sm[TM * TF];            // two stages of operands (2 x 16 x 192), then the tile's sums
+  static_assert(2 * TK * (TM + TF) <= TM * TF, "the stages fit where the sums go");
+  pdl_launch_dependents();
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), ranks = (int)cluster.num_blocks();
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int n0 = blockIdx.y * TM, o0 = (blockIdx.x / ranks) * TF;
+  const int steps_all = (k + TK - 1) / TK, per = (steps_all + ranks - 1) / ranks;
+  const int s0 = min(rank * per, steps_all), s1 = min(s0 + per, steps_all);
+  const int lr = tid >> 2, lc = tid & 3;                 // copying: 32 rows of 16 k (four float4) at a time
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 px[2], pw[4];
+  auto fetch_w = [&](int s) {
+    const int kk = s * TK + lc * 4;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = o0 + i * 32 + lr;
+      pw[i] = (kk < k && r < o) ? *reinterpret_cast<const float4*>(w + (long long)r * k + kk) : zero;
+    }
+  };
+  auto fetch_x = [&](int s) {
+    const int kk = s * TK + lc * 4;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int r = n0 + i * 32 + lr;
+      px[i] = (kk < k && r < n) ? *reinterpret_cast<const float4*>(x + (long long)r * k + kk) : zero;
+    }
+  };
+  auto put = [&](int b) {
+    float* xs = sm + b * TK * (TM + TF);
+    float* ws = xs + TK * TM;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float v[4] = {px[i].x, px[i].y, px[i].z, px[i].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) xs[(lc * 4 + e) * TM + tile_col(lc * 4, i * 32 + lr)] = v[e];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float v[4] = {pw[i].x, pw[i].y, pw[i].z, pw[i].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) ws[(lc * 4 + e) * TF + tile_col(lc * 4, i * 32 + lr)] = v[e];
+    }
+  };
+  float acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  if (s0 < s1) fetch_w(s0);
+  pdl_wait();
+  if (s0 < s1) {
+    fetch_x(s0);
+    put(0);
+  }
+  __syncthreads();
+  for (int s = s0; s < s1; ++s) {
+    const int b = (s - s0) & 1;
+    if (s + 1 < s1) {
+      fetch_w(s + 1);
+      fetch_x(s + 1);
+    }
+    const float* xs = sm + b * TK * (TM + TF);
+    const float* ws = xs + TK * TM;
+#pragma unroll
+    for (int kk = 0; kk < TK; ++kk) {
+      float a[8], f[8];
+      // rows ty*4.. and 32 + ty*4.., features tx*4.. and 64 + tx*4..
+      *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(xs + kk * TM + tile_col(kk, ty * 4));
+      *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(xs + kk * TM + tile_col(kk, 32 + ty * 4));
+      *reinterpret_cast<float4*>(f) = *reinterpret_cast<const float4*>(ws + kk * TF + tile_col(kk, tx * 4));
+      *reinterpret_cast<float4*>(f + 4) = *reinterpret_cast<const float4*>(ws + kk * TF + tile_col(kk, 64 + tx * 4));
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], f[j], acc[i][j]);
+    }
+    if (s + 1 < s1) put(b ^ 1);
+    __syncthreads();
+  }
+  auto row_of = [&](int i) { return (i >> 2) * 32 + ty * 4 + (i & 3); };
+  if (ranks == 1) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = n0 + row_of(i);
+      if (r >= n) continue;
+      const float rs = scale.ss ? row_scale_of(scale, r) : 1.0f;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int c0 = o0 + h * 64 + tx * 4;
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (c0 + e < o) out[(long long)r * o + c0 + e] = acc[i][4 * h + e] * rs;
+      }
+    }
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      *reinterpret_cast<float4*>(sm + row_of(i) * TF + h * 64 + tx * 4) =
+          make_float4(acc[i][4 * h], acc[i][4 * h + 1], acc[i][4 * h + 2], acc[i][4 * h + 3]);
+  cluster.sync();
+  const int rows = TM / ranks;                           // rows of the tile that this block adds up and stores
+  for (int i = tid; i < rows * (TF / 4); i += 128) {
+    const int row = rank * rows + i / (TF / 4), c = (i % (TF / 4)) * 4;
+    float4 v = zero;
+    for (int q = 0; q < ranks; ++q) {
+      const float4 t = *reinterpret_cast<const float4*>(cluster.map_shared_rank(sm, q) + row * TF + c);
+      v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+    }
+    const int r = n0 + row;
+    if (r < n) {
+      const float rs = scale.ss ? row_scale_of(scale, r) : 1.0f;
+      const float e[4] = {v.x * rs, v.y * rs, v.z * rs, v.w * rs};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (o0 + c + j < o) out[(long long)r * o + o0 + c + j] = e[j];
+    }
+  }
+  cluster.sync();                                        // nobody leaves while its sums may still be read
+}
+
+template <int NR, int F>
+int run_gemv(const float* x, const float* w, float* out, int n, int o, int k, const RowScale& rs, cudaStream_t stream) {
+  // warps that share k: enough for about 32 a multiprocessor, each with a float4 a lane at least
+  int wk = 1;
+  const long long groups = (o + F - 1) / F, want = 32LL * llg_sm_count();
+  while (wk < 8 && groups * ((n + NR - 1) / NR) * wk < want && k / 4 > wk * 32) wk *= 2;
+  const long long per = (long long)F * (8 / wk);
+  const long long blocks = ((o + per - 1) / per) * ((n + NR - 1) / NR);
+  LLG_REQUIRE(blocks <= 2147483647LL, "gemm_simt: too many blocks");
+  cudaError_t e = llg_launch(gemv_rows_kernel<NR, F>, dim3((unsigned)blocks), dim3(256), 0, stream, x, w, out, n, o, k, wk, rs);
+  if (e != cudaSuccess) return llg_fail("gemm_simt: launch: %s", cudaGetErrorString(e));
+  return llg_check_launch("gemm_simt");
+}
+
+int run_tile(const float* x, const float* w, float* out, int n, int o, int k, const RowScale& rs, cudaStream_t stream) {
+  const long long tiles = (long long)((n + TM - 1) / TM) * ((o + TF - 1) / TF), sms = llg_sm_count();
+  const int steps = (k + TK - 1) / TK;
+  // blocks that share a tile's k: the rounds of blocks over the multiprocessors times a block's steps and a fixed cost
+  int ranks = 1;
+  long long best = 0;
+  for (int s = 1; s <= 8; s *= 2) {
+    if (s > 1 && steps < 4 * s) break;
+    const long long cost = ((tiles * s + sms - 1) / sms) * ((steps + s - 1) / s + 8 + (s > 1 ? 4 : 0));
+    if (best == 0 || cost < best) { best = cost; ranks = s; }
+  }
+  const long long gx = (long long)((o + TF - 1) / TF) * ranks;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)gx, (unsigned)((n + TM - 1) / TM));
+  cfg.blockDim = dim3(128);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)ranks;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = llg_pdl_enabled() ? 2 : 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tile_kernel, x, w, out, n, o, k, rs);
+  if (e != cudaSuccess) return llg_fail("gemm_simt: launch: %s", cudaGetErrorString(e));
+  return llg_check_launch("gemm_simt");
+}
+
+constexpr int GEMV_ROWS_MAX = 16;     // rows up to which the weight stream is taken
+
 }  // namespace
 
 // With `scale` (may be null) row r of the result is multiplied by the scale that a norm left for row r of x.
@@ -82,6 +354,15 @@ LLG_API int llg_gemm_simt(const void* x, int x_dtype, const void* w, int w_dtype
   dim3 grid((o + BN - 1) / BN, (n + BM - 1) / BM);
   LLG_REQUIRE(grid.y <= 65535, "gemm_simt: %d rows need more than 65535 row blocks", n);
   const RowScale rs = scale ? *scale : RowScale{nullptr, 0, 0.f, 0.f};
+  if (x_dtype == LLG_F32 && w_dtype == LLG_F32 && out_dtype == LLG_F32 && k % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15u) == 0) {
+    const float *xf = (const float*)x, *wf = (const float*)w;
+    float* of = (float*)out;
+    if (n == 1) return run_gemv<1, 8>(xf, wf, of, n, o, k, rs, stream);
+    if (n == 2) return run_gemv<2, 8>(xf, wf, of, n, o, k, rs, stream);
+    if (n <= 4) return run_gemv<4, 8>(xf, wf, of, n, o, k, rs, stream);
+    if (n <= GEMV_ROWS_MAX) return run_gemv<8, 4>(xf, wf, of, n, o, k, rs, stream);
+    return run_tile(xf, wf, of, n, o, k, rs, stream);
+  }
 #define LAUNCH(AT, WT, CT) \
   gemm_tn_kernel<AT, WT, CT><<<grid, 256, 0, stream>>>((const AT*)x, (const WT*)w, (CT*)out, n, o, k, rs)
   const int key = x_dtype * 4 + w_dtype * 2 + out_dtype;

@@ -97,6 +97,21 @@ def test_gemm_simt(ops, xd, wd, od, n, o, k):
     check(out, P.linear(x, w), od if od == torch.bfloat16 else torch.float32)
 
 
+# float32 rows of 16 bytes: the weight stream up to 16 rows (chunks of 1, 2, 4 or 8 rows; a warp's k with and without a
+# remainder), the tiles of 64 x 128 above, alone and shared by a cluster's 2, 4 and 8 blocks (unequal shares among them)
+@pytest.mark.parametrize("n,o,k", [(1, 5, 4), (2, 33, 132), (3, 64, 1000), (7, 301, 2048), (9, 20, 516), (16, 4100, 260), (17, 129, 4),
+                                   (64, 128, 1036), (65, 257, 4104), (200, 300, 2052), (130, 24000, 64)])
+def test_gemm_simt_float32_rows(ops, n, o, k):
+    x, w = rnd((n, k), 5), rnd((o, k), 6, torch.float32, 1.0 / math.sqrt(k))
+    ss = rnd((n, 3), 7).abs() + 0.5
+    out = torch.full((n + 1, o), 7.0, device=DEV)
+    for scale in (None, ops.RowScale(ss.to(DEV), 96, 1e-3)):
+        ops.gemm_simt(x.to(DEV), w.to(DEV), out[:n], row_scale=scale)
+        want = P.linear(x, w) if scale is None else P.linear(x, w) * _scale_of(ss, 96, 1e-3)[:, None]
+        check(out[:n].cpu(), want, torch.float32, f"gemm_simt scale={scale is not None}")
+        assert torch.equal(out[n].cpu(), torch.full((o,), 7.0))
+
+
 @pytest.mark.parametrize("n,o,k", [(1, 128, 64), (3, 200, 72), (16, 129, 128), (17, 384, 1000), (33, 100, 8),
                                    (70, 130, 336), (129, 65, 16), (300, 1000, 520), (2, 301, 4104),
                                    (1100, 9000, 72), (2050, 4700, 136)])
