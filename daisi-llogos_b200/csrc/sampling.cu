@@ -189,6 +189,61 @@ __device__ unsigned kth_largest_key(int n, int k, KeyFn key, int* is) {
   return lo;
 }
 
+// The same for keys that every thread holds in registers (`fresh(e)`: whether element e takes part): digits of eight bits from the
+// top, a histogram of the digit among the keys that agree with the prefix so far, and one warp that finds the k-th largest's
+// digit in it.  Four passes of three barriers where the bisection above takes thirty-two of two; a slice of 8,192 logits spent
+// 13 of its 21 us in that bisection.  k must not exceed the number of elements that take part.
+struct RadixScratch {
+  int hist[256];
+  unsigned prefix;
+  int k;
+};
+template <int E, typename Part>
+__device__ unsigned kth_largest_radix(const unsigned (&key)[E], Part part, int k, RadixScratch& rs) {
+  const int tid = threadIdx.x;
+  unsigned prefix = 0u;
+#pragma unroll 1
+  for (int shift = 24; shift >= 0; shift -= 8) {
+    if (tid < 256) rs.hist[tid] = 0;
+    __syncthreads();
+    const unsigned above = shift == 24 ? 0u : 0xffffffffu << (shift + 8);
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+      if (part(e) && (key[e] & above) == prefix) atomicAdd(&rs.hist[(key[e] >> shift) & 255u], 1);
+    __syncthreads();
+    if (tid < 32) {
+      // lane l holds digits 255 - 8 l down to 248 - 8 l; `upto`: keys in its digits and all larger ones
+      int c[8], sum = 0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        c[i] = rs.hist[255 - 8 * tid - i];
+        sum += c[i];
+      }
+      int upto = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, upto, o);
+        if (tid >= o) upto += t;
+      }
+      int before = upto - sum;
+      if (before < k && upto >= k) {                    // exactly one lane
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if (before < k && before + c[i] >= k) {
+            rs.prefix = prefix | ((unsigned)(255 - 8 * tid - i) << shift);
+            rs.k = k - before;
+          }
+          before += c[i];
+        }
+      }
+    }
+    __syncthreads();
+    prefix = rs.prefix;
+    k = rs.k;
+  }
+  return prefix;
+}
+
 // New value of token t's logit `v` that occurs `count` times among the recent tokens.
 __device__ __forceinline__ float penalised(const SampleArgs& a, float v, int count) {
   if (a.repetition_penalty != 1.0f) {
@@ -517,70 +572,83 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(SampleArgs a) {
 }
 
 // First stage of the candidate way: block (slice, sequence) keeps SLICE_LEN scaled logits in registers and
-// passes on those that reach its own top_k-th largest, in index order.
-__global__ void __launch_bounds__(THREADS) sample_candidates_kernel(SampleArgs a) {
+// passes on those that reach its own top_k-th largest, in index order.  Bound by latency: a slice is 32 KB, the block's time is
+// the chain of its reads (row -> count -> recent tokens, beside the logits) and its barriers.  Penalised values are exchanged
+// through shared memory by the threads that own a recent token, not looked for by every thread.
+// Eight rows of 128,256 logits, both kernels with top-k 40 and top-p: BEFORE_AFTER.
+__global__ void __launch_bounds__(THREADS, 2) sample_candidates_kernel(SampleArgs a) {
   __shared__ int is[32];
   __shared__ float fs[32];
+  __shared__ RadixScratch radix;
   // without a top-k of its own the slice passes on its 64 largest, and what the second kernel needs of the rest
   const bool wide = !(a.top_k > 0 && a.top_k <= CAND_CAP);
   const int k_eff = wide ? CAND_CAP : a.top_k;
-  __shared__ int pen_tok[HIST_MAX];
-  __shared__ float pen_val[HIST_MAX];
+  __shared__ int hist_s[HIST_MAX];
+  __shared__ __align__(16) float sv[SLICE_LEN];
   const int s = blockIdx.x, b = blockIdx.y, n = a.vocab, tid = threadIdx.x;
+  pdl_launch_dependents();
+  pdl_wait();
   const float* logits = a.logits + (long long)b * n;
-  const int i0 = s * SLICE_LEN + tid * SLICE_PER;
+  const int s0 = s * SLICE_LEN, i0 = s0 + tid * SLICE_PER;
   float v[SLICE_PER];
+  if (i0 + SLICE_PER <= n && ((uintptr_t)(logits + i0) & 15u) == 0) {
 #pragma unroll
-  for (int e = 0; e < SLICE_PER; ++e) v[e] = i0 + e < n ? logits[i0 + e] : -INFINITY;
+    for (int q = 0; q < SLICE_PER / 4; ++q) {
+      const float4 f = *reinterpret_cast<const float4*>(logits + i0 + 4 * q);
+      v[4 * q] = f.x, v[4 * q + 1] = f.y, v[4 * q + 2] = f.z, v[4 * q + 3] = f.w;
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < SLICE_PER; ++e) v[e] = i0 + e < n ? logits[i0 + e] : -INFINITY;
+  }
   const bool penal = a.history && (a.repetition_penalty != 1.0f || a.frequency_penalty != 0.f ||
                                    a.presence_penalty != 0.f);
-  if (penal) {
-    const int hl = min(min(a.history_len[history_row(a, b)], a.history_stride), HIST_MAX);
-    const int* hist = a.history + (long long)history_row(a, b) * a.history_stride;
+  if (penal || a.n_banned > 0) {
+    int hl = 0;
+    if (penal) {
+      const int row = history_row(a, b);
+      hl = min(min(a.history_len[row], a.history_stride), HIST_MAX);
+      const int* hist = a.history + (long long)row * a.history_stride;
+      for (int j = tid; j < hl; j += THREADS) hist_s[j] = hist[j];
+    }
+#pragma unroll
+    for (int q = 0; q < SLICE_PER / 4; ++q)
+      *reinterpret_cast<float4*>(sv + tid * SLICE_PER + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    __syncthreads();
     for (int j = tid; j < hl; j += THREADS) {      // the first occurrence of a token owns it
-      const int t = hist[j];
-      int owner = t;
+      const int t = hist_s[j], d = t - s0;
+      if (t < 0 || t >= n || d < 0 || d >= SLICE_LEN || (!a.penalize_newline && (t == 10 || t == 13))) continue;
+      bool first = true;
       int count = 0;
-      if (t < 0 || t >= n || (!a.penalize_newline && (t == 10 || t == 13))) owner = -1;
+#pragma unroll 8
       for (int q = 0; q < hl; ++q)
-        if (hist[q] == t) {
-          if (q < j) owner = -1;
+        if (hist_s[q] == t) {
+          if (q < j) first = false;
           ++count;
         }
-      pen_tok[j] = owner;
-      pen_val[j] = owner >= 0 ? penalised(a, logits[t], count) : 0.f;
+      if (first) sv[d] = penalised(a, sv[d], count);
     }
     __syncthreads();
-    for (int j = 0; j < hl; ++j) {
-      const int d = pen_tok[j] - i0;
-      if (pen_tok[j] >= 0 && d >= 0 && d < SLICE_PER) {
-#pragma unroll
-        for (int e = 0; e < SLICE_PER; ++e)
-          if (e == d) v[e] = pen_val[j];
-      }
+    for (int j = tid; j < a.n_banned; j += THREADS) {
+      const int d = a.banned[j] - s0;
+      if (d >= 0 && d < SLICE_LEN) sv[d] = -INFINITY;
     }
-  }
-  for (int j = 0; j < a.n_banned; ++j) {
-    const int d = a.banned[j] - i0;
-    if (d >= 0 && d < SLICE_PER) {
+    __syncthreads();
 #pragma unroll
-      for (int e = 0; e < SLICE_PER; ++e)
-        if (e == d) v[e] = -INFINITY;
+    for (int q = 0; q < SLICE_PER / 4; ++q) {
+      const float4 f = *reinterpret_cast<const float4*>(sv + tid * SLICE_PER + 4 * q);
+      v[4 * q] = f.x, v[4 * q + 1] = f.y, v[4 * q + 2] = f.z, v[4 * q + 3] = f.w;
     }
   }
   const float inv_t = 1.0f / a.temperature;
+  unsigned key[SLICE_PER];
 #pragma unroll
-  for (int e = 0; e < SLICE_PER; ++e) v[e] *= inv_t;
-  // the slice's top_k-th largest (bisection over the key bits, counts from registers)
-  unsigned lo = 0u;
-  for (int bit = 31; bit >= 0; --bit) {
-    const unsigned t = lo | (1u << bit);
-    int c = 0;
-#pragma unroll
-    for (int e = 0; e < SLICE_PER; ++e) c += f2key(v[e]) >= t ? 1 : 0;
-    c = block_sum_int(c, is);
-    if (c >= k_eff) lo = t;
+  for (int e = 0; e < SLICE_PER; ++e) {
+    v[e] *= inv_t;
+    key[e] = f2key(v[e]);
   }
+  // the slice's top_k-th largest (entries past the vocabulary are -inf and take part: a slice may have fewer logits than k)
+  const unsigned lo = kth_largest_radix(key, [](int) { return true; }, k_eff, radix);
   const float thr = key2f(lo);
   if (wide) {
     float* w = a.work + (long long)b * n;
@@ -621,6 +689,137 @@ __global__ void __launch_bounds__(THREADS) sample_candidates_kernel(SampleArgs a
   if (tid == 0) a.cand_count[(long long)b * a.n_slices + s] = total;
 }
 
+// Filters and draw over the at most 64 tokens that top-k has left, in index order, by one warp: lane l holds entries 2 l and
+// 2 l + 1.  The same steps as filter_and_draw; the sums are over a handful of entries, so thresholds come from comparing every
+// entry with every other instead of from bisections with a barrier a step.
+__device__ void draw_from_kept(const SampleArgs& a, int b, const float* kept_v, const int* kept_t, int n, int fallback) {
+  const unsigned ALL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int min_keep = a.min_keep > 1 ? a.min_keep : 1;
+  float v[2], w[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) v[e] = 2 * lane + e < n ? kept_v[2 * lane + e] : -INFINITY;
+  const float mx = warp_max(fmaxf(v[0], v[1]));
+  // the k-th largest of x (k entries or more have to be there): the largest entry with k entries no smaller than it
+  auto kth = [&](const float (&x)[2], int k, float none) {
+    int c[2] = {0, 0};
+    for (int j = 0; j < 32; ++j)
+#pragma unroll
+      for (int f = 0; f < 2; ++f) {
+        const float o = __shfl_sync(ALL, x[f], j);
+        if (2 * j + f < n) {
+          c[0] += o >= x[0] ? 1 : 0;
+          c[1] += o >= x[1] ? 1 : 0;
+        }
+      }
+    float best = none;
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      if (2 * lane + e < n && c[e] >= k) best = fmaxf(best, x[e]);
+    return warp_max(best);
+  };
+  float bound = -INFINITY;
+  if (a.min_p > 0.f && a.min_p < 1.0f) {
+    bound = mx + logf(a.min_p);
+    if (min_keep > 1) bound = fminf(bound, kth(v, min(min_keep, n), -INFINITY));
+  }
+  // softmax over the kept tokens
+#pragma unroll
+  for (int e = 0; e < 2; ++e) w[e] = (2 * lane + e < n && v[e] >= bound) ? expf(v[e] - mx) : 0.f;
+  const float inv_z = 1.0f / warp_sum(w[0] + w[1]);
+  w[0] *= inv_z;
+  w[1] *= inv_z;
+  auto renormalise = [&]() {
+    const float s = warp_sum(w[0] + w[1]);
+    if (s > 0.f) {
+      const float r = 1.0f / s;
+      w[0] *= r;
+      w[1] *= r;
+    }
+  };
+  if (a.typical_p > 0.f && a.typical_p < 1.0f) {
+    // the tokens whose surprise is nearest the entropy until their mass reaches typical_p: those with less than typical_p
+    // of mass strictly nearer
+    float ent = 0.f, dev[2], nearer[2] = {0.f, 0.f};
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      if (w[e] > 0.f) ent -= w[e] * logf(w[e]);
+    ent = warp_sum(ent);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) dev[e] = w[e] > 0.f ? fabsf(-logf(w[e]) - ent) : INFINITY;
+    int rank[2] = {0, 0};
+    for (int j = 0; j < 32; ++j)
+#pragma unroll
+      for (int f = 0; f < 2; ++f) {
+        const float od = __shfl_sync(ALL, dev[f], j), ow = __shfl_sync(ALL, w[f], j);
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          if (od < dev[e]) {
+            nearer[e] += ow;
+            ++rank[e];
+          }
+      }
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      if (!(nearer[e] < a.typical_p || (min_keep > 1 && rank[e] < min_keep))) w[e] = 0.f;
+    renormalise();
+  }
+  if (a.top_p > 0.f && a.top_p < 1.0f) {
+    // the smallest set of most probable tokens whose mass exceeds top_p: down to the largest probability at which the
+    // tokens no less probable have more than that (all of them, where none does)
+    float mass[2] = {0.f, 0.f};
+    for (int j = 0; j < 32; ++j)
+#pragma unroll
+      for (int f = 0; f < 2; ++f) {
+        const float o = __shfl_sync(ALL, w[f], j);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) mass[e] += o >= w[e] ? o : 0.f;
+      }
+    float thr = 0.f;
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      if (mass[e] > a.top_p) thr = fmaxf(thr, w[e]);
+    thr = warp_max(thr);
+    if (min_keep > 1) thr = fminf(thr, kth(w, min(min_keep, n), 0.f));
+    if (!(w[0] >= thr)) w[0] = 0.f;
+    if (!(w[1] >= thr)) w[1] = 0.f;
+    renormalise();
+  }
+  if (a.probs_out) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      if (2 * lane + e < n) a.probs_out[(long long)b * a.vocab + kept_t[2 * lane + e]] = w[e];
+  }
+  // draw: the first entry whose cumulative probability exceeds u * total
+  const int seq = a.seq_ids ? a.seq_ids[b] : b;
+  const float u = uniform_of(a.seed, seq, a.step);
+  const float pair = w[0] + w[1];
+  float incl = pair;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float t = __shfl_up_sync(ALL, incl, o);
+    if (lane >= o) incl += t;
+  }
+  const float target = u * __shfl_sync(ALL, incl, 31), before = incl - pair;
+  int pick = 0x7fffffff;
+  if (target >= before && target < incl) {
+    if (w[0] > 0.f && target < before + w[0]) pick = 2 * lane;
+    else if (w[1] > 0.f) pick = 2 * lane + 1;
+    else if (w[0] > 0.f) pick = 2 * lane;           // rounding left the target past the lane's last kept token
+  }
+  pick = __reduce_min_sync(ALL, pick);
+  if (pick == 0x7fffffff) {
+    // rounding left the target past everything: the most probable token, the smallest among ties
+    const float top = warp_max(fmaxf(w[0], w[1]));
+    pick = __reduce_min_sync(ALL, w[0] == top ? 2 * lane : w[1] == top ? 2 * lane + 1 : 0x7fffffff);
+  }
+  if (lane == 0) {
+    const int token = pick < n ? kept_t[pick] : fallback;       // NaN everywhere (an infinite logit): the first candidate
+    a.out[b] = token;
+    history_push(a, b, token);
+  }
+}
+
 // Second stage: the candidates of sequence b, gathered in index order, go through the filters and the draw.
 __global__ void __launch_bounds__(THREADS) sample_from_candidates_kernel(SampleArgs a) {
   __shared__ float fs[32];
@@ -631,17 +830,35 @@ __global__ void __launch_bounds__(THREADS) sample_from_candidates_kernel(SampleA
   __shared__ int cidx[MAX_SLICES * CAND_CAP];
   __shared__ int offs[MAX_SLICES + 1];
   __shared__ int overflow;
+  __shared__ RadixScratch radix;
+  __shared__ float kept_v[CAND_CAP];
+  __shared__ int kept_t[CAND_CAP];
   const int b = blockIdx.x, tid = threadIdx.x, ns = a.n_slices;
-  if (tid == 0) {
-    int o = 0, ov = 0;
-    for (int s = 0; s < ns; ++s) {
-      const int c = a.cand_count[(long long)b * ns + s];
-      if (c > CAND_CAP) ov = 1;
-      offs[s] = o;
-      o += min(c, CAND_CAP);
+  pdl_launch_dependents();
+  pdl_wait();
+  if (tid < 32) {
+    // offsets of the slices' candidates: two slices a lane (MAX_SLICES of them at most)
+    static_assert(MAX_SLICES == 64, "two slices a lane");
+    int c[2], ov = 0;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int sl = 2 * tid + e;
+      c[e] = sl < ns ? a.cand_count[(long long)b * ns + sl] : 0;
+      ov |= c[e] > CAND_CAP ? 1 : 0;
+      c[e] = min(c[e], CAND_CAP);
     }
-    offs[ns] = o;
-    overflow = ov;
+    int incl = c[0] + c[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (tid >= o) incl += t;
+    }
+    const int excl = incl - c[0] - c[1];
+    if (2 * tid < ns) offs[2 * tid] = excl;
+    if (2 * tid + 1 < ns) offs[2 * tid + 1] = excl + c[0];
+    if (tid == 31) offs[ns] = incl;
+    ov = __any_sync(0xffffffffu, ov);
+    if (tid == 0) overflow = ov;
   }
   __syncthreads();
   if (overflow) {                                  // uniform over the block
@@ -657,14 +874,57 @@ __global__ void __launch_bounds__(THREADS) sample_from_candidates_kernel(SampleA
     }
   }
   __syncthreads();
+  const bool wide = !(a.top_k > 0 && a.top_k <= CAND_CAP);
+  if (!wide) {
+    // at most 64 tokens stay: found by the block, in index order, and one warp does the rest
+    int n_kept = n_c;
+    if (a.top_k < n_c) {
+      // the candidates are spread over the threads in runs, so that a scan over the threads is a scan in index order
+      constexpr int PER = MAX_SLICES * CAND_CAP / THREADS;
+      const int per = (n_c + THREADS - 1) / THREADS, c0 = tid * per;
+      unsigned key[PER];
+#pragma unroll
+      for (int e = 0; e < PER; ++e) key[e] = (e < per && c0 + e < n_c) ? f2key(cw[c0 + e]) : 0u;
+      auto part = [&](int e) { return e < per && c0 + e < n_c; };
+      const unsigned kth = kth_largest_radix(key, part, a.top_k, radix);
+      // Exactly top_k stay: of the logits equal to the k-th largest, those with the smallest tokens, as the reference's
+      // selection keeps the first it meets (Sampler.cs:249-276); larger ones in the upper, equal ones in the lower half
+      int mine = 0;
+#pragma unroll
+      for (int e = 0; e < PER; ++e)
+        if (part(e)) mine += key[e] > kth ? 0x10000 : key[e] == kth ? 1 : 0;
+      int total;
+      const int before = block_exclusive_scan_int(mine, is, &total);
+      const int places = a.top_k - (total >> 16);
+      int larger = before >> 16, equal = before & 0xffff;
+#pragma unroll
+      for (int e = 0; e < PER; ++e) {
+        if (!part(e)) continue;
+        const bool eq = key[e] == kth;
+        if (key[e] > kth || (eq && equal < places)) {
+          const int at = larger + min(equal, places);
+          kept_v[at] = cw[c0 + e];
+          kept_t[at] = cidx[c0 + e];
+        }
+        larger += key[e] > kth ? 1 : 0;
+        equal += eq ? 1 : 0;
+      }
+      n_kept = a.top_k;
+    } else {
+      for (int i = tid; i < n_c; i += THREADS) {
+        kept_v[i] = cw[i];
+        kept_t[i] = cidx[i];
+      }
+    }
+    if (a.probs_out)
+      for (int i = tid; i < a.vocab; i += THREADS) a.probs_out[(long long)b * a.vocab + i] = 0.f;
+    __syncthreads();
+    if (tid < 32) draw_from_kept(a, b, kept_v, kept_t, n_kept, n_c > 0 ? cidx[0] : 0);
+    return;
+  }
   float mx = -INFINITY;
   for (int i = tid; i < n_c; i += THREADS) mx = fmaxf(mx, cw[i]);
   mx = block_max(mx, fs);
-  const bool wide = !(a.top_k > 0 && a.top_k <= CAND_CAP);
-  if (!wide) {
-    filter_and_draw(a, b, cw, n_c, cidx, mx, fs, is, &chosen, scan);
-    return;
-  }
 
   // ---- no top-k: the candidates are the 64 largest of every slice, the slices' sums give the whole row's ----
   __shared__ float smass[MAX_SLICES];       // a slice's sum of exp(v - mx)
@@ -799,9 +1059,9 @@ LLG_API int llg_sample(const SampleArgs* args, cudaStream_t stream) {
                     8LL * a.n_seqs * slices <= 18LL * llg_sm_count();        // two resident blocks per multiprocessor, and a few more
   const bool by_candidates = scratch && (narrow || wide);
   if (by_candidates) {
-    sample_candidates_kernel<<<dim3(slices, a.n_seqs), THREADS, 0, stream>>>(a);
-    if (llg_check_launch("sample (candidates)")) return 1;
-    sample_from_candidates_kernel<<<a.n_seqs, THREADS, 0, stream>>>(a);
+    cudaError_t e = llg_launch(sample_candidates_kernel, dim3(slices, a.n_seqs), dim3(THREADS), 0, stream, a);
+    if (e == cudaSuccess) e = llg_launch(sample_from_candidates_kernel, dim3(a.n_seqs), dim3(THREADS), 0, stream, a);
+    if (e != cudaSuccess) return llg_fail("sample (candidates): launch: %s", cudaGetErrorString(e));
   } else {
     sample_kernel<<<a.n_seqs, THREADS, 0, stream>>>(a);
   }

@@ -828,6 +828,27 @@ def test_sampler_by_candidates_equals_the_general_way(ops, case):
         assert int(res[0][0][i]) == P.draw(res[0][1][i].double(), P.uniform_of(13, int(seq_ids[i]), 2))
 
 
+@pytest.mark.parametrize("case", [dict(top_k=40), dict(top_k=64, top_p=0.6), dict(top_k=2, min_keep=2, min_p=0.9), dict(top_k=50, typical_p=0.4, min_keep=9),
+                                  dict(top_k=64, top_p=0.01, min_keep=3), dict(top_k=63, top_p=0.999, min_p=1e-4, typical_p=0.95)])
+@pytest.mark.parametrize("vocab", [65, 8193, 30001])
+def test_sampler_top_k_ties_between_slices(ops, vocab, case):
+    """Equal logits at the k-th place that are spread over the slices (the smallest tokens stay), few tokens left by -inf
+    (fewer than k), and the filters behind top-k: against the general way."""
+    b = 3
+    logits = rnd((b, vocab), 75, scale=2.0)
+    logits[0, ::max(1, vocab // 60)] = 9.0    # about 60 equal logits above the rest
+    logits[1, 11:] = -math.inf                # eleven tokens left
+    res = []
+    for cand in (True, False):
+        work, out = torch.empty(b * vocab, device=DEV), torch.empty(b, dtype=torch.int32, device=DEV)
+        probs = torch.full((b, vocab), float("nan"), device=DEV)
+        ops.sample(logits.to(DEV), work, out, seed=17, step=4, probs_out=probs, candidates=cand, temperature=0.9, **case)
+        res.append((out.cpu(), probs.cpu()))
+    assert torch.equal(res[0][0], res[1][0])
+    assert ((res[0][1] > 0) == (res[1][1] > 0)).all()
+    assert float((res[0][1] - res[1][1]).abs().max()) < 1e-6
+
+
 @pytest.mark.parametrize("case", [dict(temperature=0.7), dict(temperature=1.3, repetition_penalty=1.2, banned=[5, 9000, 20010]),
                                   dict(temperature=0.8, top_p=0.9), dict(temperature=1.0, top_p=0.5, frequency_penalty=0.4),
                                   dict(temperature=0.9, min_p=0.05), dict(temperature=1.1, min_p=0.01, top_p=0.8),
