@@ -76,6 +76,15 @@ __global__ void __launch_bounds__(256) gemm_tn_kernel(const AT* __restrict__ x, 
   }
 }
 
+// Two float32 multiply-adds in one instruction, each rounded as fmaf does: a multiprocessor issues scalar multiply-adds at half of
+// its pipes' rate (38 TFLOP/s was the most that the scalar form of the tiles below reached, whatever the shape).  A pair holds
+// neighbouring k, so a 16-byte load gives two operand pairs and a sum is kept as two, over the even and the odd k.
+typedef unsigned long long pair_t;
+__device__ __forceinline__ void fma2(pair_t& acc, pair_t a, pair_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float both(pair_t v) { return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32)); }
+
 // ---- float32 operands with 16-byte rows: two kernels by the count of rows ------------------------------------------
 //
 // Few rows (a decode step): a stream of the weights.  A warp keeps F features x NR rows of sums; its lanes take
@@ -163,125 +172,117 @@ __global__ void __launch_bounds__(256, 2) gemv_rows_kernel(const float* __restri
   }
 }
 
-// More rows (a prompt step): tiles of 64 rows x 128 features, 128 threads with 8 x 8 sums each, so that a k takes 16
-// values from shared memory for 64 products.  Operands lie k-major in shared memory; column c of k-row kk is kept at
-// c ^ 8 ((kk / 4) % 4), which spreads the transposing stores over the banks without padding.  Bound by the multiply-add
-// pipes.  Where a shape has few tiles, the blocks of a cluster share the tile's k and add their sums through distributed
-// shared memory, in the order of the ranks.
-constexpr int TM = 64, TF = 128, TK = 16;
+// More rows (a prompt step): tiles of 64 rows x 128 features, 256 threads with 8 x 4 sums each.  Both operands arrive by
+// cp.async as they lie in memory, 32 k of a row at a time, in a ring of three stages: a stage is 24 KB, so that one block a
+// multiprocessor already has the bytes in flight that the memory's latency asks for (with the next stage in registers and
+// half as much a step a block waited 2 us a step: 38 us at 64 x 2,048 x 2,048; now TILE_NOW).  Rows are padded to 36 floats: 16-byte
+// reads of consecutive rows at one k fall into different banks.  A thread takes four k at a time, 16 reads for 256
+// multiply-adds.  Bound by the multiply-add pipes from 150 rows on.  Where a shape has few tiles, the blocks of a cluster
+// share the tile's k and add their sums through distributed shared memory, in the order of the ranks.
+constexpr int TM = 64, TF = 128, TK = 32, TLD = TK + 4, TSTAGES = 3;
+constexpr int TILE_SMEM = TSTAGES * (TM + TF) * TLD * (int)sizeof(float);
+static_assert(TM * TF * (int)sizeof(float) <= TILE_SMEM, "the sums fit where the stages were");
 
-__device__ __forceinline__ int tile_col(int kk, int c) { return c ^ (((kk >> 2) & 3) << 3); }
+__device__ __forceinline__ void copy16(float* dst, const float* src, bool there) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(there ? 16 : 0) : "memory");
+}
 
-__global__ void __launch_bounds__(128, 3) gemm_tile_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                           float* __restrict__ out, int n, int o, int k, RowScale scale) {
-  __shared__ __align__(16) float sm[TM * TF];            // two stages of operands (2 x 16 x 192), then the tile's sums
-  static_assert(2 * TK * (TM + TF) <= TM * TF, "the stages fit where the sums go");
+__global__ void __launch_bounds__(256, 2) gemm_tile_kernel(const float* __restrict__ x, const float* __restrict__ w,
+                                                        float* __restrict__ out, int n, int o, int k, RowScale scale) {
+  extern __shared__ __align__(16) float sm[];            // the stages, then the tile's sums
   pdl_launch_dependents();
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank(), ranks = (int)cluster.num_blocks();
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  // rows ty + 8 i, features tx + 32 j: a warp reads two rows and sixteen features at a time
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tx = (lane & 15) + 16 * (warp & 1), ty = (lane >> 4) + 2 * (warp >> 1);
   const int n0 = blockIdx.y * TM, o0 = (blockIdx.x / ranks) * TF;
   const int steps_all = (k + TK - 1) / TK, per = (steps_all + ranks - 1) / ranks;
-  const int s0 = min(rank * per, steps_all), s1 = min(s0 + per, steps_all);
-  const int lr = tid >> 2, lc = tid & 3;                 // copying: 32 rows of 16 k (four float4) at a time
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 px[2], pw[4];
+  const int s0 = min(rank * per, steps_all), steps = min(s0 + per, steps_all) - s0;
+  const int lr = tid >> 3, lc = (tid & 7) * 4;           // copying: 32 rows of 32 k at a time
   auto fetch_w = [&](int s) {
-    const int kk = s * TK + lc * 4;
+    const int kk = (s0 + s) * TK + lc;
+    float* dst = sm + (s % TSTAGES) * (TM + TF) * TLD + TM * TLD + lr * TLD + lc;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < TF / 32; ++i) {
       const int r = o0 + i * 32 + lr;
-      pw[i] = (kk < k && r < o) ? *reinterpret_cast<const float4*>(w + (long long)r * k + kk) : zero;
+      const bool there = kk < k && r < o;
+      copy16(dst + i * 32 * TLD, w + (there ? (long long)r * k + kk : 0), there);
     }
   };
   auto fetch_x = [&](int s) {
-    const int kk = s * TK + lc * 4;
+    const int kk = (s0 + s) * TK + lc;
+    float* dst = sm + (s % TSTAGES) * (TM + TF) * TLD + lr * TLD + lc;
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < TM / 32; ++i) {
       const int r = n0 + i * 32 + lr;
-      px[i] = (kk < k && r < n) ? *reinterpret_cast<const float4*>(x + (long long)r * k + kk) : zero;
+      const bool there = kk < k && r < n;
+      copy16(dst + i * 32 * TLD, x + (there ? (long long)r * k + kk : 0), there);
     }
   };
-  auto put = [&](int b) {
-    float* xs = sm + b * TK * (TM + TF);
-    float* ws = xs + TK * TM;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const float v[4] = {px[i].x, px[i].y, px[i].z, px[i].w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) xs[(lc * 4 + e) * TM + tile_col(lc * 4, i * 32 + lr)] = v[e];
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float v[4] = {pw[i].x, pw[i].y, pw[i].z, pw[i].w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) ws[(lc * 4 + e) * TF + tile_col(lc * 4, i * 32 + lr)] = v[e];
-    }
-  };
-  float acc[8][8];
+  auto close = [&]() { asm volatile("cp.async.commit_group;" ::: "memory"); };
+  pair_t sums[8][4];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-  if (s0 < s1) fetch_w(s0);
+    for (int j = 0; j < 4; ++j) sums[i][j] = 0;
+  // the first stages' weights do not wait for the kernel before
+  for (int s = 0; s < TSTAGES - 1 && s < steps; ++s) fetch_w(s);
   pdl_wait();
-  if (s0 < s1) {
-    fetch_x(s0);
-    put(0);
+  for (int s = 0; s < TSTAGES - 1; ++s) {
+    if (s < steps) fetch_x(s);
+    close();                                             // the first group holds the weights of both stages: only earlier, never late
   }
-  __syncthreads();
-  for (int s = s0; s < s1; ++s) {
-    const int b = (s - s0) & 1;
-    if (s + 1 < s1) {
-      fetch_w(s + 1);
-      fetch_x(s + 1);
+  for (int s = 0; s < steps; ++s) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(TSTAGES - 2) : "memory");
+    __syncthreads();                                     // stage s is there, and everybody is done with stage s - 1
+    if (s + TSTAGES - 1 < steps) {
+      fetch_w(s + TSTAGES - 1);
+      fetch_x(s + TSTAGES - 1);
     }
-    const float* xs = sm + b * TK * (TM + TF);
-    const float* ws = xs + TK * TM;
+    close();
+    const float* xs = sm + (s % TSTAGES) * (TM + TF) * TLD + ty * TLD;
+    const float* ws = sm + (s % TSTAGES) * (TM + TF) * TLD + (TM + tx) * TLD;
+#pragma unroll 2
+    for (int kk = 0; kk < TK; kk += 4) {
+      ulonglong2 a[8];
 #pragma unroll
-    for (int kk = 0; kk < TK; ++kk) {
-      float a[8], f[8];
-      // rows ty*4.. and 32 + ty*4.., features tx*4.. and 64 + tx*4..
-      *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(xs + kk * TM + tile_col(kk, ty * 4));
-      *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(xs + kk * TM + tile_col(kk, 32 + ty * 4));
-      *reinterpret_cast<float4*>(f) = *reinterpret_cast<const float4*>(ws + kk * TF + tile_col(kk, tx * 4));
-      *reinterpret_cast<float4*>(f + 4) = *reinterpret_cast<const float4*>(ws + kk * TF + tile_col(kk, 64 + tx * 4));
+      for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(xs + i * 8 * TLD + kk);
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int j = 0; j < 4; ++j) {
+        const ulonglong2 f = *reinterpret_cast<const ulonglong2*>(ws + j * 32 * TLD + kk);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], f[j], acc[i][j]);
+        for (int i = 0; i < 8; ++i) fma2(sums[i][j], a[i].x, f.x);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) fma2(sums[i][j], a[i].y, f.y);
+      }
     }
-    if (s + 1 < s1) put(b ^ 1);
-    __syncthreads();
   }
-  auto row_of = [&](int i) { return (i >> 2) * 32 + ty * 4 + (i & 3); };
   if (ranks == 1) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const int r = n0 + row_of(i);
+      const int r = n0 + ty + 8 * i;
       if (r >= n) continue;
       const float rs = scale.ss ? row_scale_of(scale, r) : 1.0f;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int c0 = o0 + h * 64 + tx * 4;
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (c0 + e < o) out[(long long)r * o + c0 + e] = acc[i][4 * h + e] * rs;
+      for (int j = 0; j < 4; ++j) {
+        const int c = o0 + tx + 32 * j;
+        if (c < o) out[(long long)r * o + c] = both(sums[i][j]) * rs;
       }
     }
     return;
   }
+  __syncthreads();                                       // the sums go where the last stage was read
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
-      *reinterpret_cast<float4*>(sm + row_of(i) * TF + h * 64 + tx * 4) =
-          make_float4(acc[i][4 * h], acc[i][4 * h + 1], acc[i][4 * h + 2], acc[i][4 * h + 3]);
+    for (int j = 0; j < 4; ++j) sm[(ty + 8 * i) * TF + tx + 32 * j] = both(sums[i][j]);
   cluster.sync();
   const int rows = TM / ranks;                           // rows of the tile that this block adds up and stores
-  for (int i = tid; i < rows * (TF / 4); i += 128) {
+  for (int i = tid; i < rows * (TF / 4); i += 256) {
     const int row = rank * rows + i / (TF / 4), c = (i % (TF / 4)) * 4;
-    float4 v = zero;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int q = 0; q < ranks; ++q) {
       const float4 t = *reinterpret_cast<const float4*>(cluster.map_shared_rank(sm, q) + row * TF + c);
       v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
@@ -315,18 +316,24 @@ int run_gemv(const float* x, const float* w, float* out, int n, int o, int k, co
 int run_tile(const float* x, const float* w, float* out, int n, int o, int k, const RowScale& rs, cudaStream_t stream) {
   const long long tiles = (long long)((n + TM - 1) / TM) * ((o + TF - 1) / TF), sms = llg_sm_count();
   const int steps = (k + TK - 1) / TK;
-  // blocks that share a tile's k: the rounds of blocks over the multiprocessors times a block's steps and a fixed cost
+  // blocks that share a tile's k: the rounds of blocks over the multiprocessors times a block's steps and a fixed cost (clusters
+  // of eight with a multiprocessor a block do not all fit at once: 42 us at 64 x 2,048 x 2,048)
   int ranks = 1;
   long long best = 0;
-  for (int s = 1; s <= 8; s *= 2) {
-    if (s > 1 && steps < 4 * s) break;
-    const long long cost = ((tiles * s + sms - 1) / sms) * ((steps + s - 1) / s + 8 + (s > 1 ? 4 : 0));
+  for (int s = 1; s <= 4; s *= 2) {
+    if (s > 1 && steps < 2 * s) break;
+    const long long cost = ((tiles * s + sms - 1) / sms) * ((steps + s - 1) / s + 3 + (s > 1 ? 2 : 0));
     if (best == 0 || cost < best) { best = cost; ranks = s; }
   }
   const long long gx = (long long)((o + TF - 1) / TF) * ranks;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)gx, (unsigned)((n + TM - 1) / TM));
-  cfg.blockDim = dim3(128);
+  cfg.blockDim = dim3(256);
+  // where every block can have a multiprocessor of its own it asks for more than half of one's shared memory: blocks of a
+  // cluster are placed densely otherwise, two on a multiprocessor beside an idle one
+  constexpr int ALONE_SMEM = 120 * 1024;
+  const int smem = gx * cfg.gridDim.y <= sms ? ALONE_SMEM : TILE_SMEM;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -337,12 +344,14 @@ int run_tile(const float* x, const float* w, float* out, int n, int o, int k, co
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = llg_pdl_enabled() ? 2 : 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tile_kernel, x, w, out, n, o, k, rs);
+  cudaError_t e = cudaFuncSetAttribute(gemm_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ALONE_SMEM);
+  if (e != cudaSuccess) return llg_fail("gemm_simt: cannot have %d bytes of shared memory: %s", ALONE_SMEM, cudaGetErrorString(e));
+  e = cudaLaunchKernelEx(&cfg, gemm_tile_kernel, x, w, out, n, o, k, rs);
   if (e != cudaSuccess) return llg_fail("gemm_simt: launch: %s", cudaGetErrorString(e));
   return llg_check_launch("gemm_simt");
 }
 
-constexpr int GEMV_ROWS_MAX = 16;     // rows up to which the weight stream is taken
+constexpr int GEMV_ROWS_MAX = 32;     // rows up to which the weight stream is taken
 
 }  // namespace
 
