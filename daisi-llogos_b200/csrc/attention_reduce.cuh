@@ -10,10 +10,13 @@ __global__ void attn_decode_reduce_kernel(const float* __restrict__ part_o, cons
                                           float sink_score, const float* __restrict__ gate,
                                           const float* __restrict__ sinks) {
   // (hd: elements of a value head)
+  pdl_launch_dependents();
+  pdl_wait();
   const int h = blockIdx.x, b = blockIdx.y;
   if (sinks) sink_score = sinks[h];
   const long long base = ((long long)b * nh + h) * n_splits;
   float M = -INFINITY;
+#pragma unroll 8
   for (int s = 0; s < n_splits; ++s) M = fmaxf(M, part_ml[(base + s) * 2]);
   if (has_sink) M = fmaxf(M, sink_score);
   float L = has_sink ? expf(sink_score - M) : 0.f;
