@@ -97,6 +97,21 @@ def test_gemm_simt(ops, xd, wd, od, n, o, k):
     check(out, P.linear(x, w), od if od == torch.bfloat16 else torch.float32)
 
 
+@pytest.mark.parametrize("hidden", [4, 1024, 1028, 2048, 3000, 4096, 5120, 6144, 6148, 8192, 8196])
+@pytest.mark.parametrize("dtype", DTYPES, ids=IDS)
+def test_add_rmsnorm_of_many_rows(ops, dtype, hidden):
+    """More than 256 rows with one sum to add, none, and a bias beside it; rows of one to eight float4 a thread and longer ones."""
+    n, eps = 260, 1e-5
+    w, res, branch, bias = rnd((hidden,), 3, dtype).abs() + 0.5, rnd((n, hidden), 4), rnd((1, n, hidden), 5), rnd((hidden,), 6)
+    for b, bb in ((None, None), (branch, None), (branch, bias)):
+        total = res.double() + (0 if b is None else b[0].double()) + (0 if bb is None else bb.double())
+        kw = {} if bb is None else {"branch_bias": bb.to(DEV)}
+        r, out = res.to(DEV).clone(), torch.empty(n, hidden, dtype=dtype, device=DEV)
+        ops.add_rmsnorm(r, None if b is None else b.to(DEV), w.to(DEV), eps, out, **kw)
+        check(r, total, torch.float32, "residual")
+        check(out, P.rms_norm(total, w, eps), dtype, "normed")
+
+
 # float32 rows of 16 bytes: the weight stream up to 16 rows (chunks of 1, 2, 4 or 8 rows; a warp's k with and without a
 # remainder), the tiles of 64 x 128 above, alone and shared by a cluster's 2, 4 and 8 blocks (unequal shares among them)
 @pytest.mark.parametrize("n,o,k", [(1, 5, 4), (2, 33, 132), (3, 64, 1000), (7, 301, 2048), (9, 20, 516), (16, 4100, 260), (17, 129, 4),
