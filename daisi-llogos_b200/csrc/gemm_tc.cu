@@ -181,6 +181,155 @@ __device__ __forceinline__ float vec_elem(const void* p, int dtype, int i) {
   return dtype == LLG_BF16 ? __bfloat162float(((const __nv_bfloat16*)p)[i]) : ((const float*)p)[i];
 }
 
+// The epilogue of 128 token rows, called by four warps: `acc` is where the accumulator's columns start for the warp's lanes, the
+// lane holds token `tok` (which may lie past the last one), n0 is the first feature of the tile.  EPI as at the kernel below.
+template <int TN, typename OT, int EPI>
+__device__ __forceinline__ void token_rows_epilogue(const GemmParams& p, uint32_t acc, int tok, int n0, int split) {
+  if (EPI >= 2) {
+    // lanes are tokens, columns are the features of whole heads: norm, bias, rotation, and the writes of q, k, v
+    constexpr int HD = EPI == 2 ? 128 : 64, HALF = HD / 2;
+    const QkPrepArgs& a = p.prep;
+    const int heads = a.nh + 2 * a.nkv;
+    typedef __nv_bfloat16 bf;
+    const bool live = tok < p.o;
+    const int pos = live ? a.positions[tok] : 0;
+    const int slot = (live && a.k_pages) ? a.slots[a.seq_of_token[tok]] : 0;
+    const float rs = live ? row_scale_of(a.row_scale, tok) : 1.0f;
+#pragma unroll 1
+    for (int hb = 0; hb < TN / HD; ++hb) {
+      const int head = n0 / HD + hb;
+      if (head >= heads) break;                   // uniform: the tile's tail lies past the last head
+      float h[HD];
+#pragma unroll
+      for (int c0 = 0; c0 < HD; c0 += 16) {
+        uint32_t r[16];
+        tmem_ld16(acc + (uint32_t)(hb * HD + c0), r);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int c = 0; c < 16; ++c) h[c0 + c] = __uint_as_float(r[c]) * rs;
+      }
+      const int kind = head < a.nh ? 0 : (head < a.nh + a.nkv ? 1 : 2);      // query, key, value
+      const void* nw = kind == 0 ? a.q_norm_w : (kind == 1 ? a.k_norm_w : nullptr);
+      if (nw) {
+        float ss = 0.f;
+#pragma unroll
+        for (int d = 0; d < HD; ++d) ss += h[d] * h[d];
+        const float inv = 1.0f / sqrtf(ss / (float)HD + a.norm_eps);
+#pragma unroll
+        for (int d = 0; d < HD; ++d) h[d] = h[d] * inv * vec_elem(nw, a.norm_w_dtype, d);
+      }
+      if (a.bias) {
+#pragma unroll
+        for (int d = 0; d < HD; ++d) h[d] += vec_elem(a.bias, a.bias_dtype, head * HD + d);
+      }
+      if (kind != 2 && a.cos_table) {
+        const int pp = pos < a.table_positions ? pos : a.table_positions - 1;     // bounded; the host checks capacity
+        const float4* cs = reinterpret_cast<const float4*>(a.cos_table + (long long)pp * HALF);
+        const float4* sn = reinterpret_cast<const float4*>(a.sin_table + (long long)pp * HALF);
+#pragma unroll
+        for (int i4 = 0; i4 < HALF / 4; ++i4) {
+          const float4 c = cs[i4], sgn = sn[i4];
+          const float cc[4] = {c.x, c.y, c.z, c.w}, sv[4] = {sgn.x, sgn.y, sgn.z, sgn.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int i = 4 * i4 + e;
+            const float u = h[i], v = h[i + HALF];
+            h[i] = u * cc[e] - v * sv[e];
+            h[i + HALF] = u * sv[e] + v * cc[e];
+          }
+        }
+      }
+      if (kind == 0 && a.q_scale) {
+        const float qs = a.q_scale[pos < a.q_scale_positions ? pos : a.q_scale_positions - 1];
+#pragma unroll
+        for (int d = 0; d < HD; ++d) h[d] *= qs;
+      }
+      if (live) {
+        auto store_head = [&](bf* dst) {
+#pragma unroll
+          for (int q8 = 0; q8 < HD / 8; ++q8) {
+            __nv_bfloat162 h0 = __floats2bfloat162_rn(h[8 * q8], h[8 * q8 + 1]), h1 = __floats2bfloat162_rn(h[8 * q8 + 2], h[8 * q8 + 3]);
+            __nv_bfloat162 h2 = __floats2bfloat162_rn(h[8 * q8 + 4], h[8 * q8 + 5]), h3 = __floats2bfloat162_rn(h[8 * q8 + 6], h[8 * q8 + 7]);
+            uint4 u;
+            u.x = *reinterpret_cast<uint32_t*>(&h0);
+            u.y = *reinterpret_cast<uint32_t*>(&h1);
+            u.z = *reinterpret_cast<uint32_t*>(&h2);
+            u.w = *reinterpret_cast<uint32_t*>(&h3);
+            *reinterpret_cast<uint4*>(dst + 8 * q8) = u;
+          }
+        };
+        if (kind == 0) {
+          store_head((bf*)a.q_out + ((long long)tok * a.nh + head) * HD);
+        } else {
+          const int kvh = kind == 1 ? head - a.nh : head - a.nh - a.nkv;
+          bf* packed = (bf*)(kind == 1 ? a.k_new : a.v_new);
+          if (packed) store_head(packed + ((long long)tok * a.nkv + kvh) * HD);
+          bf* pages = (bf*)(kind == 1 ? a.k_pages : a.v_pages);
+          if (pages) store_head(pages + kv_row(a.page_table, a.table_width, a.ring_pages, slot, pos, kvh, a.nkv) * HD);
+        }
+      }
+    }
+  } else {
+    // lanes are tokens (p.o of them), columns are features (p.n, or a gate half and an up half of the tile)
+    const GateForm gate = p.gate;
+    constexpr int VEC = 16 / (int)sizeof(OT);      // outputs per 16-byte store
+    const int width = EPI == 1 ? p.gated_features : p.n;
+    const bool vec_ok = width % VEC == 0;
+    OT* out = (OT*)p.out + (long long)split * p.n * p.o;
+    const float rs = tok >= p.o ? 1.0f : (EPI == 1 && p.row_weight) ? p.row_weight[tok] : row_scale_of(p.scale, tok);
+    OT* row = out + (long long)tok * width;
+    constexpr int COLS = EPI == 1 ? TN / 2 : TN;
+#pragma unroll
+    for (int c0 = 0; c0 < COLS; c0 += 16) {
+      const int f0 = EPI == 1 ? n0 / 2 + c0 : n0 + c0;      // first feature of this run (a gated tile: TN / 2 features)
+      if (f0 >= width) break;
+      float v[16];
+      uint32_t r[16];
+      tmem_ld16(acc + (uint32_t)c0, r);
+      if (EPI == 1) {
+        uint32_t ru[16];
+        tmem_ld16(acc + (uint32_t)(TN / 2 + c0), ru);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          const float g = __uint_as_float(r[c]) * rs;
+          v[c] = gate_act(gate, g, __uint_as_float(ru[c]) * rs);
+        }
+      } else {
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int c = 0; c < 16; ++c) v[c] = __uint_as_float(r[c]) * rs;
+        if (EPI == -1) act16(p.act - 1, v);
+      }
+      if (tok < p.o) {
+        if (vec_ok && f0 + 16 <= width) {
+          if (sizeof(OT) == 4) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              *reinterpret_cast<float4*>((float*)row + f0 + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+          } else {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              __nv_bfloat162 h0 = __floats2bfloat162_rn(v[8 * q], v[8 * q + 1]), h1 = __floats2bfloat162_rn(v[8 * q + 2], v[8 * q + 3]);
+              __nv_bfloat162 h2 = __floats2bfloat162_rn(v[8 * q + 4], v[8 * q + 5]), h3 = __floats2bfloat162_rn(v[8 * q + 6], v[8 * q + 7]);
+              uint4 u;
+              u.x = *reinterpret_cast<uint32_t*>(&h0);
+              u.y = *reinterpret_cast<uint32_t*>(&h1);
+              u.z = *reinterpret_cast<uint32_t*>(&h2);
+              u.w = *reinterpret_cast<uint32_t*>(&h3);
+              *reinterpret_cast<uint4*>((__nv_bfloat16*)row + f0 + 8 * q) = u;
+            }
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < 16; ++c)
+            if (f0 + c < width) row[f0 + c] = from_f32<OT>(v[c]);
+        }
+      }
+    }
+  }
+}
+
 // MT: weight tiles of 128 rows per block (1 or 2; two tiles share every activation tile, which halves
 // the shared-memory traffic per flop of a large product).  EPI 1 (MT = 2): the first tile holds gate
 // rows and the second the up rows of the same features; the block writes silu(gate) * up.  A block
@@ -445,156 +594,11 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tc_kernel(const __grid_cons
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       {
         const uint32_t lane_base = tmem_d + (uint32_t)(b * ACC_COLS) + ((uint32_t)(warp * 32) << 16);
-        if (SWAP && EPI >= 2) {
-          // lanes are tokens, columns are the features of whole heads: norm, bias, rotation, and the writes of q, k, v
-          constexpr int HD = EPI == 2 ? 128 : 64, HALF = HD / 2;
-          const QkPrepArgs& a = p.prep;
-          const int heads = a.nh + 2 * a.nkv;
-          typedef __nv_bfloat16 bf;
-  #pragma unroll 1
+        if (SWAP) {
+#pragma unroll 1
           for (int mt = 0; mt < MT; ++mt) {
             if (o0 + mt * BM >= p.o) break;
-            const int tok = o0 + mt * BM + warp * 32 + lane;
-            const bool live = tok < p.o;
-            const int pos = live ? a.positions[tok] : 0;
-            const int slot = (live && a.k_pages) ? a.slots[a.seq_of_token[tok]] : 0;
-            const float rs = live ? row_scale_of(a.row_scale, tok) : 1.0f;
-  #pragma unroll 1
-            for (int hb = 0; hb < TN / HD; ++hb) {
-              const int head = n0 / HD + hb;
-              if (head >= heads) break;                   // uniform: the tile's tail lies past the last head
-              float h[HD];
-  #pragma unroll
-              for (int c0 = 0; c0 < HD; c0 += 16) {
-                uint32_t r[16];
-                tmem_ld16(lane_base + (uint32_t)(mt * TN + hb * HD + c0), r);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-  #pragma unroll
-                for (int c = 0; c < 16; ++c) h[c0 + c] = __uint_as_float(r[c]) * rs;
-              }
-              const int kind = head < a.nh ? 0 : (head < a.nh + a.nkv ? 1 : 2);      // query, key, value
-              const void* nw = kind == 0 ? a.q_norm_w : (kind == 1 ? a.k_norm_w : nullptr);
-              if (nw) {
-                float ss = 0.f;
-  #pragma unroll
-                for (int d = 0; d < HD; ++d) ss += h[d] * h[d];
-                const float inv = 1.0f / sqrtf(ss / (float)HD + a.norm_eps);
-  #pragma unroll
-                for (int d = 0; d < HD; ++d) h[d] = h[d] * inv * vec_elem(nw, a.norm_w_dtype, d);
-              }
-              if (a.bias) {
-  #pragma unroll
-                for (int d = 0; d < HD; ++d) h[d] += vec_elem(a.bias, a.bias_dtype, head * HD + d);
-              }
-              if (kind != 2 && a.cos_table) {
-                const int pp = pos < a.table_positions ? pos : a.table_positions - 1;     // bounded; the host checks capacity
-                const float4* cs = reinterpret_cast<const float4*>(a.cos_table + (long long)pp * HALF);
-                const float4* sn = reinterpret_cast<const float4*>(a.sin_table + (long long)pp * HALF);
-  #pragma unroll
-                for (int i4 = 0; i4 < HALF / 4; ++i4) {
-                  const float4 c = cs[i4], sgn = sn[i4];
-                  const float cc[4] = {c.x, c.y, c.z, c.w}, sv[4] = {sgn.x, sgn.y, sgn.z, sgn.w};
-  #pragma unroll
-                  for (int e = 0; e < 4; ++e) {
-                    const int i = 4 * i4 + e;
-                    const float u = h[i], v = h[i + HALF];
-                    h[i] = u * cc[e] - v * sv[e];
-                    h[i + HALF] = u * sv[e] + v * cc[e];
-                  }
-                }
-              }
-              if (kind == 0 && a.q_scale) {
-                const float qs = a.q_scale[pos < a.q_scale_positions ? pos : a.q_scale_positions - 1];
-  #pragma unroll
-                for (int d = 0; d < HD; ++d) h[d] *= qs;
-              }
-              if (live) {
-                auto store_head = [&](bf* dst) {
-  #pragma unroll
-                  for (int q8 = 0; q8 < HD / 8; ++q8) {
-                    __nv_bfloat162 h0 = __floats2bfloat162_rn(h[8 * q8], h[8 * q8 + 1]), h1 = __floats2bfloat162_rn(h[8 * q8 + 2], h[8 * q8 + 3]);
-                    __nv_bfloat162 h2 = __floats2bfloat162_rn(h[8 * q8 + 4], h[8 * q8 + 5]), h3 = __floats2bfloat162_rn(h[8 * q8 + 6], h[8 * q8 + 7]);
-                    uint4 u;
-                    u.x = *reinterpret_cast<uint32_t*>(&h0);
-                    u.y = *reinterpret_cast<uint32_t*>(&h1);
-                    u.z = *reinterpret_cast<uint32_t*>(&h2);
-                    u.w = *reinterpret_cast<uint32_t*>(&h3);
-                    *reinterpret_cast<uint4*>(dst + 8 * q8) = u;
-                  }
-                };
-                if (kind == 0) {
-                  store_head((bf*)a.q_out + ((long long)tok * a.nh + head) * HD);
-                } else {
-                  const int kvh = kind == 1 ? head - a.nh : head - a.nh - a.nkv;
-                  bf* packed = (bf*)(kind == 1 ? a.k_new : a.v_new);
-                  if (packed) store_head(packed + ((long long)tok * a.nkv + kvh) * HD);
-                  bf* pages = (bf*)(kind == 1 ? a.k_pages : a.v_pages);
-                  if (pages) store_head(pages + kv_row(a.page_table, a.table_width, a.ring_pages, slot, pos, kvh, a.nkv) * HD);
-                }
-              }
-            }
-          }
-        } else if (SWAP) {
-          // lanes are tokens (p.o of them), columns are features (p.n, or gate|up blocks of 128 + 128)
-          constexpr int VEC = 16 / (int)sizeof(OT);      // outputs per 16-byte store
-          const int width = EPI == 1 ? p.gated_features : p.n;
-          const bool vec_ok = width % VEC == 0;
-          OT* out = (OT*)p.out + (long long)split * p.n * p.o;
-  #pragma unroll
-          for (int mt = 0; mt < MT; ++mt) {
-            if (o0 + mt * BM >= p.o) break;
-            const int tok = o0 + mt * BM + warp * 32 + lane;
-            const float rs = tok >= p.o ? 1.0f : (EPI == 1 && p.row_weight) ? p.row_weight[tok] : row_scale_of(p.scale, tok);
-            OT* row = out + (long long)tok * width;
-            constexpr int COLS = EPI == 1 ? TN / 2 : TN;
-  #pragma unroll
-            for (int c0 = 0; c0 < COLS; c0 += 16) {
-              const int f0 = EPI == 1 ? n0 / 2 + c0 : n0 + c0;      // first feature of this run (a gated tile: TN / 2 features)
-              if (f0 >= width) break;
-              float v[16];
-              uint32_t r[16];
-              tmem_ld16(lane_base + (uint32_t)(mt * TN + c0), r);
-              if (EPI == 1) {
-                uint32_t ru[16];
-                tmem_ld16(lane_base + (uint32_t)(mt * TN + TN / 2 + c0), ru);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-  #pragma unroll
-                for (int c = 0; c < 16; ++c) {
-                  const float g = __uint_as_float(r[c]) * rs;
-                  v[c] = gate_act(gate, g, __uint_as_float(ru[c]) * rs);
-                }
-              } else {
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-  #pragma unroll
-                for (int c = 0; c < 16; ++c) v[c] = __uint_as_float(r[c]) * rs;
-                if (EPI == -1) act16(p.act - 1, v);
-              }
-              if (tok < p.o) {
-                if (vec_ok && f0 + 16 <= width) {
-                  if (sizeof(OT) == 4) {
-  #pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                      *reinterpret_cast<float4*>((float*)row + f0 + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-                  } else {
-  #pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                      __nv_bfloat162 h0 = __floats2bfloat162_rn(v[8 * q], v[8 * q + 1]), h1 = __floats2bfloat162_rn(v[8 * q + 2], v[8 * q + 3]);
-                      __nv_bfloat162 h2 = __floats2bfloat162_rn(v[8 * q + 4], v[8 * q + 5]), h3 = __floats2bfloat162_rn(v[8 * q + 6], v[8 * q + 7]);
-                      uint4 u;
-                      u.x = *reinterpret_cast<uint32_t*>(&h0);
-                      u.y = *reinterpret_cast<uint32_t*>(&h1);
-                      u.z = *reinterpret_cast<uint32_t*>(&h2);
-                      u.w = *reinterpret_cast<uint32_t*>(&h3);
-                      *reinterpret_cast<uint4*>((__nv_bfloat16*)row + f0 + 8 * q) = u;
-                    }
-                  }
-                } else {
-  #pragma unroll
-                  for (int c = 0; c < 16; ++c)
-                    if (f0 + c < width) row[f0 + c] = from_f32<OT>(v[c]);
-                }
-              }
-            }
+            token_rows_epilogue<TN, OT, EPI>(p, lane_base + (uint32_t)(mt * TN), o0 + mt * BM + warp * 32 + lane, n0, split);
           }
         } else if (EPI <= 0) {
           // Up to 64 columns of the accumulator are asked for before their arrival is waited for: one trip to tensor
@@ -686,6 +690,220 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tc_kernel(const __grid_cons
 }
 
 
+// ---- pairs of blocks: large products ---------------------------------------------------------
+//
+// Two blocks of a cluster, on the two multiprocessors of a pair, share one tile of 256 tokens x TN features: each brings its 128
+// token rows and half of the feature rows (of a gated tile: one the gate rows, the other the up rows of the same TN / 2
+// features), and tcgen05.mma.cta_group::2, issued by the first block, reads both halves.  A multiprocessor's shared memory then
+// feeds 128 x TN products from 128 + TN / 2 rows instead of 128 + TN, its stage is 32 KB instead of 48 (six stages instead of
+// four), and the accumulator is TN columns a block, so that there are two and the read-out of one tile runs beside the
+// products of the next (two token tiles in one block leave no room for a second accumulator).  26,624 tokens, back to back under
+// the power cap: gated 27,648 x 5,120 8.5 -> 7.8 ms, the q/k/v product 2.81 -> 2.25 ms.
+//
+// Tiles are walked in bands of PAIR_BAND token tiles, feature tiles inside a band: the blocks that run at one time work on about
+// PAIR_BAND token tiles and as many feature tiles, and a band's activations stay in L2 while all weights pass by (walking all
+// token tiles first reads the activations from memory about once per feature tile where they exceed L2).
+//
+// Copies of both blocks arrive on the first block's barriers; a stage's release and an accumulator's completion are committed
+// to both blocks; the second block's read-out warps report to the first block's barrier.  Waits are bounded as above.
+constexpr int PAIR_STAGES = 6, PAIR_BAND = 8;
+constexpr double PAIR_UNIT = 0.8;
+
+__device__ __forceinline__ void tma_load_pair(uint32_t smem_dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  // the barrier's address with the block bit cleared: the same barrier in the pair's first block
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+      ::"r"(smem_dst), "l"(map), "r"(x), "r"(y), "r"(bar & 0xFEFFFFFFu)
+      : "memory");
+}
+__device__ __forceinline__ void umma_pair_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma_pair_commit(uint64_t* bar) {      // arrives on this barrier of both blocks
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(smem_u32(bar)), "h"((uint16_t)3)
+               : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_first(uint64_t* bar) {      // arrives on the first block's barrier
+  asm volatile(
+      "{\n\t.reg .b32 remote;\n\t"
+      "mapa.shared::cluster.u32 remote, %0, 0;\n\t"
+      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [remote];\n\t}"
+      ::"r"(smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int TN, typename OT, int EPI>
+__global__ void __launch_bounds__(GEMM_THREADS) gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x,
+                                                                 const __grid_constant__ CUtensorMap map_w, GemmParams p) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  constexpr int A_BYTES = BM * BK * 2, B_BYTES = TN / 2 * BK * 2;
+  constexpr int STAGE = BM * BK * 2 + 128 * BK * 2;       // stages start at multiples of 1,024 bytes whatever the width
+  constexpr int ACC_COLS = 256, NACC = 2;
+  static_assert(TN % 32 == 0 && TN <= 256, "features come in steps of 32 for a pair, an accumulator takes half of tensor memory");
+  static_assert(EPI < 2 || TN % 128 == 0, "the q/k/v epilogue works on whole heads");
+  unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  __shared__ uint64_t full_bar[PAIR_STAGES], empty_bar[PAIR_STAGES], acc_full[NACC], acc_empty[NACC];
+  __shared__ uint32_t tmem_base_slot;
+  __shared__ int abort_flag;
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  uint32_t rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  // tokens are p.o, features p.n (rows of w; of a gated product both halves)
+  const int m_tiles = (p.o + 2 * BM - 1) / (2 * BM), n_tiles = (EPI == 1 ? (p.gated_features + TN / 2 - 1) / (TN / 2) : (p.n + TN - 1) / TN);
+  const int total = m_tiles * n_tiles, nkb = (p.k + BK - 1) / BK;
+  auto token0 = [&](int tile) {
+    const int band = tile / (PAIR_BAND * n_tiles), in = tile % (PAIR_BAND * n_tiles);
+    return (band * PAIR_BAND + in % min(PAIR_BAND, m_tiles - band * PAIR_BAND)) * 2 * BM + (int)rank * BM;
+  };
+  auto feature0 = [&](int tile) {
+    const int band = tile / (PAIR_BAND * n_tiles), in = tile % (PAIR_BAND * n_tiles);
+    return in / min(PAIR_BAND, m_tiles - band * PAIR_BAND) * TN;
+  };
+  // first row of w that this block brings for the tile at n0
+  auto w_row = [&](int n0) { return EPI == 1 ? (int)rank * p.up_offset + n0 / 2 : n0 + (int)rank * (TN / 2); };
+
+  if (tid == PRODUCER_WARP * 32) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
+    for (int s = 0; s < PAIR_STAGES; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int b = 0; b < NACC; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], 2 * EPI_WARPS);
+    }
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == MMA_WARP) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)),
+                 "r"((uint32_t)(NACC * ACC_COLS))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncwarp();
+  __syncthreads();
+  cluster_barrier();                                      // the other block's barriers and tensor memory are there
+  // only now: a block of a later kernel that came to this multiprocessor first could take tensor memory and then wait for us
+  pdl_launch_dependents();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_d = tmem_base_slot;
+  volatile int* abortp = &abort_flag;
+
+  if (warp == PRODUCER_WARP) {
+    if (lane == 0) {
+      int it = 0;
+      auto expect = [&](int s) {
+        if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * (A_BYTES + B_BYTES));
+      };
+      auto load_x = [&](int s, int kb, int o0) { tma_load_pair(smem_u32(smem + s * STAGE), &map_x, kb * BK, o0, smem_u32(&full_bar[s])); };
+      auto load_w = [&](int s, int kb, int n0) {
+        tma_load_pair(smem_u32(smem + s * STAGE + A_BYTES), &map_w, kb * BK, w_row(n0), smem_u32(&full_bar[s]));
+      };
+      // the first ring of weights does not wait for the kernel before
+      const int pre = pair < total ? min(nkb, PAIR_STAGES) : 0;
+      for (int i = 0; i < pre; ++i) {
+        expect(i);
+        load_w(i, i, feature0(pair));
+      }
+      pdl_wait();
+      for (int i = 0; i < pre; ++i) load_x(i, i, token0(pair));
+      it = pre;
+      for (int tile = pair; tile < total && !*abortp; tile += pairs) {
+        const int o0 = token0(tile), n0 = feature0(tile);
+        for (int i = tile == pair ? pre : 0; i < nkb && !*abortp; ++i, ++it) {
+          const int s = it % PAIR_STAGES;
+          if (!mbar_wait(&empty_bar[s], ((it / PAIR_STAGES) & 1) ^ 1, abortp)) {
+            if (!*abortp) { *abortp = 1; atomicCAS(&g_error, 0, 1); }
+            break;
+          }
+          expect(s);
+          load_x(s, i, o0);
+          load_w(s, i, n0);
+        }
+      }
+      if (*abortp && rank == 0) {
+        // copies already requested still write into the pair's shared memory: wait for them, bounded
+        for (int i = max(0, it - PAIR_STAGES); i < it; ++i) {
+          const unsigned long long t0 = now_ns();
+          while (!mbar_try_wait(&full_bar[i % PAIR_STAGES], (i / PAIR_STAGES) & 1)) {
+            if (now_ns() - t0 > WAIT_LIMIT_NS) { atomicCAS(&g_error, 1, 4); break; }
+          }
+        }
+      }
+    }
+  } else if (warp == MMA_WARP) {
+    if (lane == 0 && rank == 0) {
+      constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(2 * BM >> 4) << 24);
+      int it = 0, round = 0;
+      for (int tile = pair; tile < total && !*abortp; tile += pairs, ++round) {
+        const int b = round % NACC;
+        if (round >= NACC && !mbar_wait(&acc_empty[b], ((round / NACC) - 1) & 1, abortp)) {
+          if (!*abortp) { *abortp = 1; atomicCAS(&g_error, 0, 3); }
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t acc = tmem_d + (uint32_t)(b * ACC_COLS);
+        bool fine = true;
+        for (int i = 0; i < nkb; ++i, ++it) {
+          const int s = it % PAIR_STAGES;
+          if (!mbar_wait(&full_bar[s], (it / PAIR_STAGES) & 1, abortp)) {
+            if (!*abortp) { *abortp = 1; atomicCAS(&g_error, 0, 2); }
+            fine = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t a_addr = smem_u32(smem + s * STAGE);
+          const uint64_t da = umma_desc(a_addr), db = umma_desc(a_addr + A_BYTES);
+#pragma unroll
+          for (int kk = 0; kk < BK / UMMA_K; ++kk) umma_pair_bf16(acc, da + 2 * kk, db + 2 * kk, IDESC, (i | kk) != 0);
+          umma_pair_commit(&empty_bar[s]);
+        }
+        if (!fine) break;
+        umma_pair_commit(&acc_full[b]);
+      }
+    }
+  } else {
+    pdl_wait();
+    int round = 0;
+    for (int tile = pair; tile < total; tile += pairs, ++round) {
+      const int b = round % NACC;
+      const bool have = mbar_wait(&acc_full[b], (round / NACC) & 1, abortp);
+      if (!have && !*abortp) { *abortp = 1; atomicCAS(&g_error, 0, 3); }
+      if (!have || *abortp) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int o0 = token0(tile);
+      if (o0 < p.o)                                       // uniform over the block: the pair's second half may lie past the tokens
+        token_rows_epilogue<TN, OT, EPI>(p, tmem_d + (uint32_t)(b * ACC_COLS) + ((uint32_t)(warp * 32) << 16), o0 + warp * 32 + lane,
+                                         feature0(tile), 0);
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive_first(&acc_empty[b]);
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncwarp();
+  __syncthreads();
+  cluster_barrier();                                      // nobody leaves while the other's products, copies or arrivals may come
+  if (warp == MMA_WARP) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"((uint32_t)(NACC * ACC_COLS)) : "memory");
+  }
+}
+
+
 // ---- host side: tensor maps ------------------------------------------------------------------
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -760,6 +978,50 @@ int launch(const CUtensorMap* mw, const CUtensorMap* mx, const GemmParams& p, in
   return llg_check_launch("gemm_tc");
 }
 
+template <int TN, typename OT, int EPI>
+int launch_pair(const void* x, const void* w, const GemmParams& p, cudaStream_t stream) {
+  constexpr int smem = PAIR_STAGES * (BM + 128) * BK * 2 + 1024;
+  static_assert(smem <= 232448 - 1024, "stage ring does not fit shared memory");
+  CUtensorMap map_x, map_w;
+  LLG_REQUIRE(tensor_map(x, p.o, p.k, BM, &map_x) && tensor_map(w, p.n, p.k, TN / 2, &map_w),
+              "gemm_tc: cuTensorMapEncodeTiled failed or is not available");
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<TN, OT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return llg_fail("gemm_tc: cannot have %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
+    configured = true;
+  }
+  const long long tiles = (long long)((p.o + 2 * BM - 1) / (2 * BM)) * (EPI == 1 ? (p.gated_features + TN / 2 - 1) / (TN / 2) : (p.n + TN - 1) / TN);
+  LLG_REQUIRE(tiles <= 2147483647LL / PAIR_BAND, "gemm_tc: too many tiles");
+  const long long pairs = llg_sm_count() / 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs)));
+  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = llg_pdl_enabled() ? 2 : 1;
+  cudaError_t le = cudaLaunchKernelEx(&cfg, gemm_pair_kernel<TN, OT, EPI>, map_x, map_w, p);
+  if (le != cudaSuccess) return llg_fail("gemm_tc: launch: %s", cudaGetErrorString(le));
+  return llg_check_launch("gemm_tc");
+}
+
+// What a prompt step's product costs in pairs of blocks with tiles of `width` features: rounds over the pairs times a round, in
+// units of the time that a block with one token tile takes per feature.  Measured at 8,192 tokens, k 4,096: a round is 26.6 us at
+// 256 features (0.80 of the other form's), 25.2 at 224, 23.6 at 192 and 22.3 at 160: it goes by the bytes brought, not by the
+// products, so narrower tiles than 224 never pay.
+double pair_cost(int tokens, int features, int width) {
+  const long long tiles = (long long)((tokens + 2 * BM - 1) / (2 * BM)) * ((features + width - 1) / width), pairs = llg_sm_count() / 2;
+  return (double)((tiles + pairs - 1) / pairs) * (width + (256 - width) / 2) * PAIR_UNIT;
+}
+
 }  // namespace
 
 // 1 if the tensor-core kernel takes these operands: k a multiple of 8 (TMA needs 16-byte row strides)
@@ -831,8 +1093,10 @@ static int gemm_tc_run(const void* x, const void* w, void* out, int out_dtype, i
               gated_features, o, splits);
   const int nkb = (k + BK - 1) / BK;
   CUtensorMap map_w, map_x;
-  if (n >= 256 && tile_n <= 0) {
-    // ---- prompt steps: activations are the first operand (128 tokens per tile), up to 256 features per tile ----
+  if (n > 128 && tile_n <= 0) {
+    // ---- prompt steps: activations are the first operand (128 tokens per tile), up to 256 features per tile.  From 129 tokens
+    // on: with the weights as first operand a gated tile of a step of few blocks fills 56 of its 128 rows, and the read-out of
+    // 256 token columns in pieces of 2 bytes is not hidden (8,192 x 2,048 gated at 232 tokens: 54 us that way, 26 this) ----
     // in this orientation the kernel's first-operand rows (field o) are the tokens, the second's (field n) the features
     GemmParams ps{out, /*n=*/o, /*o=*/n, k, (nkb + splits - 1) / splits, gated_features, o / 2, BM, QkPrepArgs{}, rs, act, nullptr, 0, gate, nullptr};
     // Tile shape: blocks run in rounds of one per SM (148 on a B200); a round costs its tile's width, and a narrower tile can save a
@@ -853,6 +1117,32 @@ static int gemm_tc_run(const void* x, const void* w, void* out, int out_dtype, i
           best_mt = mt;
         }
       }
+    }
+    // Pairs of blocks instead, where they come out cheaper.
+    if (splits == 1 && llg_sm_count() >= 2 && !(gated && out_dtype == LLG_F32)) {
+      const int pair_widths[2] = {256, 224};
+      int pw = 0;
+      double pc = best_cost;
+      for (int wi = 0; wi < 2; ++wi) {
+        const double cost = pair_cost(n, o, pair_widths[wi]);
+        if (cost < pc * 0.999) {
+          pc = cost;
+          pw = pair_widths[wi];
+        }
+      }
+#define PAIRS(OTT, EP)                                                   \
+  if (pw == 256) return launch_pair<256, OTT, EP>(x, w, ps, stream);     \
+  if (pw == 224) return launch_pair<224, OTT, EP>(x, w, ps, stream)
+      if (gated) {
+        PAIRS(__nv_bfloat16, 1);
+      } else if (act) {
+        PAIRS(__nv_bfloat16, -1);
+      } else if (out_dtype == LLG_F32) {
+        PAIRS(float, 0);
+      } else {
+        PAIRS(__nv_bfloat16, 0);
+      }
+#undef PAIRS
     }
     if (gated && out_dtype == LLG_F32) best_w = 256;
     // the gated product fetches the gate half and the up half of a feature tile with a box of half the width each
@@ -1003,6 +1293,9 @@ LLG_API int llg_gemm_tc_qkv(const void* x, const void* w, int n, int k, const Qk
   const long long sms = llg_sm_count();
   const long long t1 = (long long)((n + BM - 1) / BM) * ((o + 255) / 256), t2 = (long long)((n + 2 * BM - 1) / (2 * BM)) * ((o + 255) / 256);
   const bool two = (double)((t2 + sms - 1) / sms) * 2 * 0.85 < (double)((t1 + sms - 1) / sms);
+  // or a pair of blocks for two token tiles
+  if (sms >= 2 && pair_cost(n, o, 256) < 256.0 * (two ? (double)((t2 + sms - 1) / sms) * 2 * 0.85 : (double)((t1 + sms - 1) / sms)))
+    return a.hd == 128 ? launch_pair<256, __nv_bfloat16, 2>(x, w, ps, stream) : launch_pair<256, __nv_bfloat16, 3>(x, w, ps, stream);
   if (a.hd == 128)
     return two ? launch<256, 3, __nv_bfloat16, 2, 2, 1>(&map_x, &map_w, ps, 1, stream)
                : launch<256, 4, __nv_bfloat16, 1, 2, 1>(&map_x, &map_w, ps, 1, stream);

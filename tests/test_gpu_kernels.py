@@ -672,6 +672,30 @@ def test_qkv_product_with_the_preparation_as_its_epilogue(ops, nh, nkv, hd, k, n
 
 # ---- a norm that leaves its division to the products that consume it ------------------------------------------------
 
+@pytest.mark.parametrize("n,o,k", [(129, 21000, 64), (257, 30001, 72), (700, 9004, 264), (1030, 9000, 1032), (2305, 2600, 136)])
+def test_gemm_tc_of_large_steps(ops, n, o, k):
+    """Products of prompt steps in all their forms (one or two token tiles a block, pairs of blocks): token and feature tails, one k-block
+    and many, more tiles than blocks; plain in both types, with an activation, gated, with the rows' scales."""
+    x, w = rnd((n, k), 14, torch.bfloat16), rnd((o, k), 15, torch.bfloat16, 1.0 / math.sqrt(k))
+    ss = rnd((n, 3), 16).abs() * 40 + 1
+    scale, f = ops.RowScale(ss.to(DEV), 96, 1e-3), _scale_of(ss, 96, 1e-3)[:, None]
+    want = P.linear(x, w) * f
+    xd, wd = x.to(DEV), w.to(DEV)
+    for dtype in (torch.float32, torch.bfloat16):
+        out = torch.full((1, n, o), float("nan"), dtype=dtype, device=DEV)
+        ops.gemm_tc(xd, wd, out, row_scale=scale)
+        check(out[0].cpu(), want, dtype, "plain")
+    out = torch.full((n, o), float("nan"), dtype=torch.bfloat16, device=DEV)
+    ops.gemm_tc_act(xd, wd, out, "relu2")
+    check(out.cpu(), torch.relu(P.linear(x, w)) ** 2, torch.bfloat16, "activation")
+    feat = o // 2
+    g, u = want[:, :feat], want[:, feat:2 * feat]
+    act = torch.full((1, n, feat), float("nan"), dtype=torch.bfloat16, device=DEV)
+    ops.gemm_tc(xd, _gated(w[:feat], w[feat:2 * feat]).to(DEV), act, gated_features=feat, row_scale=scale)
+    check(act[0].cpu(), g / (1 + torch.exp(-g)) * u, torch.bfloat16, "gated")
+    assert ops.gemm_tc_status() == 0
+
+
 def _scale_of(ss, width, eps):
     """The factor a row scale stands for: 1 / sqrt(sum(ss) / width + eps) per row, float64."""
     return 1.0 / torch.sqrt(ss.double().sum(dim=1) / width + eps)
