@@ -25,6 +25,14 @@
 // A row's accumulator is rescaled in place (tcgen05.ld / tcgen05.st) only when its maximum grows by
 // more than a factor of 2^8 in the weights, warp by warp and only when some row of the warp needs it.
 //
+// Tiles of at most 128 queries (short prompts, the next turn of a chat) leave the second group without queries.  It then takes
+// part in one of two ways, which every block finds from its own tile.  SPLIT (two key tiles or more): the groups share the keys,
+// the first takes the even tiles and the second the odd ones, and the threads of a row join the two accumulators at the end: a
+// block's time is the chain of its key tiles (scores, softmax, product).  TWO_HEADS (one key tile, and more
+// blocks than multiprocessors): the second group takes the next query head of the same key/value head and that head's own block
+// ends at once; such blocks cost their set-up, so half as many are half the time.  Four sequences of 83 queries behind 1,000 to
+// 4,000 keys, 32 heads of 128: 63.4 us before, 55.8 now; five prompts of 3 to 90 tokens, 32 heads of 64: 19.0 us before, 12.7 now.
+//
 // With MAPS (differential attention) the two halves of a query and of a key are two maps over the same values: the block's
 // two groups are the two maps of ONE tile of 128 queries, whose scores are products over their half of the head; keys,
 // values and queries arrive once for both.  At the end every thread reads a half of its row of both accumulators, takes
@@ -222,6 +230,9 @@ struct TileInfo {
   int nq[GROUPS], pos0[GROUPS], n_tiles[GROUPS], n_max;
 };
 
+// What the second group does (above): queries of its own; the odd key tiles of the first group's; the next query head.
+enum { PLAIN = 0, SPLIT = 1, TWO_HEADS = 2 };
+
 template <int HD, bool MAPS>
 __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k_pages,
                                                                  const __grid_constant__ CUtensorMap map_v_pages,
@@ -236,7 +247,6 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
   // The tiles need 1024-byte alignment (swizzle); the declaration asks for it and the kernel checks it.
   extern __shared__ __align__(1024) unsigned char smem[];
   constexpr int Q_TILES = MAPS ? 1 : GROUPS;
-  constexpr int G_STEP = MAPS ? 0 : BQ;              // queries from one group's tile to the next one's
   unsigned char* Qs = smem;                          // [Q_TILES]
   unsigned char* Ks = Qs + Q_TILES * Q_BYTES;        // [KST]
   unsigned char* Vs = Ks + KST * KV_BYTES;           // [VST]
@@ -244,11 +254,54 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
   __shared__ uint64_t s_full[GROUPS][2], p_ready[GROUPS][2], o_done[GROUPS], q_ready;
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
+  __shared__ float split_share[MAPS ? 1 : GROUPS][2][MAPS ? 1 : BQ];     // SPLIT: each group's maximum and sum of a row
   __shared__ float map_share[MAPS ? 2 * GROUPS : 1][MAPS ? BQ : 1];      // 1 / sum of each map's weights, sums of squares
 
   pdl_launch_dependents();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) LLG_STAMP(5, 0, 0, blockIdx.x + gridDim.x * blockIdx.y);
+  // Blocks start in the order of blockIdx.x, then blockIdx.y: all heads of the list's first tile, then all
+  // heads of its second ...  The caller lists the tiles with the most keys first, so that the long blocks
+  // start first and the short ones fill the gaps at the end.
+  // (lengths and tiles are the step's, written before its first kernel: they need not wait for the kernel before this one)
+  TileInfo ti;
+  int mode = PLAIN;
+  {
+    const int tile_id = (int)blockIdx.y;
+    ti.b = a.tiles[2 * tile_id];
+    const int q_off = a.tiles[2 * tile_id + 1];
+    ti.tok0 = a.cu_tokens[ti.b];
+    const int total = a.cu_tokens[ti.b + 1] - ti.tok0;
+    ti.lb = a.len_before[ti.b];
+    ti.slot = a.slots[ti.b];
+    ti.n_max = 0;
+    for (int g = 0; g < GROUPS; ++g) {
+      ti.nq[g] = max(0, min(BQ, total - q_off - g * (MAPS ? 0 : BQ)));
+      ti.pos0[g] = ti.lb + q_off + g * (MAPS ? 0 : BQ);
+    }
+    if (!MAPS && ti.nq[0] > 0 && ti.nq[1] == 0) {
+      const int n_keys = ti.pos0[0] + ti.nq[0] - mask_first(ti.pos0[0], a.window, a.chunked) / TK * TK;
+      uint32_t sms;
+      asm("mov.u32 %0, %%nsmid;" : "=r"(sms));
+      if (n_keys > TK) mode = SPLIT;
+      else if ((a.nh / a.nkv) % 2 == 0 && gridDim.x * gridDim.y > sms) mode = TWO_HEADS;
+      if (mode != PLAIN) {
+        ti.nq[1] = ti.nq[0];
+        ti.pos0[1] = ti.pos0[0];
+      }
+    }
+    // the first group's window starts earliest; the second masks the tiles that lie before its own
+    int kb = mask_first(ti.pos0[0], a.window, a.chunked);
+    ti.k_begin = (kb / TK) * TK;
+    for (int g = 0; g < GROUPS; ++g) {
+      ti.n_tiles[g] = ti.nq[g] > 0 ? (ti.pos0[g] + ti.nq[g] - ti.k_begin + TK - 1) / TK : 0;
+      ti.n_max = max(ti.n_max, ti.n_tiles[g]);
+    }
+  }
+  if (mode == TWO_HEADS && (blockIdx.x & 1)) return;       // the block of the head before takes this one along
+  const int g_step = MAPS || mode != PLAIN ? 0 : BQ;       // queries from one group's tile to the next one's
+  const bool one_q = MAPS || mode == SPLIT;                // the groups read one tile of queries
+
   if ((smem_u32(smem) & 1023u) != 0) {          // uniform over the block
     if (tid == 0) atomicCAS(&g_error, 0, 3);
     return;
@@ -287,33 +340,8 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
   pdl_wait();
   if (tid == 0) LLG_STAMP(5, 1, 0, blockIdx.x + gridDim.x * blockIdx.y);
 
-  // Blocks start in the order of blockIdx.x, then blockIdx.y: all heads of the list's first tile, then all
-  // heads of its second ...  The caller lists the tiles with the most keys first, so that the long blocks
-  // start first and the short ones fill the gaps at the end.
-  TileInfo ti;
-  {
-    const int tile_id = (int)blockIdx.y;
-    ti.b = a.tiles[2 * tile_id];
-    const int q_off = a.tiles[2 * tile_id + 1];
-    ti.tok0 = a.cu_tokens[ti.b];
-    const int total = a.cu_tokens[ti.b + 1] - ti.tok0;
-    ti.lb = a.len_before[ti.b];
-    ti.slot = a.slots[ti.b];
-    ti.n_max = 0;
-    for (int g = 0; g < GROUPS; ++g) {
-      ti.nq[g] = max(0, min(BQ, total - q_off - g * G_STEP));
-      ti.pos0[g] = ti.lb + q_off + g * G_STEP;
-    }
-    // the first group's window starts earliest; the second masks the tiles that lie before its own
-    int kb = mask_first(ti.pos0[0], a.window, a.chunked);
-    ti.k_begin = (kb / TK) * TK;
-    for (int g = 0; g < GROUPS; ++g) {
-      ti.n_tiles[g] = ti.nq[g] > 0 ? (ti.pos0[g] + ti.nq[g] - ti.k_begin + TK - 1) / TK : 0;
-      ti.n_max = max(ti.n_max, ti.n_tiles[g]);
-    }
-  }
   const int h = blockIdx.x, kvh = h / (a.nh / a.nkv);
-  const int k_end = ti.pos0[0] + (ti.nq[1] > 0 ? G_STEP + ti.nq[1] : ti.nq[0]);   // keys past it are never copied
+  const int k_end = ti.pos0[0] + (ti.nq[1] > 0 ? g_step + ti.nq[1] : ti.nq[0]);   // keys past it are never copied
   const int q_tok0 = ti.tok0 + ti.pos0[0] - ti.lb;                              // first token of the first query tile
 
   // queries: thread r of group g copies its part of tile g; the issuing lane waits for all of them,
@@ -321,11 +349,12 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
   if (tid < WORKERS) {
     const int g = tid / BQ, r = tid % BQ;
     const int ch = r % CPR;
-    constexpr int ROWS = BQ / CPR;                   // rows a group copies side by side; with MAPS the groups share the tile's rows
-    for (int row = r / CPR + (MAPS ? g * ROWS : 0); row < BQ; row += MAPS ? GROUPS * ROWS : ROWS) {
+    constexpr int ROWS = BQ / CPR;                   // rows a group copies side by side; with one tile the groups share its rows
+    const int head = h + (mode == TWO_HEADS ? g : 0);
+    for (int row = r / CPR + (one_q ? g * ROWS : 0); row < BQ; row += one_q ? GROUPS * ROWS : ROWS) {
       const bool valid = row < ti.nq[g];
-      const bf16* src = (const bf16*)a.q + ((long long)(q_tok0 + g * G_STEP + (valid ? row : 0)) * a.nh + h) * HD + ch * 8;
-      cp_async16(smem_u32(Qs + (MAPS ? 0 : g * Q_BYTES)) + (uint32_t)((ch >> 3) * (BQ * 128)) + swz(row, ch & 7), src, valid);
+      const bf16* src = (const bf16*)a.q + ((long long)(q_tok0 + g * g_step + (valid ? row : 0)) * a.nh + head) * HD + ch * 8;
+      cp_async16(smem_u32(Qs + (one_q ? 0 : g * Q_BYTES)) + (uint32_t)((ch >> 3) * (BQ * 128)) + swz(row, ch & 7), src, valid);
     }
     cp_async_commit();
     cp_async_wait<0>();
@@ -411,17 +440,27 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
     if (elect_one()) {
       constexpr uint32_t IDESC_S = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TK >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
       constexpr uint32_t IDESC_O = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
-      // scores of key tile t for group g into the group's score buffer t % 2
-      auto issue_scores = [&](int g, int t) {
-        const uint32_t qa = smem_u32(Qs + (MAPS ? 0 : g * Q_BYTES)), ka = smem_u32(Ks + (t % KST) * KV_BYTES);
+      // scores of key tile t, the group's own tile i (the same number but for SPLIT), into the group's score buffer i % 2
+      auto issue_scores = [&](int g, int t, int i) {
+        const uint32_t qa = smem_u32(Qs + (one_q ? 0 : g * Q_BYTES)), ka = smem_u32(Ks + (t % KST) * KV_BYTES);
 #pragma unroll
         for (int ks = 0; ks < (MAPS ? HD / 32 : HD / 16); ++ks) {
           const int at = MAPS ? g * (HD / 32) + ks : ks;
           const uint32_t blk = at >> 2, kk = at & 3;      // 64-wide block, 16-wide step inside it (32 bytes)
-          umma_bf16(tmem + g * G_COLS + (uint32_t)(t & 1) * TK, desc_kmajor(qa + blk * (BQ * 128) + kk * 32),
+          umma_bf16(tmem + g * G_COLS + (uint32_t)(i & 1) * TK, desc_kmajor(qa + blk * (BQ * 128) + kk * 32),
                     desc_kmajor(ka + blk * (TK * 128) + kk * 32), IDESC_S, ks != 0);
         }
-        umma_commit(&s_full[g][t & 1]);
+        umma_commit(&s_full[g][i & 1]);
+      };
+      // O += P(i) V(t)
+      auto issue_values = [&](int g, int t, int i) {
+        const uint32_t pa = tmem + g * G_COLS + (uint32_t)(i & 1) * TK, va = smem_u32(Vs + (t % VST) * KV_BYTES);
+#pragma unroll
+        for (int kk = 0; kk < TK / 16; ++kk) {
+          // 16 keys further: 8 columns of packed weights, 16 rows (2048 bytes) down V
+          umma_bf16_ts(tmem + g * G_COLS + O_COL, pa + kk * 8, desc_mnmajor(va + kk * 2048, TK * 128), IDESC_O, (i | kk) != 0);
+        }
+        umma_commit(&o_done[g]);
       };
       bool ok = true;
       auto wait_or_fail = [&](uint64_t* bar, uint32_t parity, int code) {
@@ -436,10 +475,37 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
         wait_or_fail(&k_full[0], 0, 5);
         if (ok) {
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          for (int g = 0; g < GROUPS; ++g)
-            if (0 < ti.n_tiles[g]) issue_scores(g, 0);
+          for (int g = 0; g < (mode == SPLIT ? 1 : GROUPS); ++g)
+            if (0 < ti.n_tiles[g]) issue_scores(g, 0, 0);
           umma_commit(&k_free[0]);
         }
+      }
+      if (!MAPS && mode == SPLIT) {
+        // tile t is group t % 2's tile t / 2; both groups' first scores, then per tile the group's next scores and O += P V
+        wait_or_fail(&k_full[1 % KST], 0, 5);
+        if (ok) {
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          issue_scores(1, 1, 0);
+          umma_commit(&k_free[1 % KST]);
+        }
+        for (int t = 0; t < ti.n_max && ok; ++t) {
+          const int g = t & 1, i = t >> 1;
+          if (t + 2 < ti.n_max) {
+            wait_or_fail(&k_full[(t + 2) % KST], ((t + 2) / KST) & 1, 5);
+            if (i >= 1) wait_or_fail(&o_done[g], (i - 1) & 1, 6);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            issue_scores(g, t + 2, i + 1);
+            umma_commit(&k_free[(t + 2) % KST]);
+          }
+          wait_or_fail(&v_full[t % VST], (t / VST) & 1, 5);
+          wait_or_fail(&p_ready[g][i & 1], (i >> 1) & 1, 6);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          issue_values(g, t, i);
+          umma_commit(&v_free[t % VST]);
+        }
+        ok = false;                                        // (nothing is left for the loop below)
       }
       // Step j: the scores of tile j + 1 go into the buffer whose weights P(j-1) the product of step j - 1 has
       // read by now; then, once the group has turned S(j) into P(j) (written over S(j) in tensor memory),
@@ -453,18 +519,12 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
             if (j >= 1) wait_or_fail(&o_done[g], (j - 1) & 1, 6);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            issue_scores(g, j + 1);
+            issue_scores(g, j + 1, j + 1);
           }
           wait_or_fail(&p_ready[g][j & 1], (j >> 1) & 1, 6);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t pa = tmem + g * G_COLS + (uint32_t)(j & 1) * TK, va = smem_u32(Vs + (j % VST) * KV_BYTES);
-#pragma unroll
-          for (int kk = 0; kk < TK / 16; ++kk) {
-            // 16 keys further: 8 columns of packed weights, 16 rows (2048 bytes) down V
-            umma_bf16_ts(tmem + g * G_COLS + O_COL, pa + kk * 8, desc_mnmajor(va + kk * 2048, TK * 128), IDESC_O, (j | kk) != 0);
-          }
-          umma_commit(&o_done[g]);
+          issue_values(g, j, j);
         }
         if (!ok) break;
         umma_commit(&v_free[j % VST]);
@@ -475,7 +535,8 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
     // ---- softmax: thread r of group g owns query row r of tile g ------------------------------------
     const int g = tid / BQ, r = tid % BQ, gw = (tid % BQ) >> 5;       // gw: warp inside the group = its lane quarter
     const uint32_t lane_base = tmem + g * G_COLS + ((uint32_t)(gw * 32) << 16);
-    const int n_tiles = ti.n_tiles[g], pos0 = ti.pos0[g];
+    const bool split = !MAPS && mode == SPLIT;
+    const int n_tiles = split ? (ti.n_max + 1 - g) >> 1 : ti.n_tiles[g], pos0 = ti.pos0[g];
     const float sc = a.scale * LOG2E;
     // A row's weights are 2^(x - M) with x = score * scale * log2 e and M a whole number that is raised (to the
     // tile's maximum, rounded up) only when a tile exceeds it by more than 8: the weights stay below 2^8 and the
@@ -493,7 +554,7 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int kt = ti.k_begin + j * TK;
+      const int kt = ti.k_begin + (split ? 2 * j + g : j) * TK;
       float sv[TK];
       {
         uint32_t r0_[16], r1_[16], r2_[16], r3_[16];
@@ -621,12 +682,49 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
           *reinterpret_cast<uint4*>(dst + c0) = v;
         }
       }
+    } else if (split) {
+      // the two groups meet, as above: every thread joins a half of its row's two accumulators
+      split_share[g][0][r] = m_run;
+      split_share[g][1][r] = l_run;
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      asm volatile("bar.sync 1, %0;" ::"n"(WORKERS) : "memory");
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (!*abortp) {
+        const float m0 = split_share[0][0][r], m1 = split_share[1][0][r], m = fmaxf(m0, m1);
+        float w0 = m0 == -INFINITY ? 0.f : fast_exp2(m0 - m), w1 = m1 == -INFINITY ? 0.f : fast_exp2(m1 - m);
+        float l = split_share[0][1][r] * w0 + split_share[1][1][r] * w1;
+        if (a.has_sink) l += fast_exp2((a.sinks ? a.sinks[h] : a.sink_score) * LOG2E - m);
+        float inv = l > 0.f ? 1.0f / l : 0.f;
+        if (a.gate && r < ti.nq[g]) inv *= a.gate[(long long)(q_tok0 + r) * a.nh + h];
+        w0 *= inv;
+        w1 *= inv;
+        const uint32_t row = tmem + O_COL + ((uint32_t)(gw * 32) << 16) + (uint32_t)(g * (HD / 2));
+        bf16* dst = (bf16*)a.out + ((long long)(q_tok0 + r) * a.nh + h) * HD + g * (HD / 2);
+#pragma unroll
+        for (int c0 = 0; c0 < HD / 2; c0 += 16) {
+          uint32_t r0_[16], r1_[16];
+          tmem_ld16(row + c0, r0_);
+          tmem_ld16(row + G_COLS + c0, r1_);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (r < ti.nq[g]) {
+            float o[16];
+#pragma unroll
+            for (int c = 0; c < 16; ++c) o[c] = fmaf(w1, __uint_as_float(r1_[c]), w0 * __uint_as_float(r0_[c]));
+            uint4 v0, v1;
+            v0.x = pack_bf16(o[0], o[1]); v0.y = pack_bf16(o[2], o[3]); v0.z = pack_bf16(o[4], o[5]); v0.w = pack_bf16(o[6], o[7]);
+            v1.x = pack_bf16(o[8], o[9]); v1.y = pack_bf16(o[10], o[11]); v1.z = pack_bf16(o[12], o[13]); v1.w = pack_bf16(o[14], o[15]);
+            *reinterpret_cast<uint4*>(dst + c0) = v0;
+            *reinterpret_cast<uint4*>(dst + c0 + 8) = v1;
+          }
+        }
+      }
     } else if (ok && !*abortp) {
+      const int head = h + (mode == TWO_HEADS ? g : 0);
       // a sink joins the sum with its own weight 2^(sink - M) and carries no value; a gate scales the head's output
-      if (a.has_sink) l_run += fast_exp2((a.sinks ? a.sinks[h] : a.sink_score) * LOG2E - m_run);
+      if (a.has_sink) l_run += fast_exp2((a.sinks ? a.sinks[head] : a.sink_score) * LOG2E - m_run);
       float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
-      if (a.gate && r < ti.nq[g]) inv *= a.gate[(long long)(q_tok0 + g * BQ + r) * a.nh + h];
-      bf16* dst = (bf16*)a.out + ((long long)(q_tok0 + g * BQ + r) * a.nh + h) * HD;
+      if (a.gate && r < ti.nq[g]) inv *= a.gate[(long long)(q_tok0 + g * g_step + r) * a.nh + head];
+      bf16* dst = (bf16*)a.out + ((long long)(q_tok0 + g * g_step + r) * a.nh + head) * HD;
 #pragma unroll
       for (int c0 = 0; c0 < HD; c0 += 16) {
         uint32_t rr[16];

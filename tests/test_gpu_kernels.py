@@ -414,6 +414,39 @@ def test_attn_prefill_and_kv_write(ops, dtype, nh, nkv, hd, window, tc, monkeypa
         assert ops.attn_tc_status() == 0
 
 
+@pytest.mark.parametrize("before,counts,window", [([0] * 6, [3, 64, 1, 37, 63, 17], 0), ([0, 63, 64, 65, 300, 0], [128, 1, 64, 83, 100, 65], 0),
+                                                  ([10, 200, 517, 0, 0, 40], [5, 83, 128, 129, 40, 24], 100)],
+                         ids=["one key tile", "several", "window"])
+@pytest.mark.parametrize("nh,nkv", [(32, 8), (32, 32), (30, 10)])
+@pytest.mark.parametrize("hd", [64, 128])
+def test_attn_prefill_of_few_queries_per_sequence(ops, hd, nh, nkv, before, counts, window):
+    """Tiles of at most 128 queries in the tcgen05 kernel, more blocks than multiprocessors: two heads in a block where a sequence has
+    one key tile (an odd group of heads: one), the keys shared by the block's two halves where it has more; tiles of more beside them."""
+    dtype, scale = torch.bfloat16, 1 / math.sqrt(hd)
+    ring = 16 if window == 0 else (window + 63) // 64 + 1
+    total = [a + c for a, c in zip(before, counts)]
+    kp, vp, table, slots, ks, vs = _paged(nkv, hd, dtype, total, 44, ring, 80)
+    for b, n in enumerate(before):                       # the cache as it was before the step
+        for p in range(max(0, n - ring * 64), n):
+            pg = int(table[slots[b], (p // 64) % ring])
+            kp[pg, :, p % 64], vp[pg, :, p % 64] = ks[b][p], vs[b][p]
+    cu = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32)
+    q = rnd((int(cu[-1]), nh, hd), 45, dtype)
+    k_new, v_new = (torch.cat([t[b][before[b]:] for b in range(len(counts))]) for t in (ks, vs))
+    tq = ops.prefill_tile_queries(dtype, hd)
+    tiles = torch.tensor([(b, q0) for b, c in enumerate(counts) for q0 in range(0, c, tq)], dtype=torch.int32)
+    out = torch.full((int(cu[-1]), nh * hd), float("nan"), dtype=dtype, device=DEV)
+    d = lambda t: t.to(DEV)
+    ops.attn_prefill(d(q), d(k_new), d(v_new), d(kp), d(vp), d(table), ring, d(tiles), d(cu), d(torch.tensor(before, dtype=torch.int32)),
+                     d(slots), out, scale=scale, window=window, tile_queries=tq)
+    assert ops.attn_tc_status() == 0
+    for b in range(len(counts)):
+        qq = torch.zeros(total[b], nh, hd, dtype=dtype)
+        qq[before[b]:] = q[int(cu[b]):int(cu[b + 1])]
+        ref = P.attention(qq, ks[b], vs[b], scale, window)[before[b]:].reshape(counts[b], -1)
+        check(out[int(cu[b]):int(cu[b + 1])], ref, dtype, ("sequence", b))
+
+
 @pytest.mark.parametrize("tc", [True, False], ids=["tcgen05", "mma"])
 @pytest.mark.parametrize("shape", ["slow", "steps"])
 @pytest.mark.parametrize("hd", [64, 128])
