@@ -117,6 +117,11 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
+__device__ __forceinline__ float tmem_ld1(uint32_t taddr) {
+  uint32_t r;
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr));
+  return __uint_as_float(r);
+}
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -155,6 +160,10 @@ struct GemmParams {
   int group_rows;
   GateForm gate;            // EPI 1 (the gated epilogue)
   const float* row_weight;  // EPI 1, SWAP 1: null, or one number per token row that both products are multiplied by
+  // Grouped products of few tokens (SWAP 0, TN = 32 = the layout's rows per tile): a decode step's experts, a stream of their
+  // matrices.  token_of_row null: the tile's rows of x; else x holds all tokens of the step (32 at most), every tile multiplies
+  // with all of them, and row r of the layout takes token token_of_row[r]'s column (row_weight as above; negative: zeros).
+  const int* token_of_row;
 };
 
 // The activation of an epilogue on sixteen values.  The square of relu is two instructions a value and stays in line; the
@@ -403,11 +412,11 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tc_kernel(const __grid_cons
       tma_load_2d(dst, &map_x, kb * BK, row0 + n0, bar);
     }
   };
-  const bool grouped = SWAP == 1 && MT == 1 && p.tile_group != nullptr;
+  const bool grouped = (SWAP == 1 ? MT == 1 : TN == 32) && p.tile_group != nullptr;
   // first operand: MT tiles of 128 rows
-  auto load_first = [&](unsigned char* dst, int kb, int o0, uint64_t* bar) {
+  auto load_first = [&](unsigned char* dst, int kb, int o0, uint64_t* bar, int row0 = 0) {
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt) tma_load_2d(dst + mt * A_TILE, &map_w, kb * BK, w_row(o0, mt), bar);
+    for (int mt = 0; mt < MT; ++mt) tma_load_2d(dst + mt * A_TILE, &map_w, kb * BK, row0 + w_row(o0, mt), bar);
   };
   // A block works through tiles blockIdx.x, blockIdx.x + gridDim.x, ...: token tiles of one weight tile are neighbours
   // in that order, so blocks running side by side share the weight tile in L2.
@@ -434,7 +443,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tc_kernel(const __grid_cons
   auto first_offset = [&](int tile) { return tile_m(tile) * (GATED_ROWS ? p.gate_rows : BM * MT); };
   auto second_offset = [&](int tile) { return tile_n(tile) * TN; };
   // the group of a tile's tokens (read only after the dependency wait)
-  auto group_of = [&](int tile) { return p.tile_group[tile_m(tile)]; };
+  auto group_of = [&](int tile) { return p.tile_group[SWAP ? tile_m(tile) : tile_n(tile)]; };
   const int nkb_total = (p.k + BK - 1) / BK;
   const int kb0 = split * p.kb_per_split;
   const int nkb = min(p.kb_per_split, nkb_total - kb0);   // >= 1 by construction of the grid
@@ -514,8 +523,8 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tc_kernel(const __grid_cons
           }
           mbar_expect_tx(&full_bar[s], stage_tx);
           unsigned char* a = smem + s * STAGE_BYTES;
-          load_first(a, kb0 + i, o0, &full_bar[s]);
-          load_second(a + A_BYTES, kb0 + i, n0, &full_bar[s], w_row0);
+          load_first(a, kb0 + i, o0, &full_bar[s], SWAP ? 0 : w_row0);
+          load_second(a + A_BYTES, kb0 + i, !SWAP && p.token_of_row ? 0 : n0, &full_bar[s], SWAP ? w_row0 : 0);
         }
       }
       if (*abortp) {
@@ -643,6 +652,21 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tc_kernel(const __grid_cons
           const int row = warp * 32 + lane;
           const int inter = row < p.gate_rows ? p.gated_features : 0;
           const int f = o0 + row;
+          if (TN == 32 && p.token_of_row) {
+            // the layout's rows one after another: most of a decode step's tile are filling rows
+#pragma unroll 1
+            for (int j = 0; j < TN; ++j) {
+              const int tok = p.token_of_row[n0 + j];           // the same for the whole block
+              float v = 0.f;
+              if (tok >= 0 && tok < TN) {
+                const float rw = p.row_weight ? p.row_weight[n0 + j] : 1.0f;
+                const float g = tmem_ld1(lane_base + (uint32_t)tok), u = tmem_ld1(lane_base + (uint32_t)(TN + tok));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                v = gate_act(gate, g * rw, u * rw);
+              }
+              if (f < inter) out[(long long)(n0 + j) * p.gated_features + f] = from_f32<OT>(v);
+            }
+          } else {
   #pragma unroll
           for (int c0 = 0; c0 < TN; c0 += CH) {
             if (n0 + c0 >= p.n) break;
@@ -672,6 +696,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tc_kernel(const __grid_cons
                   if (n0 + c0 + 16 * q + c < p.n) dst[(long long)c * inter] = from_f32<OT>(v[c]);
               }
             }
+          }
           }
         }
       }
@@ -1098,7 +1123,7 @@ static int gemm_tc_run(const void* x, const void* w, void* out, int out_dtype, i
     // on: with the weights as first operand a gated tile of a step of few blocks fills 56 of its 128 rows, and the read-out of
     // 256 token columns in pieces of 2 bytes is not hidden (8,192 x 2,048 gated at 232 tokens: 54 us that way, 26 this) ----
     // in this orientation the kernel's first-operand rows (field o) are the tokens, the second's (field n) the features
-    GemmParams ps{out, /*n=*/o, /*o=*/n, k, (nkb + splits - 1) / splits, gated_features, o / 2, BM, QkPrepArgs{}, rs, act, nullptr, 0, gate, nullptr};
+    GemmParams ps{out, /*n=*/o, /*o=*/n, k, (nkb + splits - 1) / splits, gated_features, o / 2, BM, QkPrepArgs{}, rs, act, nullptr, 0, gate, nullptr, nullptr};
     // Tile shape: blocks run in rounds of one per SM (148 on a B200); a round costs its tile's width, and a narrower tile can save a
     // round (4096 features: 16 tiles of 256 in two token rows of 8 are 128 blocks, 18 of 240 are 144).  Two token
     // tiles per block halve the weight traffic per flop (worth about 15 %) but double the tile.
@@ -1191,7 +1216,7 @@ static int gemm_tc_run(const void* x, const void* w, void* out, int out_dtype, i
     if (gate_rows < 16) gate_rows = 16;
     if (gate_rows > BM) gate_rows = BM;
   }
-  GemmParams p{out, n, o, k, (nkb + splits - 1) / splits, gated_features, o / 2, gate_rows, QkPrepArgs{}, rs, act, nullptr, 0, gate, nullptr};
+  GemmParams p{out, n, o, k, (nkb + splits - 1) / splits, gated_features, o / 2, gate_rows, QkPrepArgs{}, rs, act, nullptr, 0, gate, nullptr, nullptr};
   LLG_REQUIRE(splits <= 65535, "gemm_tc: grid too large");
   LLG_REQUIRE(tensor_map(w, o, k, gated ? gate_rows : BM, &map_w) && tensor_map(x, n, k, tile_n, &map_x),
               "gemm_tc: cuTensorMapEncodeTiled failed or is not available");
@@ -1247,7 +1272,7 @@ LLG_API int llg_gemm_tc_grouped(const void* x, const void* w, void* out, int out
   LLG_REQUIRE((long long)n_groups * group_rows < 2147483647LL, "gemm_tc_grouped: too many rows of w");
   const int nkb = (k + BK - 1) / BK;
   const RowScale rs{nullptr, 0, 0.f, 0.f};
-  GemmParams ps{out, /*n=*/o, /*o=*/rows, k, nkb, gated_features, o / 2, BM, QkPrepArgs{}, rs, 0, tile_group, group_rows, form ? *form : SILU_FORM, row_weight};
+  GemmParams ps{out, /*n=*/o, /*o=*/rows, k, nkb, gated_features, o / 2, BM, QkPrepArgs{}, rs, 0, tile_group, group_rows, form ? *form : SILU_FORM, row_weight, nullptr};
   CUtensorMap map_w, map_x;
   LLG_REQUIRE(tensor_map(x, rows, k, BM, &map_x) && tensor_map(w, n_groups * group_rows, k, gated ? 128 : 256, &map_w),
               "gemm_tc_grouped: cuTensorMapEncodeTiled failed or is not available");
@@ -1255,6 +1280,47 @@ LLG_API int llg_gemm_tc_grouped(const void* x, const void* w, void* out, int out
   if (out_dtype == LLG_F32) return launch<256, 4, float, 1, 0, 1>(&map_x, &map_w, ps, 1, stream);
   if (out_dtype == LLG_BF16) return launch<256, 4, __nv_bfloat16, 1, 0, 1>(&map_x, &map_w, ps, 1, stream);
   return llg_fail("gemm_tc_grouped: unknown output dtype %d", out_dtype);
+}
+
+// The grouped product for few tokens, a stream of the groups' matrices: weights are the tensor cores' rows (128 features, or
+// fewer of a gated product so that the blocks are as many as the multiprocessors), 32 rows of the layout the columns.  `rows` is
+// a multiple of 32.  Plain: x [rows][k] is the layout, out [rows][o] float32.  Gated: x [n_tokens][k] holds all tokens of the step (32
+// at most), token_of_row says which token a row takes (negative: zeros), out [rows][gated_features] bfloat16.
+LLG_API int llg_gemm_tc_grouped_few(const void* x, int n_tokens, const void* w, void* out, int rows, int o, int k, int gated_features,
+                                    const int* tile_group, const int* token_of_row, int n_groups, int group_rows, const GateForm* form,
+                                    const float* row_weight, cudaStream_t stream) {
+  constexpr int TN = 32;
+  LLG_REQUIRE(rows > 0 && rows % TN == 0, "gemm_tc_grouped_few: %d rows are no multiple of %d", rows, TN);
+  LLG_REQUIRE(tile_group != nullptr && n_groups > 0 && group_rows >= o, "gemm_tc_grouped_few: needs the tiles' groups and their rows of w");
+  LLG_REQUIRE(llg_gemm_tc_supported(x, w, rows, o, k), "gemm_tc_grouped_few: needs k %% 8 == 0 and 16-byte aligned operands (k=%d)", k);
+  const bool gated = gated_features > 0;
+  LLG_REQUIRE(!gated || (o == ((gated_features + BM - 1) / BM) * 2 * BM && token_of_row && n_tokens > 0 && n_tokens <= TN),
+              "gemm_tc_grouped_few: the gated epilogue needs ceil(features / 128) * 256 rows of w per group and at most %d tokens", TN);
+  LLG_REQUIRE(gated || (!form && !row_weight && !token_of_row && n_tokens == rows),
+              "gemm_tc_grouped_few: a form of gating, row weights and tokens go with the gated layout");
+  LLG_REQUIRE((long long)n_groups * group_rows < 2147483647LL, "gemm_tc_grouped_few: too many rows of w");
+  const int nkb = (k + BK - 1) / BK;
+  // features per block of the gated product: few rounds of blocks over the multiprocessors, if about eight experts a token are in use
+  int gate_rows = BM;
+  if (gated) {
+    const long long sms = llg_sm_count(), tiles = rows / TN;
+    long long used = tiles < n_groups ? tiles : n_groups, best = 0;
+    if (used > 8LL * n_tokens) used = 8LL * n_tokens;
+    for (int gr = BM; gr >= 32; gr -= 8) {
+      const long long cost = (((gated_features + gr - 1) / gr) * used + sms - 1) / sms * (gr + 8);
+      if (best == 0 || cost < best) {
+        best = cost;
+        gate_rows = gr;
+      }
+    }
+  }
+  GemmParams p{out, rows, o, k, nkb, gated_features, o / 2, gate_rows, QkPrepArgs{}, RowScale{nullptr, 0, 0.f, 0.f}, 0, tile_group, group_rows,
+               form ? *form : SILU_FORM, row_weight, token_of_row};
+  CUtensorMap map_w, map_x;
+  LLG_REQUIRE(tensor_map(w, n_groups * group_rows, k, gate_rows, &map_w) && tensor_map(x, n_tokens, k, TN, &map_x),
+              "gemm_tc_grouped_few: cuTensorMapEncodeTiled failed or is not available");
+  return gated ? launch<TN, 5, __nv_bfloat16, 2, 1, 0>(&map_w, &map_x, p, 1, stream)
+               : launch<TN, 5, float, 1, 0, 0>(&map_w, &map_x, p, 1, stream);
 }
 
 // 1 when llg_gemm_tc_qkv takes this q/k/v projection: 256 tokens or more (tokens are the tensor cores' rows), head

@@ -311,10 +311,16 @@ __global__ void __launch_bounds__(256) grouped_linear_kernel(GroupedLinearArgs a
 // ---- the grouped products on the tensor cores (bfloat16) ------------------------------------------------------------
 //
 // A block of four warps takes one tile of LLG_MOE_TILE rows (one expert) and MM_O outputs; the activations' rows (gathered
-// through token_of_row) and the expert's matrix rows arrive in shared memory by 16-byte asynchronous copies, two stages
+// through token_of_row) and the expert's matrix rows arrive in shared memory by 16-byte asynchronous copies, STAGES
 // deep, in k-blocks of MM_K; every warp owns MM_O / 4 outputs of all rows and multiplies with mma.sync m16n8k16 (bfloat16
 // in, float32 sums).  GATED: a second matrix's tile beside the first, and what the gate's form makes of the two is stored.
-constexpr int MM_O = 128, MM_K = 64, MM_PAD = 8;            // MM_PAD halves between rows: fragment loads meet no bank twice
+//
+// Two shapes.  Many tiles (prompts): 128 outputs, two stages, the matrix rows used for the most products.  Few tiles: the kernel is
+// a stream of the chosen experts' matrices, and what bounds it is the bytes that the multiprocessors have under way: 64 outputs
+// and three stages (four of one matrix) give twice the blocks, two or three of them a multiprocessor.  100 tokens' four of 16
+// experts of 1,024 x 2,048: gated 57.4 -> 45.9 us, of 1,792 x 4,096 (eight tokens) 110 -> 88; one matrix 30.9 -> 21.5, 55 -> 59.
+constexpr int MM_K = 64, MM_PAD = 8;                        // MM_PAD halves between rows: fragment loads meet no bank twice
+constexpr int MM_WIDE = 128, MM_NARROW = 64;
 constexpr int MM_LD = MM_K + MM_PAD;
 
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* src, bool valid) {
@@ -331,7 +337,7 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const unsigned (&a)[4], 
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-template <typename YT, bool GATED>
+template <typename YT, bool GATED, int MM_O, int STAGES>
 __global__ void __launch_bounds__(128) grouped_linear_mma_kernel(GroupedLinearArgs a) {
   pdl_launch_dependents();
   pdl_wait();
@@ -384,18 +390,17 @@ __global__ void __launch_bounds__(128) grouped_linear_mma_kernel(GroupedLinearAr
         if (GATED) acc2[i][j][c] = 0.f;
       }
   const int nkb = (a.n_in + MM_K - 1) / MM_K;
-  load_stage(0, 0);
-  cp_async_commit();
+#pragma unroll
+  for (int st = 0; st < STAGES - 1; ++st) {
+    if (st < nkb) load_stage(st, st * MM_K);
+    cp_async_commit();
+  }
   for (int kb = 0; kb < nkb; ++kb) {
-    if (kb + 1 < nkb) {
-      load_stage((kb + 1) & 1, (kb + 1) * MM_K);
-      cp_async_commit();
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    const bf16* As = base + (kb & 1) * STAGE_HALVES;
+    cp_async_wait<STAGES - 2>();                              // one group a k-block, empty ones past the last: block kb is there
+    __syncthreads();                                          // for every warp; and all are done with the stage that comes next
+    if (kb + STAGES - 1 < nkb) load_stage((kb + STAGES - 1) % STAGES, (kb + STAGES - 1) * MM_K);
+    cp_async_commit();
+    const bf16* As = base + (kb % STAGES) * STAGE_HALVES;
     const bf16* Bs = As + A_HALVES + warp * (MM_O / 4) * MM_LD;
 #pragma unroll
     for (int ks = 0; ks < MM_K; ks += 16) {
@@ -421,7 +426,6 @@ __global__ void __launch_bounds__(128) grouped_linear_mma_kernel(GroupedLinearAr
         }
       }
     }
-    __syncthreads();                                          // the stage is free for the copies of the step after next
   }
   YT* y = (YT*)a.y + (long long)e * a.y_group_stride;
 #pragma unroll
@@ -516,6 +520,30 @@ __global__ void moe_combine_vec4_kernel(const float* __restrict__ y, const int* 
 
 }  // namespace
 
+// Launches the tensor-core product: `groups` along z where the group is the block's own (otherwise 1).
+template <typename YT, bool GATED, int MM_O, int STAGES>
+static int launch_mma(const char* what, const GroupedLinearArgs& a, int groups, cudaStream_t stream) {
+  const dim3 grid(a.rows / LLG_MOE_TILE, (a.n_out + MM_O - 1) / MM_O, groups);
+  LLG_REQUIRE(grid.y <= 65535, "%s: too many outputs", what);
+  const size_t smem = STAGES * (size_t)(LLG_MOE_TILE * MM_LD + (GATED ? 2 : 1) * MM_O * MM_LD) * sizeof(__nv_bfloat16);
+  cudaError_t err = cudaFuncSetAttribute(grouped_linear_mma_kernel<YT, GATED, MM_O, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (err != cudaSuccess) return llg_fail("%s: shared memory %zu: %s", what, smem, cudaGetErrorString(err));
+  err = llg_launch(grouped_linear_mma_kernel<YT, GATED, MM_O, STAGES>, grid, dim3(128), smem, stream, a);
+  if (err != cudaSuccess) return llg_fail("%s: launch: %s", what, cudaGetErrorString(err));
+  return llg_check_launch(what);
+}
+
+// 64 outputs a block where 128 would give fewer than MM_FEW blocks a multiprocessor (a tile may hold no tokens at all: the layout
+// has a tile for every expert) and the blocks of 64 stay within a grid.
+constexpr int MM_FEW = 4;
+template <typename YT, bool GATED>
+static int run_mma(const char* what, const GroupedLinearArgs& a, int groups, cudaStream_t stream) {
+  const long long wide = (long long)(a.rows / LLG_MOE_TILE) * ((a.n_out + MM_WIDE - 1) / MM_WIDE) * groups;
+  if (wide < (long long)MM_FEW * llg_sm_count() && (a.n_out + MM_NARROW - 1) / MM_NARROW <= 65535)
+    return launch_mma<YT, GATED, MM_NARROW, GATED ? 3 : 4>(what, a, groups, stream);
+  return launch_mma<YT, GATED, MM_WIDE, 2>(what, a, groups, stream);
+}
+
 static int check_rule(const char* what, const RouterRule& r, int n_exp, int top) {
   LLG_REQUIRE(r.score >= 0 && r.score <= 2, "%s: score kind %d is not known", what, r.score);
   LLG_REQUIRE(!r.raw || r.score != 0, "%s: undivided scores go with sigmoid or softmax-over-all scores", what);
@@ -597,24 +625,11 @@ LLG_API int llg_grouped_linear(const GroupedLinearArgs* args, int x_dtype, int y
   auto aligned = [](const void* p) { return ((uintptr_t)p & 15u) == 0; };
   if (x_dtype == LLG_BF16 && a.n_in % 8 == 0 && aligned(a.x) && aligned(a.w) && aligned(a.w2)) {
     // the tensor-core kernel: 16-byte copies need rows that start on 16-byte boundaries
-    dim3 mgrid(a.rows / LLG_MOE_TILE, (a.n_out + MM_O - 1) / MM_O);
-    LLG_REQUIRE(mgrid.y <= 65535, "grouped_linear: too many outputs");
-    const size_t smem = 2 * (size_t)(LLG_MOE_TILE * MM_LD + (gated ? 2 : 1) * MM_O * MM_LD) * sizeof(__nv_bfloat16);
-#define MMA_LAUNCH(YT, G)                                                                                         \
-  do {                                                                                                            \
-    cudaError_t err = cudaFuncSetAttribute(grouped_linear_mma_kernel<YT, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    if (err != cudaSuccess) return llg_fail("grouped_linear: shared memory %zu: %s", smem, cudaGetErrorString(err)); \
-    llg_launch(grouped_linear_mma_kernel<YT, G>, mgrid, dim3(128), smem, stream, a);                              \
-  } while (0)
-    if (y_dtype == LLG_BF16) {
-      if (gated) MMA_LAUNCH(__nv_bfloat16, true); else MMA_LAUNCH(__nv_bfloat16, false);
-    } else if (y_dtype == LLG_F32) {
-      if (gated) MMA_LAUNCH(float, true); else MMA_LAUNCH(float, false);
-    } else {
-      return llg_fail("grouped_linear: unsupported output dtype %d", y_dtype);
-    }
-#undef MMA_LAUNCH
-    return llg_check_launch("grouped_linear");
+    if (y_dtype == LLG_BF16)
+      return gated ? run_mma<__nv_bfloat16, true>("grouped_linear", a, 1, stream) : run_mma<__nv_bfloat16, false>("grouped_linear", a, 1, stream);
+    if (y_dtype == LLG_F32)
+      return gated ? run_mma<float, true>("grouped_linear", a, 1, stream) : run_mma<float, false>("grouped_linear", a, 1, stream);
+    return llg_fail("grouped_linear: unsupported output dtype %d", y_dtype);
   }
   dim3 grid(a.rows / LLG_MOE_TILE, (a.n_out + GT_O - 1) / GT_O);
   LLG_REQUIRE(grid.y <= 65535, "grouped_linear: too many outputs");
@@ -659,20 +674,9 @@ LLG_API int llg_head_linear_mma(const void* x, long long x_token_stride, long lo
   a.x_group_stride = x_head_stride;
   a.y_group_stride = y_head_stride;
   a.n_rows = n_tokens;
-  dim3 grid(a.rows / LLG_MOE_TILE, (n_out + MM_O - 1) / MM_O, nh);
-  LLG_REQUIRE(grid.y <= 65535, "head_linear: too many outputs");
-  const size_t smem = 2 * (size_t)(LLG_MOE_TILE * MM_LD + MM_O * MM_LD) * sizeof(__nv_bfloat16);
-#define HEAD_LAUNCH(YT)                                                                                                       \
-  do {                                                                                                                        \
-    cudaError_t err = cudaFuncSetAttribute(grouped_linear_mma_kernel<YT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    if (err != cudaSuccess) return llg_fail("head_linear: shared memory %zu: %s", smem, cudaGetErrorString(err));             \
-    llg_launch(grouped_linear_mma_kernel<YT, false>, grid, dim3(128), smem, stream, a);                                       \
-  } while (0)
-  if (y_dtype == LLG_BF16) HEAD_LAUNCH(__nv_bfloat16);
-  else if (y_dtype == LLG_F32) HEAD_LAUNCH(float);
-  else return llg_fail("head_linear: unknown output type %d", y_dtype);
-#undef HEAD_LAUNCH
-  return llg_check_launch("head_linear");
+  if (y_dtype == LLG_BF16) return run_mma<__nv_bfloat16, false>("head_linear", a, nh, stream);
+  if (y_dtype == LLG_F32) return run_mma<float, false>("head_linear", a, nh, stream);
+  return llg_fail("head_linear: unknown output type %d", y_dtype);
 }
 
 LLG_API int llg_moe_gather_rows(const void* x, const int* token_of_row, void* out, int rows, int row_bytes, cudaStream_t stream) {

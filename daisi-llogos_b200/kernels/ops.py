@@ -435,6 +435,8 @@ def _load_lib(name: str):
         lib.llg_gemm_tc_qkv.argtypes = [c_void_p, c_void_p, c_int, c_int, POINTER(_QkPrepArgs), c_void_p]
         lib.llg_gemm_tc_gate_form.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                               POINTER(_GateForm), POINTER(_RowScale), c_void_p]
+        lib.llg_gemm_tc_grouped_few.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
+                                                c_int, POINTER(_GateForm), c_void_p, c_void_p]
         lib.llg_gemm_tc_grouped.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int,
                                             c_int, POINTER(_GateForm), c_void_p, c_void_p]
         lib.llg_gemm_tc_act.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
@@ -1534,6 +1536,32 @@ def _grouped_tc(x, tile_expert, w, out, gated_features: int, form: Optional[Gate
                                         byref(form.c) if form is not None else None, _ptr(row_weight, torch.float32), _stream()))
 
 
+# Steps of at most this many tokens run their experts' gated product as a stream on tcgen05: every tile multiplies with all of the
+# step's tokens.  Eight tokens, 16 experts of 1,024 x 2,048 (14 in use): 26.4 us (4.4 TB/s) against 36 to 57 of the mma.sync kernel's
+# shapes; 1,792 x 4,096: 82 against 88 to 110.  The down product runs there at any number of tokens in tiles of 32 rows: 13.1 us
+# against 21.1 to 27 at eight tokens, 15.6 against 21.7 at 100, 27.4 against 50.5 at 400.
+GROUPED_FEW_TOKENS = 32
+
+
+def _few_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
+    return (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and x.data_ptr() % 16 == 0
+            and w.data_ptr() % 16 == 0)
+
+
+def _grouped_few(x, tile_expert, token_of_row, w, out, gated_features: int, form: Optional[GateForm] = None,
+                 row_weight: Optional[torch.Tensor] = None) -> None:
+    lib = _lib("gemm_tc")
+    rows = out.shape[0]
+    n_groups, group_rows, k = w.shape
+    assert x.shape[1] == k and tile_expert.numel() * MOE_TILE_ROWS == rows and (token_of_row is None or token_of_row.numel() == rows)
+    assert out.shape[1] == (gated_features or group_rows)
+    _check(lib, lib.llg_gemm_tc_grouped_few(_ptr(x, torch.bfloat16), x.shape[0], _ptr(w, torch.bfloat16),
+                                            _ptr(out, torch.bfloat16 if gated_features else torch.float32), rows, group_rows, k,
+                                            gated_features, _ptr(tile_expert, torch.int32), _ptr(token_of_row, torch.int32), n_groups,
+                                            group_rows, byref(form.c) if form is not None else None, _ptr(row_weight, torch.float32),
+                                            _stream()))
+
+
 def _grouped(x, token_of_row, tile_expert, w, w2_offset, n_out, y, form: GateForm = SILU_FORM, row_weight=None) -> None:
     """The kernels of csrc/moe.cu: ``w`` ``[E, rows per expert, n_in]``, of which the first ``n_out`` rows of an expert are the
     (first) matrix and, with ``w2_offset``, the rows from there on the second."""
@@ -1571,6 +1599,9 @@ def moe_gated(x: torch.Tensor, token_of_row: Optional[torch.Tensor], tile_expert
             raise KernelError("moe_gated: tiles of 128 rows take the gathered rows")
         _grouped_tc(x, tile_expert, w_gate_up, act, inner, form, row_weight)
         return
+    if token_of_row is not None and 0 < x.shape[0] <= GROUPED_FEW_TOKENS and act.dtype == torch.bfloat16 and _few_supported(x, w_gate_up):
+        _grouped_few(x, tile_expert, token_of_row, w_gate_up, act, inner, form, row_weight)
+        return
     _grouped(x, token_of_row, tile_expert, w_gate_up, pad, inner, act, form or SILU_FORM, row_weight)
 
 
@@ -1580,6 +1611,9 @@ def moe_down(act: torch.Tensor, tile_expert: torch.Tensor, w_down: torch.Tensor,
         raise KernelError("moe_down: the experts' outputs are float32")
     if _tile_of(y.shape[0], tile_expert) == MOE_TC_TILE_ROWS:
         _grouped_tc(act, tile_expert, w_down, y, 0)
+        return
+    if act.shape[0] > 0 and _few_supported(act, w_down):
+        _grouped_few(act, tile_expert, None, w_down, y, 0)
         return
     _grouped(act, None, tile_expert, w_down, None, w_down.shape[1], y)
 
