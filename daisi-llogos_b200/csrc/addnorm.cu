@@ -43,14 +43,19 @@ template <int VEC> __device__ __forceinline__ void store(__nv_bfloat16* p, const
 }
 
 // VEC 4: every access moves four neighbouring elements (the host has checked sizes and addresses).  A term's partial sums
-// are fetched four sets at a time, so that the few rows of a decode step do not wait for one load after another.
+// are fetched eight sets at a time, so that the few rows of a decode step do not wait for one load after another.
 template <typename OT, int VEC>
 __global__ void __launch_bounds__(1024) multi_add_rmsnorm_kernel(AddNormArgs a) {
   pdl_launch_dependents();
-  pdl_wait();
   extern __shared__ __align__(16) float smem[];
   __shared__ float part[32];
   const int hidden = a.hidden;
+  // the weights of the elements that a thread meets first (all it has, in a decode step) are there when a sum is
+  Pack<VEC> out_w[LLG_ADDNORM_OUTS], norm_w;
+#pragma unroll
+  for (int o = 0; o < LLG_ADDNORM_OUTS; ++o)
+    if (o < a.n_outs && a.outs[o].weight && threadIdx.x * VEC < hidden) out_w[o] = load_f32<VEC>(a.outs[o].weight + threadIdx.x * VEC);
+  pdl_wait();
   float* row = smem;
   float* tmp = smem + hidden;
   const int j = blockIdx.x;
@@ -62,20 +67,15 @@ __global__ void __launch_bounds__(1024) multi_add_rmsnorm_kernel(AddNormArgs a) 
   for (int t = 0; t < a.n_terms; ++t) {
     const AddNormTerm& term = a.terms[t];
     const float* p = term.data + (long long)r * hidden;
+    if (term.norm_w && first < hidden) norm_w = load_f32<VEC>(term.norm_w + first);
     float ss = 0.f;
     for (int i = first; i < hidden; i += stride) {
-      Pack<VEC> y = load_f32<VEC>(p + i);
-      int s = 1;
-      for (; s + 3 < term.n_partials; s += 4) {
-        const Pack<VEC> y0 = load_f32<VEC>(p + s * a.partial_stride + i), y1 = load_f32<VEC>(p + (s + 1) * a.partial_stride + i);
-        const Pack<VEC> y2 = load_f32<VEC>(p + (s + 2) * a.partial_stride + i), y3 = load_f32<VEC>(p + (s + 3) * a.partial_stride + i);
-#pragma unroll
-        for (int c = 0; c < VEC; ++c) y.v[c] = (((y.v[c] + y0.v[c]) + y1.v[c]) + y2.v[c]) + y3.v[c];
-      }
-      for (; s < term.n_partials; ++s) {
-        const Pack<VEC> y0 = load_f32<VEC>(p + s * a.partial_stride + i);
-#pragma unroll
-        for (int c = 0; c < VEC; ++c) y.v[c] += y0.v[c];
+      Pack<VEC> y;
+      if (VEC == 4) {
+        const float4 t4 = sum_partials(reinterpret_cast<const float4*>(p + i), a.partial_stride / 4, term.n_partials);
+        y.v[0] = t4.x; y.v[VEC > 1 ? 1 : 0] = t4.y; y.v[VEC > 2 ? 2 : 0] = t4.z; y.v[VEC > 3 ? 3 : 0] = t4.w;
+      } else {
+        y.v[0] = sum_partials(p + i, a.partial_stride, term.n_partials);
       }
       if (term.norm_w) {
         store<VEC>(tmp + i, y);
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(1024) multi_add_rmsnorm_kernel(AddNormArgs a) 
       const float inv = 1.0f / sqrtf(ss / (float)hidden + term.norm_eps);
       for (int i = first; i < hidden; i += stride) {
         Pack<VEC> v = load_f32<VEC>(row + i);
-        const Pack<VEC> y = load_f32<VEC>(tmp + i), w = load_f32<VEC>(term.norm_w + i);
+        const Pack<VEC> y = load_f32<VEC>(tmp + i), w = i == first ? norm_w : load_f32<VEC>(term.norm_w + i);
 #pragma unroll
         for (int c = 0; c < VEC; ++c) v.v[c] += term.scale * (y.v[c] * inv * w.v[c]);
         store<VEC>(row + i, v);
@@ -114,14 +114,16 @@ __global__ void __launch_bounds__(1024) multi_add_rmsnorm_kernel(AddNormArgs a) 
     ss = block_sum(ss, part);
     inv = 1.0f / sqrtf(ss / (float)hidden + a.eps);
   }
-  for (int o = 0; o < a.n_outs; ++o) {
+#pragma unroll
+  for (int o = 0; o < LLG_ADDNORM_OUTS; ++o) {
+    if (o >= a.n_outs) break;
     OT* out = (OT*)a.outs[o].out + (long long)j * hidden;
     const float* w = a.outs[o].weight;
     const float off = a.outs[o].offset;
     for (int i = first; i < hidden; i += stride) {
       Pack<VEC> v = load_f32<VEC>(row + i);
       if (w) {
-        const Pack<VEC> ww = load_f32<VEC>(w + i);
+        const Pack<VEC> ww = i == first ? out_w[o] : load_f32<VEC>(w + i);
 #pragma unroll
         for (int c = 0; c < VEC; ++c) v.v[c] = v.v[c] * inv * (off + ww.v[c]);
       }

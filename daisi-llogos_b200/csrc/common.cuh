@@ -191,6 +191,31 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
   return t;
 }
 
+// The sum of n partial sums that lie `stride` elements apart, added in their order.  Eight are asked for before the first is added:
+// the few rows of a decode step have nothing else to hide a trip to L2 behind, and a loop that adds them one by one makes a
+// trip each.
+__device__ __forceinline__ float sum_partials(const float* p, long long stride, int n, float y = 0.f) {
+  for (int s0 = 0; s0 < n; s0 += 8) {
+    float t[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) t[q] = s0 + q < n ? p[(s0 + q) * stride] : 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) y += t[q];
+  }
+  return y;
+}
+__device__ __forceinline__ float4 sum_partials(const float4* p, long long stride, int n) {
+  float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s0 = 0; s0 < n; s0 += 8) {
+    float4 t[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) t[q] = s0 + q < n ? p[(s0 + q) * stride] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) { y.x += t[q].x; y.y += t[q].y; y.z += t[q].z; y.w += t[q].w; }
+  }
+  return y;
+}
+
 // Row of the paged key/value store that holds position `pos` of the sequence in `slot`,
 // for key/value head `kvh`.  Pages are [n_pages][n_kv][LLG_PAGE][head_dim]; a sequence's
 // logical page j lies at table[slot][j % ring_pages] (ring_pages = table width for a group

@@ -25,6 +25,7 @@ __global__ void embed_rows_kernel(const TT* __restrict__ table, const int* __res
   if (id < 0 || id >= vocab) id = 0;  // ids are validated on the host; never read out of range
   const TT* row = table + (long long)id * hidden;
   float* o = out + (long long)n * hidden;
+#pragma unroll 4
   for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
     const float v = to_f32(row[i]);
     for (int c = 0; c < copies; ++c) o[c * copy_stride + i] = v;
@@ -39,7 +40,7 @@ LLG_API int llg_embed_rows_copies(const void* table, int table_dtype, const int*
   LLG_REQUIRE(n_tokens >= 0 && hidden > 0 && vocab > 0 && copies >= 1, "embed_rows: bad sizes n=%d hidden=%d vocab=%d copies=%d",
               n_tokens, hidden, vocab, copies);
   if (n_tokens == 0) return 0;
-  const int threads = hidden >= 1024 ? 256 : 128;
+  const int threads = hidden >= 2048 && n_tokens <= 64 ? 1024 : hidden >= 1024 ? 256 : 128;      // few rows: a trip to memory or two
   if (table_dtype == LLG_F32)
     llg_launch(embed_rows_kernel<float>, n_tokens, threads, 0, stream, (const float*)table, ids, out, hidden, vocab, copies, copy_stride);
   else if (table_dtype == LLG_BF16)
@@ -342,7 +343,7 @@ LLG_API int llg_add_rmsnorm(float* residual, const float* branch, int n_partials
   if (vec) {
     const int nv = hidden / 4;
     if (n_out <= 256) {
-      threads = nv >= 1024 ? 1024 : (nv >= 256 ? 256 : 128);
+      threads = nv >= 1024 ? 1024 : (nv >= 512 ? 512 : (nv >= 256 ? 256 : 128));
     } else {
       threads = nv >= 1024 ? 512 : 256;
     }
@@ -1031,8 +1032,9 @@ __global__ void hc_add_rmsnorm_kernel(HyperNormArgs a) {
 // The same for rows whose length is a multiple of 4 and 16-byte aligned operands: 16-byte accesses, the read-out stays in
 // registers between the two passes (VPT float4 per thread), and the partial sums of an element are asked for together.
 // SMAX: the most streams an instance holds (its register arrays have that size).
-template <typename OT, typename WT, int VPT, int SMAX>
-__global__ void __launch_bounds__(512) hc_add_rmsnorm_vec4_kernel(HyperNormArgs a) {
+// MAXT: threads of the largest block; a decode step's row of 4,096 with two streams is one float4 a thread of 1,024.
+template <typename OT, typename WT, int VPT, int SMAX, int MAXT = 512>
+__global__ void __launch_bounds__(MAXT) hc_add_rmsnorm_vec4_kernel(HyperNormArgs a) {
   pdl_launch_dependents();
   __shared__ float red[32];
   __shared__ float c_mix[HC_MAX * HC_MAX], c_write[HC_MAX], c_read[HC_MAX];
@@ -1067,19 +1069,7 @@ __global__ void __launch_bounds__(512) hc_add_rmsnorm_vec4_kernel(HyperNormArgs 
       for (int s = 0; s < SMAX; ++s) x[s] = s < S ? base[s * ss4 + i] : make_float4(0.f, 0.f, 0.f, 0.f);
       if (a.branch) {
         const float4* b = reinterpret_cast<const float4*>(a.branch + (long long)r * a.hidden) + i;
-        float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
-        int p = 0;
-        for (; p + 4 <= a.n_partials; p += 4) {
-          const float4 b0 = b[(p + 0) * ps4], b1 = b[(p + 1) * ps4], b2 = b[(p + 2) * ps4], b3 = b[(p + 3) * ps4];
-          y.x += b0.x; y.y += b0.y; y.z += b0.z; y.w += b0.w;
-          y.x += b1.x; y.y += b1.y; y.z += b1.z; y.w += b1.w;
-          y.x += b2.x; y.y += b2.y; y.z += b2.z; y.w += b2.w;
-          y.x += b3.x; y.y += b3.y; y.z += b3.z; y.w += b3.w;
-        }
-        for (; p < a.n_partials; ++p) {
-          const float4 b0 = b[p * ps4];
-          y.x += b0.x; y.y += b0.y; y.z += b0.z; y.w += b0.w;
-        }
+        const float4 y = sum_partials(b, ps4, a.n_partials);
         float4 nx[SMAX];
 #pragma unroll
         for (int t = 0; t < SMAX; ++t) {
@@ -1147,6 +1137,7 @@ LLG_API int llg_hc_add_rmsnorm(const HyperNormArgs* args, cudaStream_t stream) {
     const int nv = a.hidden / 4;
     // (at most 512 threads: a thread holds S float4 of the streams beside its part of the read-out)
     threads = a.n_out <= 256 ? (nv >= 512 ? 512 : (nv >= 256 ? 256 : 128)) : (nv >= 1024 ? 512 : 256);
+    if (a.n_out <= 64 && nv > 512 && nv <= 1024 && a.n_streams <= 2) threads = 1024;
     vpt = (nv + threads - 1) / threads;
     if (vpt > 4) {
       threads = 512;
@@ -1156,7 +1147,8 @@ LLG_API int llg_hc_add_rmsnorm(const HyperNormArgs* args, cudaStream_t stream) {
   const bool vec_ok = vec && vpt <= 4 && a.n_streams <= HC_VEC_MAX;
 #define LAUNCH_V(OT, WT, SM)                                                                                        \
   do {                                                                                                              \
-    if (vpt <= 1) llg_launch(hc_add_rmsnorm_vec4_kernel<OT, WT, 1, SM>, a.n_out, threads, 0, stream, a);            \
+    if (threads > 512) llg_launch(hc_add_rmsnorm_vec4_kernel<OT, WT, 1, 2, 1024>, a.n_out, threads, 0, stream, a);  \
+    else if (vpt <= 1) llg_launch(hc_add_rmsnorm_vec4_kernel<OT, WT, 1, SM>, a.n_out, threads, 0, stream, a);       \
     else if (vpt <= 2) llg_launch(hc_add_rmsnorm_vec4_kernel<OT, WT, 2, SM>, a.n_out, threads, 0, stream, a);       \
     else llg_launch(hc_add_rmsnorm_vec4_kernel<OT, WT, 4, SM>, a.n_out, threads, 0, stream, a);                     \
   } while (0)
@@ -1267,11 +1259,7 @@ __global__ void qkv_row_prep_vec4_kernel(QkvRowPrepArgs a) {
   float ss_q = 0.f, ss_k = 0.f;
   for (int i4 = threadIdx.x; i4 < W4; i4 += blockDim.x) {
     const int i = i4 << 2;
-    float4 v = src[i4];
-    for (int p = 1; p < a.n_partials; ++p) {
-      const float4 t = src[p * ps4 + i4];
-      v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
-    }
+    float4 v = sum_partials(src + i4, ps4, a.n_partials);
     if (bias && i < Q + K + V) {
       float b[4];
       vec_load4(bias + i, b);

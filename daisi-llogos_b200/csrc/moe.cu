@@ -188,9 +188,7 @@ __global__ void __launch_bounds__(128) moe_topk_kernel(const float* __restrict__
   const int width = n_exp + (extra ? 1 : 0);
   float* z = sm + warp * ((rule.correction ? 3 : 2) * n_exp + 1);
   for (int e = lane; e < width; e += 32) {
-    float v = bias && e < n_exp ? bias[e] : 0.f;
-    for (int s = 0; s < n_partials; ++s) v += logits[s * partial_stride + (long long)n * width + e];
-    z[e] = v;
+    z[e] = sum_partials(logits + (long long)n * width + e, partial_stride, n_partials, bias && e < n_exp ? bias[e] : 0.f);
   }
   __syncwarp();
   if (extra && lane == 0) extra[n] = 1.0f / (1.0f + expf(-z[n_exp]));

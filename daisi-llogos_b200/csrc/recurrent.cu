@@ -176,10 +176,7 @@ __global__ void __launch_bounds__(128) causal_conv_kernel(ConvArgs a) {
   float w[LLG_CONV_MAX_TAPS];
   for (int j = 0; j < K; ++j) w[j] = a.weight[(long long)c * K + j];
   auto input = [&](int q) {                        // the input at step token q of this sequence
-    const float* r = a.rows + (long long)(t0 + q) * a.row_width + a.col0 + c;
-    float v = r[0];
-    for (int s = 1; s < a.n_partials; ++s) v += r[s * a.partial_stride];
-    return v + ib;
+    return sum_partials(a.rows + (long long)(t0 + q) * a.row_width + a.col0 + c, a.partial_stride, a.n_partials) + ib;
   };
   O2* out2 = (O2*)a.out2;
   auto put = [&](int token, float v) {
