@@ -92,6 +92,9 @@ __device__ __forceinline__ float both(pair_t v) { return __uint_as_float((unsign
 // feature group share k.  Bound by the weight stream: a float4 of weights is used for NR products of four, and the rows'
 // float4s come from the first-level cache once per F features, so F x NR = 32 keeps the CUDA cores and that cache below
 // half of what the memory's rate asks of them.  The weights of the first group do not wait for the kernel before.
+// 16,384 x 2,048: 23.5 us for one row (5.7 TB/s), 28.4 for three (4.7), 36.5 for eight (3.7; there the cores bound it); 128,256 x
+// 2,048 at three rows 169 us (6.2 TB/s).  gemm_tn_kernel, which took these before, pays for 64 rows: 618 us on average over a 1B
+// model's products.
 template <int NR, int F>
 __global__ void __launch_bounds__(256, 2) gemv_rows_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                         float* __restrict__ out, int n, int o, int k, int wk, RowScale scale) {
@@ -175,9 +178,9 @@ __global__ void __launch_bounds__(256, 2) gemv_rows_kernel(const float* __restri
 // More rows (a prompt step): tiles of 64 rows x 128 features, 256 threads with 8 x 4 sums each.  Both operands arrive by
 // cp.async as they lie in memory, 32 k of a row at a time, in a ring of three stages: a stage is 24 KB, so that one block a
 // multiprocessor already has the bytes in flight that the memory's latency asks for (with the next stage in registers and
-// half as much a step a block waited 2 us a step: 38 us at 64 x 2,048 x 2,048; now TILE_NOW).  Rows are padded to 36 floats: 16-byte
-// reads of consecutive rows at one k fall into different banks.  A thread takes four k at a time, 16 reads for 256
-// multiply-adds.  Bound by the multiply-add pipes from 150 rows on.  Where a shape has few tiles, the blocks of a cluster
+// half as much a step a block waited 2 us a step: 100 x 2,048 x 2,048 81.5 us before, 38.6 now).  Rows are padded to 36 floats: 16-byte
+// reads of consecutive rows at one k fall into different banks.  A thread takes four k at a time, 12 reads for 128
+// multiply-adds.  From 300 rows on the multiply-add pipes (two thirds busy) and the 16-byte shared reads bound it: 38 TFLOP/s.  Where a shape has few tiles, the blocks of a cluster
 // share the tile's k and add their sums through distributed shared memory, in the order of the ranks.
 constexpr int TM = 64, TF = 128, TK = 32, TLD = TK + 4, TSTAGES = 3;
 constexpr int TILE_SMEM = TSTAGES * (TM + TF) * TLD * (int)sizeof(float);
@@ -351,7 +354,9 @@ int run_tile(const float* x, const float* w, float* out, int n, int o, int k, co
   return llg_check_launch("gemm_simt");
 }
 
-constexpr int GEMV_ROWS_MAX = 32;     // rows up to which the weight stream is taken
+// Rows up to which the weight stream is taken: at 32 rows of 2,048 x 2,048 it takes 21 us and the tiles 38, at 40 rows 27 and 38, but
+// at 2,048 x 16,384 the tiles are even from 40 on (142 us both).
+constexpr int GEMV_ROWS_MAX = 32;
 
 }  // namespace
 

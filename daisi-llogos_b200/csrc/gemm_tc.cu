@@ -762,8 +762,9 @@ __device__ __forceinline__ void mbar_arrive_first(uint64_t* bar) {      // arriv
       ::"r"(smem_u32(bar))
       : "memory");
 }
+// (not the .aligned form: one lane of a warp comes from its role's loop, and nothing promises that the warp is whole again)
 __device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
 template <int TN, typename OT, int EPI>
@@ -819,7 +820,6 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_pair_kernel(const __grid_co
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncwarp();
   __syncthreads();
   cluster_barrier();                                      // the other block's barriers and tensor memory are there
   // only now: a block of a later kernel that came to this multiprocessor first could take tensor memory and then wait for us
@@ -908,7 +908,8 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_pair_kernel(const __grid_co
       const int b = round % NACC;
       const bool have = mbar_wait(&acc_full[b], (round / NACC) & 1, abortp);
       if (!have && !*abortp) { *abortp = 1; atomicCAS(&g_error, 0, 3); }
-      if (!have || *abortp) break;
+      // one answer for the warp: reading tensor memory wants all of its lanes
+      if (__any_sync(0xffffffffu, !have || *abortp)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int o0 = token0(tile);
       if (o0 < p.o)                                       // uniform over the block: the pair's second half may lie past the tokens
@@ -924,6 +925,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_pair_kernel(const __grid_co
   __syncthreads();
   cluster_barrier();                                      // nobody leaves while the other's products, copies or arrivals may come
   if (warp == MMA_WARP) {
+    __syncwarp();                                         // the next instruction wants the whole warp
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"((uint32_t)(NACC * ACC_COLS)) : "memory");
   }
 }
