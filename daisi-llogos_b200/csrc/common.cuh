@@ -204,8 +204,7 @@ __device__ __forceinline__ float sum_partials(const float* p, long long stride, 
   }
   return y;
 }
-__device__ __forceinline__ float4 sum_partials(const float4* p, long long stride, int n) {
-  float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+__device__ __forceinline__ float4 sum_partials(const float4* p, long long stride, int n, float4 y = make_float4(0.f, 0.f, 0.f, 0.f)) {
   for (int s0 = 0; s0 < n; s0 += 8) {
     float4 t[8];
 #pragma unroll

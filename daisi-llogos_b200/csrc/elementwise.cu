@@ -155,7 +155,6 @@ __global__ void add_rmsnorm_vec4_kernel(float* __restrict__ residual, const floa
         }
         const float4* b = reinterpret_cast<const float4*>(branch + (long long)r * hidden) + i;
         const long long ps = partial_stride >> 2;
-        int s = 0;
         if (VPT == 1) {
           // few rows (one float4 a thread): nothing to hide a load behind, so the first twelve partials are all asked
           // for before the first is added (one trip to L2 instead of one per group); they are added in their order
@@ -166,18 +165,9 @@ __global__ void add_rmsnorm_vec4_kernel(float* __restrict__ residual, const floa
 #pragma unroll
           for (int q = 0; q < AT_ONCE; ++q)
             if (q < n_partials) { v.x += pv[q].x; v.y += pv[q].y; v.z += pv[q].z; v.w += pv[q].w; }
-          s = n_partials < AT_ONCE ? n_partials : AT_ONCE;
-        }
-        for (; s + 4 <= n_partials; s += 4) {
-          const float4 b0 = b[(s + 0) * ps], b1 = b[(s + 1) * ps], b2 = b[(s + 2) * ps], b3 = b[(s + 3) * ps];
-          v.x += b0.x; v.y += b0.y; v.z += b0.z; v.w += b0.w;
-          v.x += b1.x; v.y += b1.y; v.z += b1.z; v.w += b1.w;
-          v.x += b2.x; v.y += b2.y; v.z += b2.z; v.w += b2.w;
-          v.x += b3.x; v.y += b3.y; v.z += b3.z; v.w += b3.w;
-        }
-        for (; s < n_partials; ++s) {
-          const float4 b0 = b[s * ps];
-          v.x += b0.x; v.y += b0.y; v.z += b0.z; v.w += b0.w;
+          if (n_partials > AT_ONCE) v = sum_partials(b + AT_ONCE * ps, ps, n_partials - AT_ONCE, v);
+        } else {
+          v = sum_partials(b, ps, n_partials, v);
         }
         res[i] = v;
       }
@@ -201,15 +191,16 @@ __global__ void add_rmsnorm_vec4_kernel(float* __restrict__ residual, const floa
   if (threadIdx.x == 0) LLG_STAMP(3, 3, 0, blockIdx.x);
 }
 
-// The same for the many rows of a prompt step, whose branch is one sum (or none): a row is 256 threads' work and everything that
-// memory has to give, VPT float4 of the residual stream and of the branch a thread, is asked for before the first is used; the
-// weights, which stay in the caches, come last.  With the general form's loop over partials between the loads a thread had one
+// The same for the many rows of a prompt step: a row is 256 threads' work and everything that
+// memory has to give, VPT float4 of the residual stream and of one partial sum of the branch a thread, is asked for before the first
+// is used; the weights, which stay in the caches, come last.  With the general form's loop over partials between the loads a thread had one
 // float4 of each under way at a time.  Bound by memory: 26,600 rows of 5,120 1.14 ms before, 0.32 now (1.9 GB); 2,048 rows of 4,096
 // 23 us before, 16 now.
 constexpr int ROWS_THREADS = 256;
 
 template <typename OT, typename WT, int VPT>
 __global__ void __launch_bounds__(ROWS_THREADS) add_rmsnorm_rows_kernel(float* __restrict__ residual, const float* __restrict__ branch,
+                                                                        int n_partials, long long partial_stride,
                                                                         const WT* __restrict__ weight, float eps, OT* __restrict__ out,
                                                                         const int* __restrict__ rows, int hidden,
                                                                         float* __restrict__ ss_out, const float* __restrict__ branch_bias) {
@@ -240,6 +231,20 @@ __global__ void __launch_bounds__(ROWS_THREADS) add_rmsnorm_rows_kernel(float* _
           const float4 bb = reinterpret_cast<const float4*>(branch_bias)[i];
           v[k].x += bb.x; v[k].y += bb.y; v[k].z += bb.z; v[k].w += bb.w;
         }
+      }
+    }
+#pragma unroll 1
+    for (int s = 1; s < n_partials; ++s) {               // the next partial is on its way while this one is added
+      float4 next[VPT];
+#pragma unroll
+      for (int k = 0; k < VPT; ++k) {
+        const int i = threadIdx.x + k * ROWS_THREADS;
+        next[k] = i < nv ? __ldcs(b + s * (partial_stride >> 2) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int k = 0; k < VPT; ++k) {
+        v[k].x += add[k].x; v[k].y += add[k].y; v[k].z += add[k].z; v[k].w += add[k].w;
+        add[k] = next[k];
       }
     }
 #pragma unroll
@@ -354,13 +359,13 @@ LLG_API int llg_add_rmsnorm(float* residual, const float* branch, int n_partials
     }
   }
   const bool vec_ok = vec && vpt <= 8;
-  // a prompt step's rows, one sum to add: up to eight float4 a thread (above, the threads would hold too much)
-  const int rows_vpt = vec && n_out > 256 && n_partials <= 1 ? (hidden / 4 + ROWS_THREADS - 1) / ROWS_THREADS : 0;
+  // a prompt step's rows: up to eight float4 a thread (above, the threads would hold too much)
+  const int rows_vpt = vec && n_out > 256 ? (hidden / 4 + ROWS_THREADS - 1) / ROWS_THREADS : 0;
   // the division left to the consumer and few rows: every slice of a row is a block of its own
   const int parts = ss_out ? llg_add_rmsnorm_parts(n_out, hidden) : 1;
   LLG_REQUIRE(parts == 1 || vec, "add_rmsnorm: operands of a norm in parts must be 16-byte aligned");
 #define ROWS(OT, WT, V)                                                                                        \
-  llg_launch(add_rmsnorm_rows_kernel<OT, WT, V>, n_out, ROWS_THREADS, 0, stream, residual, branch, (const WT*)weight, eps, (OT*)out, \
+  llg_launch(add_rmsnorm_rows_kernel<OT, WT, V>, n_out, ROWS_THREADS, 0, stream, residual, branch, n_partials, partial_stride, (const WT*)weight, eps, (OT*)out, \
              rows, hidden, ss_out, branch_bias)
 #define LAUNCH(OT, WT)                                                                                         \
   do {                                                                                                         \

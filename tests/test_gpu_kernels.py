@@ -100,11 +100,11 @@ def test_gemm_simt(ops, xd, wd, od, n, o, k):
 @pytest.mark.parametrize("hidden", [4, 1024, 1028, 2048, 3000, 4096, 5120, 6144, 6148, 8192, 8196])
 @pytest.mark.parametrize("dtype", DTYPES, ids=IDS)
 def test_add_rmsnorm_of_many_rows(ops, dtype, hidden):
-    """More than 256 rows with one sum to add, none, and a bias beside it; rows of one to eight float4 a thread and longer ones."""
+    """More than 256 rows with one sum to add, none, a bias beside it, and three sums; rows of one to eight float4 a thread and longer ones."""
     n, eps = 260, 1e-5
     w, res, branch, bias = rnd((hidden,), 3, dtype).abs() + 0.5, rnd((n, hidden), 4), rnd((1, n, hidden), 5), rnd((hidden,), 6)
-    for b, bb in ((None, None), (branch, None), (branch, bias)):
-        total = res.double() + (0 if b is None else b[0].double()) + (0 if bb is None else bb.double())
+    for b, bb in ((None, None), (branch, None), (branch, bias), (rnd((3, n, hidden), 7), bias)):
+        total = res.double() + (0 if b is None else b.double().sum(0)) + (0 if bb is None else bb.double())
         kw = {} if bb is None else {"branch_bias": bb.to(DEV)}
         r, out = res.to(DEV).clone(), torch.empty(n, hidden, dtype=dtype, device=DEV)
         ops.add_rmsnorm(r, None if b is None else b.to(DEV), w.to(DEV), eps, out, **kw)
