@@ -327,6 +327,7 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
+    warp_whole();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)),
                  "r"((uint32_t)TMEM_COLS)
                  : "memory");
@@ -384,10 +385,9 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
     int requested = 0;                          // tiles whose copies have been requested
     for (int t = 0; t < ti.n_max; ++t) {
       const int st = t % stages;
-      if (t >= stages && !mbar_wait(&freeb[st], (t / stages - 1) & 1, abortp)) {
-        if (!*abortp) { *abortp = 1; atomicCAS(&g_error, 0, 4); }
-        break;
-      }
+      const bool left = t < stages || mbar_wait(&freeb[st], (t / stages - 1) & 1, abortp);
+      if (!left && !*abortp) { *abortp = 1; atomicCAS(&g_error, 0, 4); }
+      if (!warp_all(left)) break;          // one answer for the warp: its lanes meet again below
       requested = t + 1;
       const int kt = ti.k_begin + t * TK;
       const uint32_t dst = smem_u32(base + st * KV_BYTES);
@@ -548,11 +548,10 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
     float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     for (int j = 0; j < n_tiles; ++j) {
-      if (!mbar_wait(&s_full[g][j & 1], (j >> 1) & 1, abortp)) {
-        if (!*abortp) { *abortp = 1; atomicCAS(&g_error, 0, 1); }
-        ok = false;
-        break;
-      }
+      const bool scored = mbar_wait(&s_full[g][j & 1], (j >> 1) & 1, abortp);
+      if (!scored && !*abortp) { *abortp = 1; atomicCAS(&g_error, 0, 1); }
+      ok = warp_all(scored);
+      if (!ok) break;                      // uniform: one answer for the warp, tensor memory's instructions want all of its lanes
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int kt = ti.k_begin + (split ? 2 * j + g : j) * TK;
       float sv[TK];
@@ -599,11 +598,12 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
       const float2 sc2 = make_float2(sc, sc), nms2 = make_float2(-ms, -ms);
       float2 ps2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       // P(j) takes the place of S(j) in tensor memory: 64 weights of a row in 32 columns
+      warp_whole();
 #pragma unroll
-      for (int c16 = 0; c16 < TK / 32; ++c16) {
+      for (int c16 = 0; c16 < TK / 32; ++c16) {        // uniform
         uint32_t pk[16];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
+        for (int e = 0; e < 16; ++e) {                 // uniform
           const float2 x = __ffma2_rn(make_float2(sv[c16 * 32 + 2 * e], sv[c16 * 32 + 2 * e + 1]), sc2, nms2);
           const float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
           ps2[e & 1] = __fadd2_rn(ps2[e & 1], p);
@@ -615,15 +615,14 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
 
       if (j > 0) {
         // O += P(j-1) V(j-1) has finished: the accumulator may be rescaled
-        if (!mbar_wait(&o_done[g], (j - 1) & 1, abortp)) {
-          if (!*abortp) { *abortp = 1; atomicCAS(&g_error, 0, 2); }
-          ok = false;
-          break;
-        }
+        const bool added = mbar_wait(&o_done[g], (j - 1) & 1, abortp);
+        if (!added && !*abortp) { *abortp = 1; atomicCAS(&g_error, 0, 2); }
+        ok = warp_all(added);
+        if (!ok) break;                                // uniform
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (__any_sync(0xffffffffu, corr != 1.f)) {
+        if (!warp_all(corr == 1.f)) {
 #pragma unroll
-          for (int c0 = 0; c0 < HD; c0 += 16) {
+          for (int c0 = 0; c0 < HD; c0 += 16) {        // uniform
             uint32_t rr[16];
             tmem_ld16(lane_base + O_COL + c0, rr);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -637,9 +636,10 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       mbar_arrive(&p_ready[g][j & 1]);
     }
-    if (ok && !mbar_wait(&o_done[g], (n_tiles - 1) & 1, abortp)) {
-      if (!*abortp) { *abortp = 1; atomicCAS(&g_error, 0, 2); }
-      ok = false;
+    if (ok) {
+      const bool added = mbar_wait(&o_done[g], (n_tiles - 1) & 1, abortp);
+      if (!added && !*abortp) { *abortp = 1; atomicCAS(&g_error, 0, 2); }
+      ok = warp_all(added);
     }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (MAPS) {
@@ -656,6 +656,7 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
 #pragma unroll
         for (int c0 = 0; c0 < HD / 2; c0 += 16) {
           uint32_t r1[16], r2[16];
+          warp_whole();
           tmem_ld16(row + c0, r1);
           tmem_ld16(row + G_COLS + c0, r2);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -703,6 +704,7 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
 #pragma unroll
         for (int c0 = 0; c0 < HD / 2; c0 += 16) {
           uint32_t r0_[16], r1_[16];
+          warp_whole();                                   // (the last columns' stores are those of the queries that there are)
           tmem_ld16(row + c0, r0_);
           tmem_ld16(row + G_COLS + c0, r1_);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -718,7 +720,7 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
           }
         }
       }
-    } else if (ok && !*abortp) {
+    } else if (warp_all(ok && !*abortp)) {
       const int head = h + (mode == TWO_HEADS ? g : 0);
       // a sink joins the sum with its own weight 2^(sink - M) and carries no value; a gate scales the head's output
       if (a.has_sink) l_run += fast_exp2((a.sinks ? a.sinks[head] : a.sink_score) * LOG2E - m_run);
@@ -728,6 +730,7 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
 #pragma unroll
       for (int c0 = 0; c0 < HD; c0 += 16) {
         uint32_t rr[16];
+        warp_whole();                                     // (the last columns' stores are those of the queries that there are)
         tmem_ld16(lane_base + O_COL + c0, rr);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (r < ti.nq[g]) {
@@ -752,6 +755,7 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
   __syncthreads();
   if (tid == 0) LLG_STAMP(5, 3, 0, blockIdx.x + gridDim.x * blockIdx.y);
   if (warp == 1) {
+    warp_whole();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)TMEM_COLS) : "memory");
   }
 }

@@ -215,6 +215,13 @@ __device__ __forceinline__ float4 sum_partials(const float4* p, long long stride
   return y;
 }
 
+// The warp's lanes, together again.  The tensor memory's instructions (tcgen05.ld, st, alloc, dealloc: .sync.aligned) want all 32 lanes of
+// a warp at the same instruction; behind a wait in which every lane polls by itself, a branch that differs by lane (the store of a
+// row that not every lane has) or a role that one lane plays, nothing but this promises that.
+__device__ __forceinline__ void warp_whole() { __syncwarp(); }
+// One answer of the whole warp, which is together again behind it: whether `v` holds in all lanes.
+__device__ __forceinline__ bool warp_all(bool v) { return __all_sync(0xffffffffu, v); }
+
 // Row of the paged key/value store that holds position `pos` of the sequence in `slot`,
 // for key/value head `kvh`.  Pages are [n_pages][n_kv][LLG_PAGE][head_dim]; a sequence's
 // logical page j lies at table[slot][j % ring_pages] (ring_pages = table width for a group

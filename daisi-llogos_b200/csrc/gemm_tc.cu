@@ -212,6 +212,7 @@ __device__ __forceinline__ void token_rows_epilogue(const GemmParams& p, uint32_
 #pragma unroll
       for (int c0 = 0; c0 < HD; c0 += 16) {
         uint32_t r[16];
+        warp_whole();                             // (the last head's stores are the live tokens')
         tmem_ld16(acc + (uint32_t)(hb * HD + c0), r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
@@ -294,8 +295,9 @@ __device__ __forceinline__ void token_rows_epilogue(const GemmParams& p, uint32_
       if (f0 >= width) break;
       float v[16];
       uint32_t r[16];
+      warp_whole();                                         // (the last run's stores are those of the tokens that there are)
       tmem_ld16(acc + (uint32_t)c0, r);
-      if (EPI == 1) {
+      if (EPI == 1) {                                       // uniform
         uint32_t ru[16];
         tmem_ld16(acc + (uint32_t)(TN / 2 + c0), ru);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -476,6 +478,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tc_kernel(const __grid_cons
     }
   }
   if (warp == MMA_WARP) {
+    warp_whole();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)),
                  "r"((uint32_t)TMEM_COLS)
                  : "memory");
@@ -591,14 +594,14 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tc_kernel(const __grid_cons
         // tokens along the columns: their scales, worked out while the products run
         for (int c = tid; c < TN; c += EPI_WARPS * 32) col_scales[round & 1][c] = n0 + c < p.n ? row_scale_of(p.scale, n0 + c) : 0.f;
         mbar_arrive(&scale_bar);
-        if (!mbar_wait(&scale_bar, round & 1, abortp)) {
-          if (!*abortp) { *abortp = 1; atomicCAS(&g_error, 0, 3); }
-          break;
-        }
+        const bool there = mbar_wait(&scale_bar, round & 1, abortp);
+        if (!there && !*abortp) { *abortp = 1; atomicCAS(&g_error, 0, 3); }
+        if (!warp_all(there)) break;
       }
       const bool have = mbar_wait(&acc_full[b], (round / NACC) & 1, abortp);
       if (!have && !*abortp) { *abortp = 1; atomicCAS(&g_error, 0, 3); }
-      if (!have || *abortp) break;
+      // one answer for the warp: reading tensor memory wants all of its lanes
+      if (!warp_all(have && !*abortp)) break;
       if (tid == 0 && round == 0) LLG_STAMP(1, 2, st_aux, st_blk);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       {
@@ -622,9 +625,10 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tc_kernel(const __grid_cons
             for (int c0 = 0; c0 < TN; c0 += CH) {
               if (n0 + c0 >= p.n) break;        // uniform over the block: the tile's tail holds no tokens
               uint32_t r[CH / 16][16];
+              warp_whole();                     // (the last columns' stores are those of the features that there are)
   #pragma unroll
-              for (int q = 0; q < CH / 16; ++q)
-                if (n0 + c0 + 16 * q < p.n) tmem_ld16(lane_base + (uint32_t)(mt * TN + c0 + 16 * q), r[q]);
+              for (int q = 0; q < CH / 16; ++q)       // uniform
+                if (n0 + c0 + 16 * q < p.n) tmem_ld16(lane_base + (uint32_t)(mt * TN + c0 + 16 * q), r[q]);   // uniform
               asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
               if (o < p.o) {
   #pragma unroll
@@ -660,6 +664,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tc_kernel(const __grid_cons
               float v = 0.f;
               if (tok >= 0 && tok < TN) {
                 const float rw = p.row_weight ? p.row_weight[n0 + j] : 1.0f;
+                warp_whole();                                   // (the last row's store is that of the features that there are)
                 const float g = tmem_ld1(lane_base + (uint32_t)tok), u = tmem_ld1(lane_base + (uint32_t)(TN + tok));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 v = gate_act(gate, g * rw, u * rw);
@@ -671,9 +676,10 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tc_kernel(const __grid_cons
           for (int c0 = 0; c0 < TN; c0 += CH) {
             if (n0 + c0 >= p.n) break;
             uint32_t rg[CH / 16][16], ru[CH / 16][16];
+            warp_whole();
   #pragma unroll
-            for (int q = 0; q < CH / 16; ++q) {
-              if (n0 + c0 + 16 * q < p.n) {
+            for (int q = 0; q < CH / 16; ++q) {       // uniform
+              if (n0 + c0 + 16 * q < p.n) {           // uniform
                 tmem_ld16(lane_base + (uint32_t)(c0 + 16 * q), rg[q]);
                 tmem_ld16(lane_base + (uint32_t)(TN + c0 + 16 * q), ru[q]);
               }
@@ -710,6 +716,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tc_kernel(const __grid_cons
   __syncthreads();
   if (tid == 0) LLG_STAMP(1, 3, st_aux, st_blk);
   if (warp == MMA_WARP) {
+    warp_whole();                                         // one lane comes from its role's loop
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"((uint32_t)TMEM_COLS) : "memory");
   }
 }
@@ -814,6 +821,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_pair_kernel(const __grid_co
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == MMA_WARP) {
+    warp_whole();
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)),
                  "r"((uint32_t)(NACC * ACC_COLS))
                  : "memory");
@@ -909,7 +917,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_pair_kernel(const __grid_co
       const bool have = mbar_wait(&acc_full[b], (round / NACC) & 1, abortp);
       if (!have && !*abortp) { *abortp = 1; atomicCAS(&g_error, 0, 3); }
       // one answer for the warp: reading tensor memory wants all of its lanes
-      if (__any_sync(0xffffffffu, !have || *abortp)) break;
+      if (!warp_all(have && !*abortp)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int o0 = token0(tile);
       if (o0 < p.o)                                       // uniform over the block: the pair's second half may lie past the tokens
@@ -925,7 +933,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_pair_kernel(const __grid_co
   __syncthreads();
   cluster_barrier();                                      // nobody leaves while the other's products, copies or arrivals may come
   if (warp == MMA_WARP) {
-    __syncwarp();                                         // the next instruction wants the whole warp
+    warp_whole();                                         // one lane comes from its role's loop
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"((uint32_t)(NACC * ACC_COLS)) : "memory");
   }
 }
