@@ -284,7 +284,7 @@ __device__ __forceinline__ void token_rows_epilogue(const GemmParams& p, uint32_
     const GateForm gate = p.gate;
     constexpr int VEC = 16 / (int)sizeof(OT);      // outputs per 16-byte store
     const int width = EPI == 1 ? p.gated_features : p.n;
-    const bool vec_ok = width % VEC == 0;
+    const bool vec_ok = width % VEC == 0 && ((uintptr_t)p.out & 15u) == 0;      // `out` may start at any element
     OT* out = (OT*)p.out + (long long)split * p.n * p.o;
     const float rs = tok >= p.o ? 1.0f : (EPI == 1 && p.row_weight) ? p.row_weight[tok] : row_scale_of(p.scale, tok);
     OT* row = out + (long long)tok * width;

@@ -729,6 +729,32 @@ def test_gemm_tc_of_large_steps(ops, n, o, k):
     assert ops.gemm_tc_status() == 0
 
 
+@pytest.mark.parametrize("n", [128, 129, 200, 256, 1030])
+def test_gemm_tc_into_rows_that_start_anywhere(ops, n):
+    """``out`` as a view that starts one element into its storage, in either orientation and in pairs of blocks: 16-byte stores would fault."""
+    o, k = 9216, 72
+    x, w = rnd((n, k), 17, torch.bfloat16), rnd((o, k), 18, torch.bfloat16, 1.0 / math.sqrt(k))
+    want, xd, wd = P.linear(x, w), x.to(DEV), w.to(DEV)
+
+    def view(cols, dtype):
+        whole = torch.full((2 + n * cols,), 7.0, dtype=dtype, device=DEV)
+        return whole, whole[1:1 + n * cols].view(1, n, cols)
+
+    for dtype in (torch.float32, torch.bfloat16):
+        whole, out = view(o, dtype)
+        ops.gemm_tc(xd, wd, out)
+        check(out[0].cpu(), want, dtype, "plain")
+        assert float(whole[0]) == float(whole[-1]) == 7.0
+    whole, out = view(o, torch.bfloat16)
+    ops.gemm_tc_act(xd, wd, out[0], "relu2")
+    check(out[0].cpu(), torch.relu(want) ** 2, torch.bfloat16, "activation")
+    whole, out = view(o // 2, torch.bfloat16)
+    ops.gemm_tc(xd, _gated(w[:o // 2], w[o // 2:]).to(DEV), out, gated_features=o // 2)
+    g, u = want[:, :o // 2], want[:, o // 2:]
+    check(out[0].cpu(), g / (1 + torch.exp(-g)) * u, torch.bfloat16, "gated")
+    assert float(whole[0]) == float(whole[-1]) == 7.0 and ops.gemm_tc_status() == 0
+
+
 def _scale_of(ss, width, eps):
     """The factor a row scale stands for: 1 / sqrt(sum(ss) / width + eps) per row, float64."""
     return 1.0 / torch.sqrt(ss.double().sum(dim=1) / width + eps)
