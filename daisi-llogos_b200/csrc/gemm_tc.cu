@@ -1052,12 +1052,68 @@ int launch_pair(const void* x, const void* w, const GemmParams& p, cudaStream_t 
 // units of the time that a block with one token tile takes per feature.  Measured at 8,192 tokens, k 4,096: a round is 26.6 us at
 // 256 features (0.80 of the other form's), 25.2 at 224, 23.6 at 192 and 22.3 at 160: it goes by the bytes brought, not by the
 // products, so narrower tiles than 224 never pay.
-double pair_cost(int tokens, int features, int width) {
-  const long long tiles = (long long)((tokens + 2 * BM - 1) / (2 * BM)) * ((features + width - 1) / width), pairs = llg_sm_count() / 2;
+double pair_cost(int tokens, int features, int width, long long sms) {
+  const long long tiles = (long long)((tokens + 2 * BM - 1) / (2 * BM)) * ((features + width - 1) / width), pairs = sms / 2;
   return (double)((tiles + pairs - 1) / pairs) * (width + (256 - width) / 2) * PAIR_UNIT;
 }
 
+// Whether tokens are the tensor cores' rows (128 of them a tile, up to 256 features) or the weights are (128 features a tile, up to 256
+// tokens).  From 256 tokens on tokens are.  Below, at 129 to 255, by what the product writes, measured in both orientations (one
+// split, one block a tile, k 2,048 to 14,336, 512 to 128,256 features): gated, tokens always (weights first takes 1.02 to 2.8
+// times as long: a tile of a step of few blocks fills 56 of its 128 rows, and the read-out in pieces of 2 bytes is not hidden; 8,192 x
+// 2,048 at 232 tokens 54 -> 26 us); bfloat16, tokens from 224 on (0.98 to 1.3 times; 0.93 to 1.1 at 129 and 144); float32, weights
+// (0.70 to 1.0 times; a thread that owns a token writes its features 16 bytes at a time, lanes a row apart, where lanes that are
+// features write whole lines: 6,144 x 4,096 at 160 tokens, with the splits of either plan, 15.6 us against 23.0).
+bool tokens_first(int n, bool gated, int out_dtype) { return n >= 256 || (n > 128 && gated) || (n >= 224 && out_dtype == LLG_BF16); }
+
+// The form of a prompt step's product.
+struct PromptForm {
+  int width;      // features per tile, 0: the weights are the first operand
+  int mt;         // token tiles per block
+  bool pair;      // a pair of blocks for two token tiles
+};
+PromptForm prompt_form(int n, int o, int splits, bool gated, int out_dtype, long long sms) {
+  if (!tokens_first(n, gated, out_dtype)) return {0, 0, false};
+  // Tile shape: blocks run in rounds of one per SM (148 on a B200); a round costs its tile's width, and a narrower tile can save a
+  // round (4096 features: 16 tiles of 256 in two token rows of 8 are 128 blocks, 18 of 240 are 144).  Two token
+  // tiles per block halve the weight traffic per flop (worth about 15 %) but double the tile.
+  const int widths[5] = {256, gated ? 192 : 240, 224, gated ? 256 : 208, gated ? 256 : 176};
+  PromptForm best{256, 1, false};
+  double best_cost = 0;
+  for (int wi = 0; wi < 5; ++wi) {
+    for (int mt = 1; mt <= 2; ++mt) {
+      if (mt == 1 && widths[wi] < 224) continue;      // a single token tile wants a wide second operand
+      const long long tiles = (long long)((n + mt * BM - 1) / (mt * BM)) * ((o + widths[wi] - 1) / widths[wi]) * splits;
+      const double cost = (double)((tiles + sms - 1) / sms) * widths[wi] * mt * (mt == 2 ? 0.85 : 1.0);
+      if (best_cost == 0 || cost < best_cost * 0.999) {
+        best_cost = cost;
+        best = {widths[wi], mt, false};
+      }
+    }
+  }
+  if (gated && out_dtype == LLG_F32) return {256, best.mt, false};      // float32 out of a gated product: the widest tile only
+  // Pairs of blocks instead, where they come out cheaper.
+  if (splits == 1 && sms >= 2) {
+    const int pair_widths[2] = {256, 224};
+    for (int w : pair_widths) {
+      const double cost = pair_cost(n, o, w, sms);
+      if (cost < best_cost * 0.999) {
+        best_cost = cost;
+        best = {w, 2, true};
+      }
+    }
+  }
+  return best;
+}
+
 }  // namespace
+
+// The form that llg_gemm_tc and its relatives take for these sizes on a GPU of `sms` multiprocessors: 0 with the weights as first
+// operand, else the features per tile plus 1,000 for one token tile a block, 2,000 for two, 3,000 for a pair of blocks.
+LLG_API int llg_gemm_tc_form(int n, int o, int splits, int gated, int out_dtype, int sms) {
+  const PromptForm f = prompt_form(n, o, splits < 1 ? 1 : splits, gated != 0, out_dtype, sms < 1 ? 1 : sms);
+  return f.width ? f.width + 1000 * (f.pair ? 3 : f.mt) : 0;
+}
 
 // 1 if the tensor-core kernel takes these operands: k a multiple of 8 (TMA needs 16-byte row strides)
 // and 16-byte aligned base addresses.
@@ -1128,58 +1184,21 @@ static int gemm_tc_run(const void* x, const void* w, void* out, int out_dtype, i
               gated_features, o, splits);
   const int nkb = (k + BK - 1) / BK;
   CUtensorMap map_w, map_x;
-  if (n > 128 && tile_n <= 0) {
-    // ---- prompt steps: activations are the first operand (128 tokens per tile), up to 256 features per tile.  From 129 tokens
-    // on: with the weights as first operand a gated tile of a step of few blocks fills 56 of its 128 rows, and the read-out of
-    // 256 token columns in pieces of 2 bytes is not hidden (8,192 x 2,048 gated at 232 tokens: 54 us that way, 26 this) ----
+  if (tile_n <= 0 && tokens_first(n, gated, out_dtype)) {
+    // ---- prompt steps: activations are the first operand (128 tokens per tile), up to 256 features per tile ----
     // in this orientation the kernel's first-operand rows (field o) are the tokens, the second's (field n) the features
     GemmParams ps{out, /*n=*/o, /*o=*/n, k, (nkb + splits - 1) / splits, gated_features, o / 2, BM, QkPrepArgs{}, rs, act, nullptr, 0, gate, nullptr, nullptr};
-    // Tile shape: blocks run in rounds of one per SM (148 on a B200); a round costs its tile's width, and a narrower tile can save a
-    // round (4096 features: 16 tiles of 256 in two token rows of 8 are 128 blocks, 18 of 240 are 144).  Two token
-    // tiles per block halve the weight traffic per flop (worth about 15 %) but double the tile.
-    const int widths[5] = {256, gated ? 192 : 240, 224, gated ? 256 : 208, gated ? 256 : 176};
-    int best_w = 256, best_mt = 1;
-    double best_cost = 0;
-    const long long sms = llg_sm_count();
-    for (int wi = 0; wi < 5; ++wi) {
-      for (int mt = 1; mt <= 2; ++mt) {
-        if (mt == 1 && widths[wi] < 224) continue;      // a single token tile wants a wide second operand
-        const long long tiles = (long long)((n + mt * BM - 1) / (mt * BM)) * ((o + widths[wi] - 1) / widths[wi]) * splits;
-        const double cost = (double)((tiles + sms - 1) / sms) * widths[wi] * mt * (mt == 2 ? 0.85 : 1.0);
-        if (best_cost == 0 || cost < best_cost * 0.999) {
-          best_cost = cost;
-          best_w = widths[wi];
-          best_mt = mt;
-        }
-      }
-    }
-    // Pairs of blocks instead, where they come out cheaper.
-    if (splits == 1 && llg_sm_count() >= 2 && !(gated && out_dtype == LLG_F32)) {
-      const int pair_widths[2] = {256, 224};
-      int pw = 0;
-      double pc = best_cost;
-      for (int wi = 0; wi < 2; ++wi) {
-        const double cost = pair_cost(n, o, pair_widths[wi]);
-        if (cost < pc * 0.999) {
-          pc = cost;
-          pw = pair_widths[wi];
-        }
-      }
+    const PromptForm form = prompt_form(n, o, splits, gated, out_dtype, llg_sm_count());
+    const int best_w = form.width, best_mt = form.mt;
+    if (form.pair) {
 #define PAIRS(OTT, EP)                                                   \
-  if (pw == 256) return launch_pair<256, OTT, EP>(x, w, ps, stream);     \
-  if (pw == 224) return launch_pair<224, OTT, EP>(x, w, ps, stream)
-      if (gated) {
-        PAIRS(__nv_bfloat16, 1);
-      } else if (act) {
-        PAIRS(__nv_bfloat16, -1);
-      } else if (out_dtype == LLG_F32) {
-        PAIRS(float, 0);
-      } else {
-        PAIRS(__nv_bfloat16, 0);
-      }
+  return best_w == 256 ? launch_pair<256, OTT, EP>(x, w, ps, stream) : launch_pair<224, OTT, EP>(x, w, ps, stream)
+      if (gated) PAIRS(__nv_bfloat16, 1);
+      if (act) PAIRS(__nv_bfloat16, -1);
+      if (out_dtype == LLG_F32) PAIRS(float, 0);
+      PAIRS(__nv_bfloat16, 0);
 #undef PAIRS
     }
-    if (gated && out_dtype == LLG_F32) best_w = 256;
     // the gated product fetches the gate half and the up half of a feature tile with a box of half the width each
     LLG_REQUIRE(tensor_map(x, n, k, BM, &map_x) && tensor_map(w, o, k, gated ? best_w / 2 : best_w, &map_w),
                 "gemm_tc: cuTensorMapEncodeTiled failed or is not available");
@@ -1370,7 +1389,7 @@ LLG_API int llg_gemm_tc_qkv(const void* x, const void* w, int n, int k, const Qk
   const long long t1 = (long long)((n + BM - 1) / BM) * ((o + 255) / 256), t2 = (long long)((n + 2 * BM - 1) / (2 * BM)) * ((o + 255) / 256);
   const bool two = (double)((t2 + sms - 1) / sms) * 2 * 0.85 < (double)((t1 + sms - 1) / sms);
   // or a pair of blocks for two token tiles
-  if (sms >= 2 && pair_cost(n, o, 256) < 256.0 * (two ? (double)((t2 + sms - 1) / sms) * 2 * 0.85 : (double)((t1 + sms - 1) / sms)))
+  if (sms >= 2 && pair_cost(n, o, 256, sms) < 256.0 * (two ? (double)((t2 + sms - 1) / sms) * 2 * 0.85 : (double)((t1 + sms - 1) / sms)))
     return a.hd == 128 ? launch_pair<256, __nv_bfloat16, 2>(x, w, ps, stream) : launch_pair<256, __nv_bfloat16, 3>(x, w, ps, stream);
   if (a.hd == 128)
     return two ? launch<256, 3, __nv_bfloat16, 2, 2, 1>(&map_x, &map_w, ps, 1, stream)

@@ -38,10 +38,10 @@ def _plan_splits(n: int, o: int, k: int, n_sms: int) -> int:
     if n > SPLIT_ROWS_MAX:
         return 1
     nkb = -(-k // 64)
-    if n > 128:                   # tokens are the MMA rows: 128 tokens x 256 features per tile, one block per SM
+    if n >= 256:                  # tokens are the MMA rows: 128 tokens x 256 features per tile, one block per SM
         tiles, tile_bytes, resident = -(-n // 128) * -(-o // 256), (128 + 256) * 128, n_sms
     else:                         # weights are the MMA rows: 128 features x a token tile
-        tile_n = 16 if n <= 16 else 32 if n <= 32 else 64 if n <= 64 else 128
+        tile_n = 16 if n <= 16 else 32 if n <= 32 else 64 if n <= 64 else 128 if n <= 128 else 256
         tiles, tile_bytes = -(-o // 128) * -(-n // tile_n), (128 + tile_n) * 128
         resident = 2 * n_sms if tile_n <= 64 else n_sms
     unit_us = tile_bytes / _BLOCK_BYTES_PER_US

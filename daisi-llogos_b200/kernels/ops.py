@@ -428,6 +428,7 @@ def _load_lib(name: str):
     elif name == "gemm_tc":
         lib.llg_gemm_tc_supported.argtypes = [c_void_p, c_void_p, c_int, c_int, c_int]
         lib.llg_gemm_tc_splits.argtypes = [c_int, c_int]
+        lib.llg_gemm_tc_form.argtypes = [c_int, c_int, c_int, c_int, c_int, c_int]
         lib.llg_gemm_tc.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                     POINTER(_RowScale), c_void_p]
         lib.llg_gemm_tc_gated.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
@@ -630,6 +631,12 @@ def gemm_tc_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
         return False
     # the library's rule (llg_gemm_tc_supported), kept here because this runs before every product
     return x.shape[0] > 0 and x.shape[1] % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+
+
+def gemm_tc_form(n: int, o: int, out_dtype: torch.dtype, *, splits: int = 1, gated: bool = False, sms: int = 0) -> int:
+    """The form that ``gemm_tc`` takes for ``n`` rows and ``o`` rows of the matrix: 0 with the weights as first operand, else the features
+    per tile plus 1000 (one token tile a block), 2000 (two) or 3000 (a pair of blocks).  ``sms``: multiprocessors (0: this GPU's)."""
+    return _lib("gemm_tc").llg_gemm_tc_form(n, o, splits, int(gated), F32 if out_dtype == torch.float32 else BF16, sms or sm_count())
 
 
 _splits_cache = {}

@@ -729,6 +729,23 @@ def test_gemm_tc_of_large_steps(ops, n, o, k):
     assert ops.gemm_tc_status() == 0
 
 
+@pytest.mark.parametrize("n", [129, 192, 223, 224, 255])
+def test_gemm_tc_of_129_to_255_tokens(ops, n):
+    """What a product of a step of that size writes says which operand comes first: float32 sums (one split and several) the weights, a
+    gated product the tokens, bfloat16 the tokens from 224 on."""
+    o, k = 2600, 520
+    assert ops.gemm_tc_form(n, o, torch.float32, splits=3) == ops.gemm_tc_form(n, o, torch.float32) == 0
+    assert ops.gemm_tc_form(n, o, torch.bfloat16, gated=True) > 0 and (ops.gemm_tc_form(n, o, torch.bfloat16) > 0) == (n >= 224)
+    x, w = rnd((n, k), 19, torch.bfloat16), rnd((o, k), 20, torch.bfloat16, 1.0 / math.sqrt(k))
+    ss = rnd((n, 3), 21).abs() * 40 + 1
+    scale, want = ops.RowScale(ss.to(DEV), 96, 1e-3), P.linear(x, w) * _scale_of(ss, 96, 1e-3)[:, None]
+    for splits, dtype in ((1, torch.float32), (3, torch.float32), (1, torch.bfloat16)):
+        out = torch.full((splits, n, o), float("nan"), dtype=dtype, device=DEV)
+        ops.gemm_tc(x.to(DEV), w.to(DEV), out, row_scale=scale)
+        check(out.float().sum(0).cpu(), want, dtype, (splits, dtype))
+    assert ops.gemm_tc_status() == 0
+
+
 @pytest.mark.parametrize("n", [128, 129, 200, 256, 1030])
 def test_gemm_tc_into_rows_that_start_anywhere(ops, n):
     """``out`` as a view that starts one element into its storage, in either orientation and in pairs of blocks: 16-byte stores would fault."""
