@@ -373,6 +373,60 @@ def test_expert_kernels(llogos, dtype, n, hidden, n_exp, top, ff):
     assert float((out.cpu().double() - want).abs().max()) < tol * float(want.abs().max())
 
 
+@pytest.mark.parametrize("weighted", [False, True], ids=["", "weighted rows, clamped"])
+@pytest.mark.parametrize("n,hidden,n_exp,top,ff", [(2, 520, 17, 1, 136), (3, 2048, 16, 4, 1024), (8, 2048, 16, 4, 1000), (31, 520, 20, 4, 300),
+                                                   (32, 328, 16, 3, 264), (33, 520, 20, 2, 304)])
+def test_expert_products_of_few_tokens(llogos, n, hidden, n_exp, top, ff, weighted):
+    """The experts' two products as a stream of their matrices (at most 32 tokens for the gated one; 33 take the other kernel): rings that
+    wrap, widths that end inside a k-block, several feature tiles of an expert, the last one short, fewer features a tile than 128 where the
+    step uses few experts, experts without a token.  Every row of a used tile is written, filling rows with zeros."""
+    ops = ops_module()
+    g = torch.Generator().manual_seed(n + ff)
+    x = torch.randn((n, hidden), generator=g).bfloat16()
+    gate, up = ((1.5 * torch.randn((n_exp, ff, hidden), generator=g) / math.sqrt(hidden)).bfloat16() for _ in range(2))
+    down = (torch.randn((n_exp, hidden, ff), generator=g) / math.sqrt(ff)).bfloat16()
+    choice = torch.stack([torch.randperm(n_exp - 2, generator=g)[:top] for _ in range(n)]).int()        # two experts get no token
+    pair_weight = torch.rand((n, top), generator=g) + 0.25
+    cap = ops.moe_row_capacity(n * top, n_exp)
+    row_of_pair = torch.empty((n * top,), dtype=torch.int32, device="cuda")
+    token_of_row = torch.empty((cap,), dtype=torch.int32, device="cuda")
+    tile_expert = torch.empty((cap // ops.MOE_TILE_ROWS,), dtype=torch.int32, device="cuda")
+    row_weight = torch.empty((cap,), device="cuda") if weighted else None
+    ops.moe_plan(choice.cuda(), n_exp, row_of_pair, token_of_row, tile_expert, pair_weight.cuda() if weighted else None, row_weight)
+    pad = -(-ff // 128) * 128
+    gate_up = torch.full((n_exp, 2 * pad, hidden), 3.0, dtype=torch.bfloat16)                         # (the rows between are nobody's)
+    gate_up[:, :ff], gate_up[:, pad:pad + ff] = gate, up
+    act = torch.full((cap, ff), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.moe_gated(x.cuda(), token_of_row, tile_expert, gate_up.cuda(), act, ops.GateForm(1.702, 0.7, 1.0) if weighted else None, row_weight)
+    y = torch.full((cap, hidden), float("nan"), device="cuda")
+    ops.moe_down(act, tile_expert, down.cuda(), y)
+    assert ops.gemm_tc_status() == 0
+    tok, tile = token_of_row.cpu().long(), tile_expert.cpu().long()
+    used = 0
+    for t in range(tile.numel()):
+        rows = slice(t * ops.MOE_TILE_ROWS, (t + 1) * ops.MOE_TILE_ROWS)
+        if tile[t] < 0:
+            continue
+        e, live = int(tile[t]), tok[rows] >= 0
+        xr = torch.where(live[:, None], x.double()[tok[rows].clamp(min=0)], 0.0)
+        if weighted:
+            xr = xr * row_weight.cpu().double()[rows, None]
+        a, b = xr @ gate[e].double().t(), xr @ up[e].double().t()
+        if weighted:
+            a = a.clamp(max=0.7)
+            want = a * torch.sigmoid(1.702 * a) * (b.clamp(-0.7, 0.7) + 1.0)
+        else:
+            want = a * torch.sigmoid(a) * b
+        got = act[rows].cpu()
+        # bfloat16 outputs of float32 sums: half a unit of the last place, and the sums' own rounding
+        assert bool(((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-4).all()), (t, float((got.double() - want).abs().max()))
+        assert float(got[~live].abs().sum()) == 0.0
+        want = got.double() @ down[e].double().t()
+        assert float((y[rows].cpu().double() - want).abs().max()) <= 2e-5 * max(1.0, float(want.abs().max()))
+        used += int(live.sum())
+    assert used == n * top
+
+
 # ---- whole models ------------------------------------------------------------------------------------
 
 @pytest.mark.parametrize("dtype", DTYPES, ids=IDS)

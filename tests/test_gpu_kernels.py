@@ -112,9 +112,11 @@ def test_add_rmsnorm_of_many_rows(ops, dtype, hidden):
         check(out, P.rms_norm(total, w, eps), dtype, "normed")
 
 
-# float32 rows of 16 bytes: the weight stream up to 16 rows (chunks of 1, 2, 4 or 8 rows; a warp's k with and without a
-# remainder), the tiles of 64 x 128 above, alone and shared by a cluster's 2, 4 and 8 blocks (unequal shares among them)
+# float32 rows of 16 bytes: the weight stream up to 32 rows (chunks of 1, 2, 4 or 8 rows, the last one short; a warp's k with and
+# without a remainder), the tiles of 64 x 128 above, whose k one block, two (100 x 3,170: 50 tiles of eight steps) or four share, the
+# last of four with less than the others or with nothing (65 x 300: nine steps, three a block)
 @pytest.mark.parametrize("n,o,k", [(1, 5, 4), (2, 33, 132), (3, 64, 1000), (7, 301, 2048), (9, 20, 516), (16, 4100, 260), (17, 129, 4),
+                                   (25, 301, 2052), (32, 4100, 260), (33, 200, 132), (63, 129, 1036), (100, 3170, 252), (65, 300, 288),
                                    (64, 128, 1036), (65, 257, 4104), (200, 300, 2052), (130, 24000, 64)])
 def test_gemm_simt_float32_rows(ops, n, o, k):
     x, w = rnd((n, k), 5), rnd((o, k), 6, torch.float32, 1.0 / math.sqrt(k))
@@ -414,14 +416,25 @@ def test_attn_prefill_and_kv_write(ops, dtype, nh, nkv, hd, window, tc, monkeypa
         assert ops.attn_tc_status() == 0
 
 
+def _log_sum(q, k, scale, window):
+    """log sum over the visible keys of e^score, per query and head: [T, nh] in float64."""
+    t, nh, _ = q.shape
+    at = torch.arange(t)
+    hidden = (at[None] > at[:, None]) | ((at[None] <= at[:, None] - window) if window else torch.zeros(t, t, dtype=torch.bool))
+    scores = torch.einsum("qhd,khd->hqk", q.double(), k.double().repeat_interleave(nh // k.shape[1], 1)) * scale
+    return torch.logsumexp(scores.masked_fill(hidden, -math.inf), -1).t()
+
+
 @pytest.mark.parametrize("before,counts,window", [([0] * 6, [3, 64, 1, 37, 63, 17], 0), ([0, 63, 64, 65, 300, 0], [128, 1, 64, 83, 100, 65], 0),
                                                   ([10, 200, 517, 0, 0, 40], [5, 83, 128, 129, 40, 24], 100)],
                          ids=["one key tile", "several", "window"])
 @pytest.mark.parametrize("nh,nkv", [(32, 8), (32, 32), (30, 10)])
 @pytest.mark.parametrize("hd", [64, 128])
-def test_attn_prefill_of_few_queries_per_sequence(ops, hd, nh, nkv, before, counts, window):
+@pytest.mark.parametrize("sinks", [False, True], ids=["", "sinks and a gate"])
+def test_attn_prefill_of_few_queries_per_sequence(ops, hd, nh, nkv, before, counts, window, sinks):
     """Tiles of at most 128 queries in the tcgen05 kernel, more blocks than multiprocessors: two heads in a block where a sequence has
-    one key tile (an odd group of heads: one), the keys shared by the block's two halves where it has more; tiles of more beside them."""
+    one key tile (an odd group of heads: one), the keys shared by the block's two halves where it has more; tiles of more beside them.
+    The sinks differ widely from head to head, the gates from token to token, so that another head's shows."""
     dtype, scale = torch.bfloat16, 1 / math.sqrt(hd)
     ring = 16 if window == 0 else (window + 63) // 64 + 1
     total = [a + c for a, c in zip(before, counts)]
@@ -433,17 +446,25 @@ def test_attn_prefill_of_few_queries_per_sequence(ops, hd, nh, nkv, before, coun
     cu = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32)
     q = rnd((int(cu[-1]), nh, hd), 45, dtype)
     k_new, v_new = (torch.cat([t[b][before[b]:] for b in range(len(counts))]) for t in (ks, vs))
-    tq = ops.prefill_tile_queries(dtype, hd)
+    sink = 3.0 * rnd((nh,), 46) if sinks else None
+    gate = torch.rand((int(cu[-1]), nh), generator=torch.Generator().manual_seed(47)) if sinks else None
+    form = ops.AttentionForm(sinks=sink.to(DEV), gated=True) if sinks else None
+    tq = ops.prefill_tile_queries(dtype, hd, form)
     tiles = torch.tensor([(b, q0) for b, c in enumerate(counts) for q0 in range(0, c, tq)], dtype=torch.int32)
     out = torch.full((int(cu[-1]), nh * hd), float("nan"), dtype=dtype, device=DEV)
     d = lambda t: t.to(DEV)
     ops.attn_prefill(d(q), d(k_new), d(v_new), d(kp), d(vp), d(table), ring, d(tiles), d(cu), d(torch.tensor(before, dtype=torch.int32)),
-                     d(slots), out, scale=scale, window=window, tile_queries=tq)
+                     d(slots), out, scale=scale, window=window, tile_queries=tq, form=form, gate=d(gate) if sinks else None)
     assert ops.attn_tc_status() == 0
     for b in range(len(counts)):
         qq = torch.zeros(total[b], nh, hd, dtype=dtype)
         qq[before[b]:] = q[int(cu[b]):int(cu[b + 1])]
-        ref = P.attention(qq, ks[b], vs[b], scale, window)[before[b]:].reshape(counts[b], -1)
+        ref = P.attention(qq, ks[b], vs[b], scale, window)[before[b]:]
+        if sinks:
+            # a sink s takes its share of the weights: those of the keys shrink by 1 / (1 + e^(s - log sum e^score))
+            share = torch.sigmoid(_log_sum(qq, ks[b], scale, window)[before[b]:] - sink.double())
+            ref = ref * (share * gate[int(cu[b]):int(cu[b + 1])].double())[:, :, None]
+        ref = ref.reshape(counts[b], -1)
         check(out[int(cu[b]):int(cu[b + 1])], ref, dtype, ("sequence", b))
 
 
@@ -705,10 +726,19 @@ def test_qkv_product_with_the_preparation_as_its_epilogue(ops, nh, nkv, hd, k, n
 
 # ---- a norm that leaves its division to the products that consume it ------------------------------------------------
 
-@pytest.mark.parametrize("n,o,k", [(129, 21000, 64), (257, 30001, 72), (700, 9004, 264), (1030, 9000, 1032), (2305, 2600, 136)])
-def test_gemm_tc_of_large_steps(ops, n, o, k):
-    """Products of prompt steps in all their forms (one or two token tiles a block, pairs of blocks): token and feature tails, one k-block
-    and many, more tiles than blocks; plain in both types, with an activation, gated, with the rows' scales."""
+# (tokens, features, k), the form that a GPU of 148 multiprocessors takes for float32, bfloat16 and gated outputs: 256 and 224 features in
+# pairs of blocks with token and feature tails, one tile a pair (500) and several, a k below the ring's six stages and above, one band of
+# eight token tiles and two (2,305); one and two token tiles a block
+@pytest.mark.parametrize("n,o,k,forms", [(129, 21000, 64, (0, 0, 2192)), (257, 30001, 72, (1224, 1224, 1224)), (700, 9004, 264, (2208, 2208, 2192)),
+                                         (1030, 9000, 1032, (3224, 3224, 3224)), (2305, 2600, 136, (2208, 2208, 2224)),
+                                         (500, 9000, 1032, (3256, 3256, 3256)), (700, 18900, 72, (3256, 3256, 3256)),
+                                         (2305, 9000, 136, (3256, 3256, 3256))])
+def test_gemm_tc_of_large_steps(ops, n, o, k, forms):
+    """Products of prompt steps in their forms (one or two token tiles a block, pairs of blocks, or the weights first): plain in both types,
+    with an activation, gated, with the rows' scales."""
+    taken = (ops.gemm_tc_form(n, o, torch.float32, sms=148), ops.gemm_tc_form(n, o, torch.bfloat16, sms=148),
+             ops.gemm_tc_form(n, -(-(o // 2) // 128) * 256, torch.bfloat16, gated=True, sms=148))
+    assert taken == forms, "the size no longer shows the form that it stands for"
     x, w = rnd((n, k), 14, torch.bfloat16), rnd((o, k), 15, torch.bfloat16, 1.0 / math.sqrt(k))
     ss = rnd((n, 3), 16).abs() * 40 + 1
     scale, f = ops.RowScale(ss.to(DEV), 96, 1e-3), _scale_of(ss, 96, 1e-3)[:, None]
