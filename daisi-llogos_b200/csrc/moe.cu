@@ -621,12 +621,11 @@ LLG_API int llg_grouped_linear(const GroupedLinearArgs* args, int x_dtype, int y
   if (a.rows == 0) return 0;
   const bool gated = a.w2 != nullptr;
   auto aligned = [](const void* p) { return ((uintptr_t)p & 15u) == 0; };
-  if (x_dtype == LLG_BF16 && a.n_in % 8 == 0 && aligned(a.x) && aligned(a.w) && aligned(a.w2)) {
-    // the tensor-core kernel: 16-byte copies need rows that start on 16-byte boundaries
-    if (y_dtype == LLG_BF16)
-      return gated ? run_mma<__nv_bfloat16, true>("grouped_linear", a, 1, stream) : run_mma<__nv_bfloat16, false>("grouped_linear", a, 1, stream);
-    if (y_dtype == LLG_F32)
-      return gated ? run_mma<float, true>("grouped_linear", a, 1, stream) : run_mma<float, false>("grouped_linear", a, 1, stream);
+  if (gated && x_dtype == LLG_BF16 && a.n_in % 8 == 0 && aligned(a.x) && aligned(a.w) && aligned(a.w2)) {
+    // the tensor-core kernel: 16-byte copies need rows that start on 16-byte boundaries (one matrix with such rows is
+    // llg_gemm_tc_grouped_few's, whatever the number of tokens)
+    if (y_dtype == LLG_BF16) return run_mma<__nv_bfloat16, true>("grouped_linear", a, 1, stream);
+    if (y_dtype == LLG_F32) return run_mma<float, true>("grouped_linear", a, 1, stream);
     return llg_fail("grouped_linear: unsupported output dtype %d", y_dtype);
   }
   dim3 grid(a.rows / LLG_MOE_TILE, (a.n_out + GT_O - 1) / GT_O);
