@@ -316,7 +316,9 @@ __global__ void __launch_bounds__(256) grouped_linear_kernel(GroupedLinearArgs a
 // Two shapes.  Many tiles (prompts): 128 outputs, two stages, the matrix rows used for the most products.  Few tiles: the kernel is
 // a stream of the chosen experts' matrices, and what bounds it is the bytes that the multiprocessors have under way: 64 outputs
 // and three stages (four of one matrix) give twice the blocks, two or three of them a multiprocessor.  100 tokens' four of 16
-// experts of 1,024 x 2,048: gated 57.4 -> 45.9 us, of 1,792 x 4,096 (eight tokens) 110 -> 88; one matrix 30.9 -> 21.5, 55 -> 59.
+// experts of 1,024 x 2,048: gated 57.4 -> 45.9 us, of 1,792 x 4,096 (eight tokens) 110 -> 88.  One matrix is only the per-head
+// products' now, which follow the same rule and were not timed by themselves (experts' down products, which have left for the
+// stream of gemm_tc.cu: 30.9 -> 21.5 of 1,024 x 2,048, but 55 -> 59 of 1,792 x 4,096).
 constexpr int MM_K = 64, MM_PAD = 8;                        // MM_PAD halves between rows: fragment loads meet no bank twice
 constexpr int MM_WIDE = 128, MM_NARROW = 64;
 constexpr int MM_LD = MM_K + MM_PAD;
