@@ -448,7 +448,7 @@ def test_attn_prefill_of_few_queries_per_sequence(ops, hd, nh, nkv, before, coun
     k_new, v_new = (torch.cat([t[b][before[b]:] for b in range(len(counts))]) for t in (ks, vs))
     sink = 3.0 * rnd((nh,), 46) if sinks else None
     gate = torch.rand((int(cu[-1]), nh), generator=torch.Generator().manual_seed(47)) if sinks else None
-    form = ops.AttentionForm(sinks=sink.to(DEV), gated=True) if sinks else None
+    form = ops.AttentionForm(sinks=sink.to(DEV), gated=True) if sinks else ops.PLAIN_ATTENTION
     tq = ops.prefill_tile_queries(dtype, hd, form)
     tiles = torch.tensor([(b, q0) for b, c in enumerate(counts) for q0 in range(0, c, tq)], dtype=torch.int32)
     out = torch.full((int(cu[-1]), nh * hd), float("nan"), dtype=dtype, device=DEV)
