@@ -95,7 +95,8 @@ __device__ __forceinline__ float both(pair_t v) { return __uint_as_float((unsign
 // 16,384 x 2,048: 23.5 us for one row (5.7 TB/s), 28.4 for three (4.7), 36.5 for eight (3.7; there the cores bound it); 128,256 x
 // 2,048 at three rows 169 us (6.2 TB/s).  gemm_tn_kernel, which took these before, pays for 64 rows: 618 us on average over a 1B
 // model's products.
-template <int NR, int F>
+// LIVE of the NR rows are there (the rest of the sums stay zero).
+template <int NR, int F, int LIVE>
 __global__ void __launch_bounds__(256, 2) gemv_rows_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                         float* __restrict__ out, int n, int o, int k, int wk, RowScale scale) {
   constexpr int NV = NR * F;
@@ -130,7 +131,7 @@ __global__ void __launch_bounds__(256, 2) gemv_rows_kernel(const float* __restri
 #pragma unroll
     for (int f = 0; f < F; ++f) wn[f] = cn < k4 ? __ldcs(wp[f] + cn) : zero;
 #pragma unroll
-    for (int r = 0; r < NR; ++r) {
+    for (int r = 0; r < LIVE; ++r) {
       const float4 xv = xp[r][c];
 #pragma unroll
       for (int f = 0; f < F; ++f) {
@@ -175,24 +176,28 @@ __global__ void __launch_bounds__(256, 2) gemv_rows_kernel(const float* __restri
   }
 }
 
-// More rows (a prompt step): tiles of 64 rows x 128 features, 256 threads with 8 x 4 sums each.  Both operands arrive by
+// More rows (a prompt step): tiles of up to 64 rows x 128 features, 256 threads with up to 8 x 4 sums each.  Both operands arrive by
 // cp.async as they lie in memory, 32 k of a row at a time, in a ring of three stages: a stage is 24 KB, so that one block a
 // multiprocessor already has the bytes in flight that the memory's latency asks for (with the next stage in registers and
 // half as much a step a block waited 2 us a step: 100 x 2,048 x 2,048 81.5 us before, 38.6 now).  Rows are padded to 36 floats: 16-byte
 // reads of consecutive rows at one k fall into different banks.  A thread takes four k at a time, 12 reads for 128
 // multiply-adds.  From 300 rows on the multiply-add pipes (two thirds busy) and the 16-byte shared reads bound it: 38 TFLOP/s.  Where a shape has few tiles, the blocks of a cluster
 // share the tile's k and add their sums through distributed shared memory, in the order of the ranks.
-constexpr int TM = 64, TF = 128, TK = 32, TLD = TK + 4, TSTAGES = 3;
-constexpr int TILE_SMEM = TSTAGES * (TM + TF) * TLD * (int)sizeof(float);
-static_assert(TM * TF * (int)sizeof(float) <= TILE_SMEM, "the sums fit where the stages were");
+// A tile has 40, 48, 56 or 64 rows (R = 5 to 8 a thread), by the rows that a count of tokens leaves empty: 44 x 16,384 x 2,048 141 us in
+// tiles of 64, 96 in tiles of 48 (two blocks a tile); 44 x 2,048 x 8,192 142 us and 97 (tiles of 40, four blocks).
+constexpr int TF = 128, TK = 32, TLD = TK + 4, TSTAGES = 3;
+__host__ __device__ constexpr int tile_smem(int rows) { return TSTAGES * (rows + TF) * TLD * (int)sizeof(float); }
 
 __device__ __forceinline__ void copy16(float* dst, const float* src, bool there) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
                "r"(there ? 16 : 0) : "memory");
 }
 
+template <int R>
 __global__ void __launch_bounds__(256, 2) gemm_tile_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                         float* __restrict__ out, int n, int o, int k, RowScale scale) {
+  constexpr int TM = 8 * R;                              // rows of a tile, R a thread
+  static_assert(TM * TF * (int)sizeof(float) <= tile_smem(TM) && TM <= 64, "the sums fit where the stages were");
   extern __shared__ __align__(16) float sm[];            // the stages, then the tile's sums
   pdl_launch_dependents();
   cg::cluster_group cluster = cg::this_cluster();
@@ -218,16 +223,16 @@ __global__ void __launch_bounds__(256, 2) gemm_tile_kernel(const float* __restri
     const int kk = (s0 + s) * TK + lc;
     float* dst = sm + (s % TSTAGES) * (TM + TF) * TLD + lr * TLD + lc;
 #pragma unroll
-    for (int i = 0; i < TM / 32; ++i) {
+    for (int i = 0; i < (TM + 31) / 32; ++i) {
       const int r = n0 + i * 32 + lr;
       const bool there = kk < k && r < n;
-      copy16(dst + i * 32 * TLD, x + (there ? (long long)r * k + kk : 0), there);
+      if (i * 32 + lr < TM) copy16(dst + i * 32 * TLD, x + (there ? (long long)r * k + kk : 0), there);
     }
   };
   auto close = [&]() { asm volatile("cp.async.commit_group;" ::: "memory"); };
-  pair_t sums[8][4];
+  pair_t sums[R][4];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < R; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) sums[i][j] = 0;
   // the first stages' weights do not wait for the kernel before
@@ -249,22 +254,22 @@ __global__ void __launch_bounds__(256, 2) gemm_tile_kernel(const float* __restri
     const float* ws = sm + (s % TSTAGES) * (TM + TF) * TLD + (TM + tx) * TLD;
 #pragma unroll 2
     for (int kk = 0; kk < TK; kk += 4) {
-      ulonglong2 a[8];
+      ulonglong2 a[R];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(xs + i * 8 * TLD + kk);
+      for (int i = 0; i < R; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(xs + i * 8 * TLD + kk);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const ulonglong2 f = *reinterpret_cast<const ulonglong2*>(ws + j * 32 * TLD + kk);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) fma2(sums[i][j], a[i].x, f.x);
+        for (int i = 0; i < R; ++i) fma2(sums[i][j], a[i].x, f.x);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) fma2(sums[i][j], a[i].y, f.y);
+        for (int i = 0; i < R; ++i) fma2(sums[i][j], a[i].y, f.y);
       }
     }
   }
   if (ranks == 1) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < R; ++i) {
       const int r = n0 + ty + 8 * i;
       if (r >= n) continue;
       const float rs = scale.ss ? row_scale_of(scale, r) : 1.0f;
@@ -278,7 +283,7 @@ __global__ void __launch_bounds__(256, 2) gemm_tile_kernel(const float* __restri
   }
   __syncthreads();                                       // the sums go where the last stage was read
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < R; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) sm[(ty + 8 * i) * TF + tx + 32 * j] = both(sums[i][j]);
   cluster.sync();
@@ -302,7 +307,7 @@ __global__ void __launch_bounds__(256, 2) gemm_tile_kernel(const float* __restri
   cluster.sync();                                        // nobody leaves while its sums may still be read
 }
 
-template <int NR, int F>
+template <int NR, int F, int LIVE = NR>
 int run_gemv(const float* x, const float* w, float* out, int n, int o, int k, const RowScale& rs, cudaStream_t stream) {
   // warps that share k: enough for about 32 a multiprocessor, each with a float4 a lane at least
   int wk = 1;
@@ -311,32 +316,21 @@ int run_gemv(const float* x, const float* w, float* out, int n, int o, int k, co
   const long long per = (long long)F * (8 / wk);
   const long long blocks = ((o + per - 1) / per) * ((n + NR - 1) / NR);
   LLG_REQUIRE(blocks <= 2147483647LL, "gemm_simt: too many blocks");
-  cudaError_t e = llg_launch(gemv_rows_kernel<NR, F>, dim3((unsigned)blocks), dim3(256), 0, stream, x, w, out, n, o, k, wk, rs);
+  cudaError_t e = llg_launch(gemv_rows_kernel<NR, F, LIVE>, dim3((unsigned)blocks), dim3(256), 0, stream, x, w, out, n, o, k, wk, rs);
   if (e != cudaSuccess) return llg_fail("gemm_simt: launch: %s", cudaGetErrorString(e));
   return llg_check_launch("gemm_simt");
 }
 
-int run_tile(const float* x, const float* w, float* out, int n, int o, int k, const RowScale& rs, cudaStream_t stream) {
-  const long long tiles = (long long)((n + TM - 1) / TM) * ((o + TF - 1) / TF), sms = llg_sm_count();
-  const int steps = (k + TK - 1) / TK;
-  // blocks that share a tile's k: the rounds of blocks over the multiprocessors times a block's steps and a fixed cost (clusters
-  // of eight with a multiprocessor a block do not all fit at once: 42 us at 64 x 2,048 x 2,048)
-  int ranks = 1;
-  long long best = 0;
-  for (int s = 1; s <= 4; s *= 2) {
-    if (s > 1 && steps < 2 * s) break;
-    const long long cost = ((tiles * s + sms - 1) / sms) * ((steps + s - 1) / s + 3 + (s > 1 ? 2 : 0));
-    if (best == 0 || cost < best) { best = cost; ranks = s; }
-  }
-  const long long gx = (long long)((o + TF - 1) / TF) * ranks;
+template <int R>
+int launch_tile(const float* x, const float* w, float* out, int n, int o, int k, int ranks, const RowScale& rs, cudaStream_t stream) {
+  const long long gx = (long long)((o + TF - 1) / TF) * ranks, sms = llg_sm_count();
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)gx, (unsigned)((n + TM - 1) / TM));
+  cfg.gridDim = dim3((unsigned)gx, (unsigned)((n + 8 * R - 1) / (8 * R)));
   cfg.blockDim = dim3(256);
   // where every block can have a multiprocessor of its own it asks for more than half of one's shared memory: blocks of a
   // cluster are placed densely otherwise, two on a multiprocessor beside an idle one
   constexpr int ALONE_SMEM = 120 * 1024;
-  const int smem = gx * cfg.gridDim.y <= sms ? ALONE_SMEM : TILE_SMEM;
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = gx * cfg.gridDim.y <= sms ? ALONE_SMEM : tile_smem(8 * R);
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -347,11 +341,45 @@ int run_tile(const float* x, const float* w, float* out, int n, int o, int k, co
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = llg_pdl_enabled() ? 2 : 1;
-  cudaError_t e = cudaFuncSetAttribute(gemm_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ALONE_SMEM);
+  cudaError_t e = cudaFuncSetAttribute(gemm_tile_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, ALONE_SMEM);
   if (e != cudaSuccess) return llg_fail("gemm_simt: cannot have %d bytes of shared memory: %s", ALONE_SMEM, cudaGetErrorString(e));
-  e = cudaLaunchKernelEx(&cfg, gemm_tile_kernel, x, w, out, n, o, k, rs);
+  e = cudaLaunchKernelEx(&cfg, gemm_tile_kernel<R>, x, w, out, n, o, k, rs);
   if (e != cudaSuccess) return llg_fail("gemm_simt: launch: %s", cudaGetErrorString(e));
   return llg_check_launch("gemm_simt");
+}
+
+// Rows of a tile (40, 48, 56 or 64) and the blocks that share a tile's k: the multiprocessor with the most blocks has their steps to do, each as
+// long as the tile has rows (two blocks a multiprocessor take as long as one with twice the steps, to 5 %), and every block a fixed
+// cost.  Clusters of four leave some multiprocessors out (288 blocks, 100 x 3,072 x 2,048: 68 us, where 144 in clusters of two take 51), clusters
+// of eight more (42 us at 64 x 2,048 x 2,048).  Of the twelve forms, timed at 36 to 600 rows of a 1B model's four matrices, it takes the
+// fastest or one within 15 % of it.
+struct TileForm { int rows, ranks; };
+TileForm tile_form(int n, int o, int k, long long sms) {
+  const int steps = (k + TK - 1) / TK;
+  TileForm best{64, 1};
+  double best_cost = 0;
+  for (int rows = 64; rows >= 40; rows -= 8) {
+    const long long tiles = (long long)((n + rows - 1) / rows) * ((o + TF - 1) / TF);
+    for (int s = 1; s <= 4; s *= 2) {
+      if (s > 1 && steps < 2 * s) break;
+      const long long places = s == 4 ? sms - sms / 14 : sms, per_sm = (tiles * s + places - 1) / places;
+      const double cost = rows / 64.0 * (per_sm == 1 ? 1.0 : 0.95 * per_sm) * ((steps + s - 1) / s) + 3.0 + (s > 1 ? 2.0 : 0.0);
+      if (best_cost == 0 || cost < best_cost * 0.999) {
+        best_cost = cost;
+        best = {rows, s};
+      }
+    }
+  }
+  return best;
+}
+
+int run_tile(const float* x, const float* w, float* out, int n, int o, int k, TileForm form, const RowScale& rs, cudaStream_t stream) {
+  switch (form.rows) {
+    case 40: return launch_tile<5>(x, w, out, n, o, k, form.ranks, rs, stream);
+    case 48: return launch_tile<6>(x, w, out, n, o, k, form.ranks, rs, stream);
+    case 56: return launch_tile<7>(x, w, out, n, o, k, form.ranks, rs, stream);
+    default: return launch_tile<8>(x, w, out, n, o, k, form.ranks, rs, stream);
+  }
 }
 
 // Rows up to which the weight stream is taken: at 32 rows of 2,048 x 2,048 it takes 21 us and the tiles 38, at 40 rows 27 and 38, but
@@ -373,9 +401,11 @@ LLG_API int llg_gemm_simt(const void* x, int x_dtype, const void* w, int w_dtype
     float* of = (float*)out;
     if (n == 1) return run_gemv<1, 8>(xf, wf, of, n, o, k, rs, stream);
     if (n == 2) return run_gemv<2, 8>(xf, wf, of, n, o, k, rs, stream);
-    if (n <= 4) return run_gemv<4, 8>(xf, wf, of, n, o, k, rs, stream);
+    if (n == 3) return run_gemv<4, 8, 3>(xf, wf, of, n, o, k, rs, stream);
+    if (n == 4) return run_gemv<4, 8>(xf, wf, of, n, o, k, rs, stream);
+    if (n <= 6) return run_gemv<8, 4, 6>(xf, wf, of, n, o, k, rs, stream);
     if (n <= GEMV_ROWS_MAX) return run_gemv<8, 4>(xf, wf, of, n, o, k, rs, stream);
-    return run_tile(xf, wf, of, n, o, k, rs, stream);
+    return run_tile(xf, wf, of, n, o, k, tile_form(n, o, k, llg_sm_count()), rs, stream);
   }
 #define LAUNCH(AT, WT, CT) \
   gemm_tn_kernel<AT, WT, CT><<<grid, 256, 0, stream>>>((const AT*)x, (const WT*)w, (CT*)out, n, o, k, rs)
@@ -393,4 +423,21 @@ LLG_API int llg_gemm_simt(const void* x, int x_dtype, const void* w, int w_dtype
   }
 #undef LAUNCH
   return llg_check_launch("gemm_simt");
+}
+
+// The float32 product in tiles of `rows` rows (40, 48, 56 or 64), `ranks` blocks (1, 2 or 4) sharing a tile's k: the form that llg_gemm_simt
+// chooses by itself above some rows.  k in whole fours, operands on 16 bytes.
+LLG_API int llg_gemm_simt_tile(const float* x, const float* w, float* out, int n, int o, int k, int rows, int ranks, const RowScale* scale,
+                               cudaStream_t stream) {
+  LLG_REQUIRE(n > 0 && o > 0 && k > 0 && k % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15u) == 0, "gemm_simt_tile: n=%d o=%d k=%d", n, o, k);
+  LLG_REQUIRE((rows == 40 || rows == 48 || rows == 56 || rows == 64) && (ranks == 1 || ranks == 2 || ranks == 4) &&
+                  (ranks == 1 || (k + TK - 1) / TK >= 2 * ranks) && (n + rows - 1) / rows <= 65535,
+              "gemm_simt_tile: tiles of %d rows, %d blocks", rows, ranks);
+  return run_tile(x, w, out, n, o, k, TileForm{rows, ranks}, scale ? *scale : RowScale{nullptr, 0, 0.f, 0.f}, stream);
+}
+
+// The form that llg_gemm_simt takes for these sizes above the rows of its weight stream: rows + 1,000 times the blocks of a tile.
+LLG_API int llg_gemm_simt_form(int n, int o, int k, int sms) {
+  const TileForm f = tile_form(n, o, k, sms);
+  return f.rows + 1000 * f.ranks;
 }

@@ -425,6 +425,8 @@ def _load_lib(name: str):
     elif name == "gemm_simt":
         lib.llg_gemm_simt.argtypes = [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int,
                                       POINTER(_RowScale), c_void_p]
+        lib.llg_gemm_simt_tile.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, POINTER(_RowScale), c_void_p]
+        lib.llg_gemm_simt_form.argtypes = [c_int, c_int, c_int, c_int]
     elif name == "gemm_tc":
         lib.llg_gemm_tc_supported.argtypes = [c_void_p, c_void_p, c_int, c_int, c_int]
         lib.llg_gemm_tc_splits.argtypes = [c_int, c_int]
@@ -704,6 +706,16 @@ def gemm_tc_act(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, kind: str, 
         raise KernelError(f"gemm_tc_act: activation '{kind}' is not known ({', '.join(ACTIVATIONS)})")
     _check(lib, lib.llg_gemm_tc_act(_ptr(x, torch.bfloat16), _ptr(w, torch.bfloat16), _ptr(out, torch.bfloat16), _dt(out), n, o, k,
                                     ACTIVATIONS[kind], _scale_ref(row_scale, n), _stream()))
+
+
+def gemm_simt_tile(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, rows: int, ranks: int, row_scale: Optional[RowScale] = None) -> None:
+    """The float32 product ``gemm_simt`` in tiles of ``rows`` rows with ``ranks`` blocks sharing a tile's k, whatever it would choose."""
+    lib = _lib("gemm_simt")
+    n, k = x.shape
+    o, k2 = w.shape
+    assert k == k2 and out.shape == (n, o), (x.shape, w.shape, out.shape)
+    _check(lib, lib.llg_gemm_simt_tile(_ptr(x, torch.float32), _ptr(w, torch.float32), _ptr(out, torch.float32), n, o, k, rows, ranks,
+                                       _scale_ref(row_scale, n), _stream()))
 
 
 def gemm_tc_status() -> int:

@@ -129,6 +129,20 @@ def test_gemm_simt_float32_rows(ops, n, o, k):
         assert torch.equal(out[n].cpu(), torch.full((o,), 7.0))
 
 
+@pytest.mark.parametrize("n,o,k", [(33, 130, 256), (44, 300, 260), (100, 129, 1028), (129, 400, 520)])
+@pytest.mark.parametrize("rows,ranks", [(r, s) for r in (40, 48, 56, 64) for s in (1, 2, 4)])
+def test_gemm_simt_tiles(ops, n, o, k, rows, ranks):
+    """Every tile height and every count of blocks that share a tile's k, rows and features that fill no tile."""
+    x, w = rnd((n, k), 5), rnd((o, k), 6, torch.float32, 1.0 / math.sqrt(k))
+    ss = rnd((n, 3), 7).abs() + 0.5
+    out = torch.full((n + 1, o), 7.0, device=DEV)
+    for scale in (None, ops.RowScale(ss.to(DEV), 96, 1e-3)):
+        ops.gemm_simt_tile(x.to(DEV), w.to(DEV), out[:n], rows, ranks, row_scale=scale)
+        want = P.linear(x, w) if scale is None else P.linear(x, w) * _scale_of(ss, 96, 1e-3)[:, None]
+        check(out[:n].cpu(), want, torch.float32, f"scale={scale is not None}")
+        assert torch.equal(out[n].cpu(), torch.full((o,), 7.0))
+
+
 @pytest.mark.parametrize("n,o,k", [(1, 128, 64), (3, 200, 72), (16, 129, 128), (17, 384, 1000), (33, 100, 8),
                                    (70, 130, 336), (129, 65, 16), (300, 1000, 520), (2, 301, 4104),
                                    (1100, 9000, 72), (2050, 4700, 136)])
