@@ -8,22 +8,28 @@
 //
 // A block owns 256 queries of one head as two tiles of 128.  Each tile has a group of four softmax
 // warps: thread r of a group owns query row r of its tile, which is lane r of tensor memory, so the
-// softmax of a row needs no exchange between threads.  Three more warps serve both groups: one lane
-// issues every product, one warp copies the key tiles and one the value tiles (TMA boxes from the
+// softmax of a row needs no exchange between threads.  Four more warps serve the groups: a lane each
+// issues a group's products, one warp copies the key tiles and one the value tiles (TMA boxes from the
 // step's packed buffer or from a cache page; the one tile per sequence that lies partly in each row by
-// row with cp.async; three stages each).
-// The roles meet only at mbarriers: tiles full / free between the copying warps and the issuing lane,
-// scores ready, weights ready and accumulator updated between the issuing lane and a group.  Each
+// row with cp.async; four stages each).
+// The roles meet only at mbarriers: tiles full / free between the copying warps and the issuing lanes,
+// scores ready, weights ready and accumulator updated between a group and its issuing lane.  Each
 // group has two score buffers in tensor memory, so that the tensor core computes the next tile's
 // scores and the previous tile's O += P V while the group runs the softmax of the current one; the
 // scores of tile j + 1 are issued when O += P(j-1) V(j-1) has finished with the buffer they go into.
 //
 // Q and K are K-major operands in shared memory with the 128-byte swizzle; V is stored as it lies in
 // memory ([key][dim], dim contiguous), which makes it the MN-major second operand of the second product;
-// P never leaves tensor memory (the products' operand fetch from shared memory is what bounds this
-// kernel, and P would be a third of it).
-// A row's accumulator is rescaled in place (tcgen05.ld / tcgen05.st) only when its maximum grows by
-// more than a factor of 2^8 in the weights, warp by warp and only when some row of the warp needs it.
+// P never leaves tensor memory.
+// A row's accumulator is rescaled in place (tcgen05.ld / tcgen05.st) only when a tile's weights add up to more than
+// 2^14, warp by warp and only when some row of the warp needs it; only then are the tile's maxima worked out.
+//
+// A key tile's time is a softmax warp's chain of it, about 2,000 cycles: 64 exponentials a row (700 cycles with the other
+// group's beside them 980; the special-function unit is busy 43 % of the time, the tensor cores 42), the way in and out of
+// tensor memory, and 100 to 200 cycles for each barrier that is passed.  So a tile has no maximum and no wait that it
+// can do without.  8,192 tokens x 32 heads of 128: 634 us with a lane for both groups' products, a maximum and a wait for the
+// accumulator in every tile, 584 now; 2,048 tokens 81 and 69; four prompts of 1,100 tokens, heads of 64, 128 and 100; 300 tokens 25 and 18.
+// (Taking turns with the exponentials, group by group: 650 us at 8,192 tokens, 82 at 2,048.)
 //
 // Tiles of at most 128 queries (short prompts, the next turn of a chat) leave the second group without queries.  It then takes
 // part in one of two ways, which every block finds from its own tile.  SPLIT (two key tiles or more): the groups share the keys,
@@ -31,7 +37,7 @@
 // block's time is the chain of its key tiles (scores, softmax, product).  TWO_HEADS (one key tile, and more
 // blocks than multiprocessors): the second group takes the next query head of the same key/value head and that head's own block
 // ends at once; such blocks cost their set-up, so half as many are half the time.  Four sequences of 83 queries behind 1,000 to
-// 4,000 keys, 32 heads of 128: 63.4 us before, 55.8 now; five prompts of 3 to 90 tokens, 32 heads of 64: 19.0 us before, 12.7 now.
+// 4,000 keys, 32 heads of 128: 46 us (two groups of queries a block: 63); five prompts of 3 to 90 tokens, 32 heads of 64: 15 us (19).
 //
 // With MAPS (differential attention) the two halves of a query and of a key are two maps over the same values: the block's
 // two groups are the two maps of ONE tile of 128 queries, whose scores are products over their half of the head; keys,
@@ -197,12 +203,15 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 __device__ __forceinline__ uint32_t swz(int row, int chunk) { return (uint32_t)(row * 128 + ((chunk ^ (row & 7)) << 4)); }
 
 constexpr int GROUPS = 2;                     // query tiles of 128 rows per block, each with its own softmax warps
-constexpr int KST = 3, VST = 3;               // stages of keys and of values
+constexpr int KST = 4, VST = 4;               // stages of keys and of values
+static_assert(KST % 2 == 0 && VST % 2 == 0, "where the groups take turns with the key tiles, a stage belongs to one of them: a wait for its next phase "
+              "by parity means something only to who has seen the last one");
 constexpr int WORKERS = GROUPS * BQ;          // softmax threads: thread r of group g owns query row r of tile g
-constexpr int ISSUE_WARP = WORKERS / 32;      // one lane of this warp issues every product
+constexpr int ISSUE_WARP = WORKERS / 32;      // one lane of this warp issues the first group's products
 constexpr int K_LOAD_WARP = ISSUE_WARP + 1;   // copies key tiles
 constexpr int V_LOAD_WARP = ISSUE_WARP + 2;   // copies value tiles
-constexpr int THREADS = (V_LOAD_WARP + 1) * 32;
+constexpr int ISSUE_WARP_2 = ISSUE_WARP + 3;  // issues the second group's products
+constexpr int THREADS = (ISSUE_WARP_2 + 1) * 32;
 
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
@@ -309,17 +318,17 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
   if (tid == 0) {
     for (int s = 0; s < KST; ++s) {
       mbar_init(&k_full[s], 1);
-      mbar_init(&k_free[s], 1);
+      mbar_init(&k_free[s], mode == SPLIT ? 1 : GROUPS);       // who reads a tile: one group, or both
     }
     for (int s = 0; s < VST; ++s) {
       mbar_init(&v_full[s], 1);
-      mbar_init(&v_free[s], 1);
+      mbar_init(&v_free[s], mode == SPLIT ? 1 : GROUPS);
     }
     for (int g = 0; g < GROUPS; ++g) {
       mbar_init(&s_full[g][0], 1);
       mbar_init(&s_full[g][1], 1);
-      mbar_init(&p_ready[g][0], BQ);
-      mbar_init(&p_ready[g][1], BQ);
+      mbar_init(&p_ready[g][0], BQ / 32);
+      mbar_init(&p_ready[g][1], BQ / 32);
       mbar_init(&o_done[g], 1);
     }
     mbar_init(&q_ready, WORKERS);
@@ -434,14 +443,33 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
         }
       }
     }
-  } else if (warp == ISSUE_WARP) {
-    // ---- products: one lane issues them all.  The tensor core takes them one after the other, and a
-    // lane that issues is held up while its queue is full, which is why no softmax warp does this. ------
+  } else if (warp == ISSUE_WARP || warp == ISSUE_WARP_2) {
+    // ---- products: one lane per group issues them.  The tensor core takes them one after the other, and a lane that issues is
+    // held up while its queue is full, which is why no softmax warp does this; one lane for both groups let each group's next
+    // scores wait for the other group's weights. ------
     if (elect_one()) {
+      const int g = warp == ISSUE_WARP ? 0 : 1;
+      const bool split = !MAPS && mode == SPLIT;
       constexpr uint32_t IDESC_S = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TK >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
       constexpr uint32_t IDESC_O = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
-      // scores of key tile t, the group's own tile i (the same number but for SPLIT), into the group's score buffer i % 2
-      auto issue_scores = [&](int g, int t, int i) {
+      bool ok = true;
+      auto wait_or_fail = [&](uint64_t* bar, uint32_t parity, int code) {
+        if (!ok) return;
+        if (!mbar_wait(bar, parity, abortp)) {
+          if (!*abortp) { *abortp = 1; atomicCAS(&g_error, 0, code); }
+          ok = false;
+        }
+      };
+      // the group's own tile i is key tile i, or (SPLIT) every second one
+      const int n_own = split ? (ti.n_max + 1 - g) >> 1 : ti.n_tiles[g];
+      auto tile_of = [&](int i) { return split ? 2 * i + g : i; };
+      // scores of the group's tile i into its score buffer i % 2
+      auto issue_scores = [&](int i) {
+        const int t = tile_of(i);
+        wait_or_fail(&k_full[t % KST], (t / KST) & 1, 5);
+        if (i >= 2) wait_or_fail(&o_done[g], i & 1, 6);            // O += P(i-2) V(i-2) has read the buffer
+        if (!ok) return;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t qa = smem_u32(Qs + (one_q ? 0 : g * Q_BYTES)), ka = smem_u32(Ks + (t % KST) * KV_BYTES);
 #pragma unroll
         for (int ks = 0; ks < (MAPS ? HD / 32 : HD / 16); ++ks) {
@@ -451,9 +479,19 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
                     desc_kmajor(ka + blk * (TK * 128) + kk * 32), IDESC_S, ks != 0);
         }
         umma_commit(&s_full[g][i & 1]);
+        umma_commit(&k_free[t % KST]);
       };
-      // O += P(i) V(t)
-      auto issue_values = [&](int g, int t, int i) {
+      wait_or_fail(&q_ready, 0, 5);
+      if (n_own > 0) issue_scores(0);
+      // Step i: the scores of tile i + 1; then, once the group has turned S(i) into P(i) (written over S(i) in tensor memory),
+      // O += P(i) V(i).
+      for (int i = 0; i < n_own && ok; ++i) {
+        const int t = tile_of(i);
+        if (i + 1 < n_own) issue_scores(i + 1);
+        wait_or_fail(&v_full[t % VST], (t / VST) & 1, 5);
+        wait_or_fail(&p_ready[g][i & 1], (i >> 1) & 1, 6);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t pa = tmem + g * G_COLS + (uint32_t)(i & 1) * TK, va = smem_u32(Vs + (t % VST) * KV_BYTES);
 #pragma unroll
         for (int kk = 0; kk < TK / 16; ++kk) {
@@ -461,74 +499,16 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
           umma_bf16_ts(tmem + g * G_COLS + O_COL, pa + kk * 8, desc_mnmajor(va + kk * 2048, TK * 128), IDESC_O, (i | kk) != 0);
         }
         umma_commit(&o_done[g]);
-      };
-      bool ok = true;
-      auto wait_or_fail = [&](uint64_t* bar, uint32_t parity, int code) {
-        if (!ok) return;
-        if (!mbar_wait(bar, parity, abortp)) {
-          if (!*abortp) { *abortp = 1; atomicCAS(&g_error, 0, code); }
-          ok = false;
-        }
-      };
-      wait_or_fail(&q_ready, 0, 5);
-      if (ok && ti.n_max > 0) {
-        wait_or_fail(&k_full[0], 0, 5);
-        if (ok) {
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          for (int g = 0; g < (mode == SPLIT ? 1 : GROUPS); ++g)
-            if (0 < ti.n_tiles[g]) issue_scores(g, 0, 0);
-          umma_commit(&k_free[0]);
-        }
+        umma_commit(&v_free[t % VST]);
       }
-      if (!MAPS && mode == SPLIT) {
-        // tile t is group t % 2's tile t / 2; both groups' first scores, then per tile the group's next scores and O += P V
-        wait_or_fail(&k_full[1 % KST], 0, 5);
-        if (ok) {
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          issue_scores(1, 1, 0);
-          umma_commit(&k_free[1 % KST]);
-        }
-        for (int t = 0; t < ti.n_max && ok; ++t) {
-          const int g = t & 1, i = t >> 1;
-          if (t + 2 < ti.n_max) {
-            wait_or_fail(&k_full[(t + 2) % KST], ((t + 2) / KST) & 1, 5);
-            if (i >= 1) wait_or_fail(&o_done[g], (i - 1) & 1, 6);
-            if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            issue_scores(g, t + 2, i + 1);
-            umma_commit(&k_free[(t + 2) % KST]);
-          }
+      // tiles that only the other group sees: given back as they arrive
+      if (!split) {
+        for (int t = n_own; t < ti.n_max && ok; ++t) {
+          wait_or_fail(&k_full[t % KST], (t / KST) & 1, 5);
+          if (ok) mbar_arrive(&k_free[t % KST]);
           wait_or_fail(&v_full[t % VST], (t / VST) & 1, 5);
-          wait_or_fail(&p_ready[g][i & 1], (i >> 1) & 1, 6);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          issue_values(g, t, i);
-          umma_commit(&v_free[t % VST]);
+          if (ok) mbar_arrive(&v_free[t % VST]);
         }
-        ok = false;                                        // (nothing is left for the loop below)
-      }
-      // Step j: the scores of tile j + 1 go into the buffer whose weights P(j-1) the product of step j - 1 has
-      // read by now; then, once the group has turned S(j) into P(j) (written over S(j) in tensor memory),
-      // O += P(j) V(j).
-      for (int j = 0; j < ti.n_max && ok; ++j) {
-        wait_or_fail(&v_full[j % VST], (j / VST) & 1, 5);
-        if (j + 1 < ti.n_max) wait_or_fail(&k_full[(j + 1) % KST], ((j + 1) / KST) & 1, 5);
-        for (int g = 0; g < GROUPS && ok; ++g) {
-          if (j >= ti.n_tiles[g]) continue;
-          if (j + 1 < ti.n_tiles[g]) {
-            if (j >= 1) wait_or_fail(&o_done[g], (j - 1) & 1, 6);
-            if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            issue_scores(g, j + 1, j + 1);
-          }
-          wait_or_fail(&p_ready[g][j & 1], (j >> 1) & 1, 6);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          issue_values(g, j, j);
-        }
-        if (!ok) break;
-        umma_commit(&v_free[j % VST]);
-        if (j + 1 < ti.n_max) umma_commit(&k_free[(j + 1) % KST]);
       }
     }
   } else if (tid < WORKERS && ti.nq[tid / BQ] > 0) {
@@ -539,11 +519,11 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
     const int n_tiles = split ? (ti.n_max + 1 - g) >> 1 : ti.n_tiles[g], pos0 = ti.pos0[g];
     const float sc = a.scale * LOG2E;
     // A row's weights are 2^(x - M) with x = score * scale * log2 e and M a whole number that is raised (to the
-    // tile's maximum, rounded up) only when a tile exceeds it by more than 8: the weights stay below 2^8 and the
-    // accumulator is rescaled rarely, by an exact power of two.  The common factor cancels in the final division,
+    // tile's maximum, rounded up) only when a tile's weights add up to more than 2^14, so some weight is above 2^8: no weight
+    // exceeds 2^14 and the accumulator is rescaled rarely, by an exact power of two.  The common factor cancels in the final division,
     // and rounding a weight to bfloat16 gives the same bits whatever M was: how the keys are cut into tiles or
     // steps does not show in the rounded weights.
-    const float raise_by = 8.0f;
+    const float sum_bound = 16384.0f;
     const int qpos = pos0 + r;
     float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
@@ -580,47 +560,63 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
           sv[c] = valid ? sv[c] : -INFINITY;
         }
       }
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      // The weights of the tile at the M there is, and their sum: a sum within the bound says that no weight is far out of
+      // range, so most tiles need no maximum (its 32 instructions a row took a quarter of a tile's time).
+      // Two elements per instruction where the arithmetic allows it (fma.rn.f32x2, add.rn.f32x2).
+      uint32_t pk[TK / 2];
+      float psum;
+      auto weights = [&](float m) {
+        const float ms = m == -INFINITY ? 0.f : m;
+        const float2 sc2 = make_float2(sc, sc), nms2 = make_float2(-ms, -ms);
+        float2 ps2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-      for (int c = 0; c < TK; c += 8) {
+        for (int e = 0; e < TK / 2; ++e) {
+          const float2 x = __ffma2_rn(make_float2(sv[2 * e], sv[2 * e + 1]), sc2, nms2);
+          const float2 w = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+          ps2[e & 1] = __fadd2_rn(ps2[e & 1], w);
+          pk[e] = pack_bf16(w.x, w.y);
+        }
+        psum = (ps2[0].x + ps2[0].y) + (ps2[1].x + ps2[1].y);
+      };
+      float corr = 1.f;
+      bool fits = false, rescale = false;                // the latter one answer for the warp
+#pragma unroll 1
+      for (int pass = j == 0; ; ++pass) {
+        if (pass == 1) {
+          // the first tile, one whose scores rise, rows that have seen no key yet
+          float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int k = 0; k < 4; ++k) mx4[k] = max3(mx4[k], sv[c + 2 * k], sv[c + 2 * k + 1]);
+          for (int c = 0; c < TK; c += 8) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) mx4[k] = max3(mx4[k], sv[c + 2 * k], sv[c + 2 * k + 1]);
+          }
+          const float mxs = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * sc;
+          const float m_new = fits ? m_run : fmaxf(m_run, ceilf(mxs));
+          corr = m_new == m_run || m_new == -INFINITY ? 1.f : pow2_whole(m_run - m_new);
+          m_run = m_new;
+          rescale = !warp_all(corr == 1.f);
+        }
+        weights(m_run);
+        fits = m_run != -INFINITY && psum <= sum_bound;
+        if (pass == 1 || warp_all(fits)) break;          // uniform
       }
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      const float mxs = mx * sc;
-      const bool raise = mxs > m_run + raise_by || m_run == -INFINITY;
-      const float m_new = raise ? fmaxf(m_run, ceilf(mxs)) : m_run;
-      const float corr = (!raise || m_new == -INFINITY) ? 1.f : pow2_whole(m_run - m_new);
-      const float ms = (m_new == -INFINITY) ? 0.f : m_new;
-      m_run = m_new;
-      // two elements per instruction where the arithmetic allows it (fma.rn.f32x2, add.rn.f32x2); the
-      // weights go straight into the tile's P buffer, which the product of two tiles ago has left
-      const float2 sc2 = make_float2(sc, sc), nms2 = make_float2(-ms, -ms);
-      float2 ps2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       // P(j) takes the place of S(j) in tensor memory: 64 weights of a row in 32 columns
       warp_whole();
 #pragma unroll
-      for (int c16 = 0; c16 < TK / 32; ++c16) {        // uniform
-        uint32_t pk[16];
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {                 // uniform
-          const float2 x = __ffma2_rn(make_float2(sv[c16 * 32 + 2 * e], sv[c16 * 32 + 2 * e + 1]), sc2, nms2);
-          const float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
-          ps2[e & 1] = __fadd2_rn(ps2[e & 1], p);
-          pk[e] = pack_bf16(p.x, p.y);
-        }
-        tmem_st16(lane_base + (uint32_t)(j & 1) * TK + c16 * 16, pk);
-      }
-      l_run = l_run * corr + ((ps2[0].x + ps2[0].y) + (ps2[1].x + ps2[1].y));
+      for (int c16 = 0; c16 < TK / 32; ++c16)          // uniform
+        tmem_st16(lane_base + (uint32_t)(j & 1) * TK + c16 * 16, reinterpret_cast<const uint32_t(&)[16]>(pk[c16 * 16]));
+      l_run = l_run * corr + psum;
 
-      if (j > 0) {
-        // O += P(j-1) V(j-1) has finished: the accumulator may be rescaled
+      // A rescaled accumulator, and the last tile's: O += P(j-1) V(j-1) has finished.  (Scores of tile j mean that O += P(j-2) V(j-2) has, so a
+      // wait by parity is for that product's end and no other.)
+      const bool rescale_now = j > 0 && rescale;
+      if (rescale_now || (j > 0 && j + 1 == n_tiles)) {
         const bool added = mbar_wait(&o_done[g], (j - 1) & 1, abortp);
         if (!added && !*abortp) { *abortp = 1; atomicCAS(&g_error, 0, 2); }
         ok = warp_all(added);
         if (!ok) break;                                // uniform
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (!warp_all(corr == 1.f)) {
+        if (rescale_now) {
 #pragma unroll
           for (int c0 = 0; c0 < HD; c0 += 16) {        // uniform
             uint32_t rr[16];
@@ -634,7 +630,8 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
       }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      mbar_arrive(&p_ready[g][j & 1]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_ready[g][j & 1]);      // one arrival a warp: 128 on one barrier stand in line
     }
     if (ok) {
       const bool added = mbar_wait(&o_done[g], (n_tiles - 1) & 1, abortp);
