@@ -39,6 +39,12 @@
 // ends at once; such blocks cost their set-up, so half as many are half the time.  Four sequences of 83 queries behind 1,000 to
 // 4,000 keys, 32 heads of 128: 46 us (two groups of queries a block: 63); five prompts of 3 to 90 tokens, 32 heads of 64: 15 us (19).
 //
+// FEW, an instance of its own: a step whose time is the chain of a few long blocks (the next turns of a few long chats).  The query heads of a
+// key/value head see the same keys, so their queries are rows of one list, a head's behind the last head's, that its blocks take 128 at a
+// time, all of them SPLIT; and the keys of a tile may go to the blocks of a cluster, a consecutive run each, which leave their
+// accumulators in shared memory and join them there, each block some of the columns, in the blocks' order.  few_form chooses by the
+// step's lengths.
+//
 // With MAPS (differential attention) the two halves of a query and of a key are two maps over the same values: the block's
 // two groups are the two maps of ONE tile of 128 queries, whose scores are products over their half of the head; keys,
 // values and queries arrive once for both.  At the end every thread reads a half of its row of both accumulators, takes
@@ -242,7 +248,28 @@ struct TileInfo {
 // What the second group does (above): queries of its own; the odd key tiles of the first group's; the next query head.
 enum { PLAIN = 0, SPLIT = 1, TWO_HEADS = 2 };
 
-template <int HD, bool MAPS>
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// an address of this block's shared memory, in the cluster's block `rank`
+__device__ __forceinline__ uint32_t peer_smem(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float4 peer_ld4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 peer_ld2(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+  return v;
+}
+constexpr int MAX_PARTS = 8;                  // blocks of a cluster that share a tile's keys
+
+template <int HD, bool MAPS, bool FEW>
 __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k_pages,
                                                                  const __grid_constant__ CUtensorMap map_v_pages,
                                                                  const __grid_constant__ CUtensorMap map_k_new,
@@ -255,7 +282,8 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
   constexpr int CPR = HD / 8;                 // 16-byte chunks per row of the head
   // The tiles need 1024-byte alignment (swizzle); the declaration asks for it and the kernel checks it.
   extern __shared__ __align__(1024) unsigned char smem[];
-  constexpr int Q_TILES = MAPS ? 1 : GROUPS;
+  constexpr int Q_TILES = MAPS || FEW ? 1 : GROUPS;
+  static_assert(!(MAPS && FEW), "two maps are two groups of one tile of queries");
   unsigned char* Qs = smem;                          // [Q_TILES]
   unsigned char* Ks = Qs + Q_TILES * Q_BYTES;        // [KST]
   unsigned char* Vs = Ks + KST * KV_BYTES;           // [VST]
@@ -264,9 +292,10 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
   __shared__ float split_share[MAPS ? 1 : GROUPS][2][MAPS ? 1 : BQ];     // SPLIT: each group's maximum and sum of a row
+  __shared__ float2 part_share[FEW ? BQ : 1];                            // this block's maximum and sum of a row
   __shared__ float map_share[MAPS ? 2 * GROUPS : 1][MAPS ? BQ : 1];      // 1 / sum of each map's weights, sums of squares
 
-  pdl_launch_dependents();
+  if (!FEW) pdl_launch_dependents();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) LLG_STAMP(5, 0, 0, blockIdx.x + gridDim.x * blockIdx.y);
   // Blocks start in the order of blockIdx.x, then blockIdx.y: all heads of the list's first tile, then all
@@ -275,7 +304,35 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
   // (lengths and tiles are the step's, written before its first kernel: they need not wait for the kernel before this one)
   TileInfo ti;
   int mode = PLAIN;
-  {
+  const int parts = FEW ? (int)gridDim.z : 1, heads_per_kv = a.nh / a.nkv;
+  int queries = 0, row0 = 0, q_off_few = 0;   // FEW: the tile's queries, the block's first row of the list, the tile's first query
+  if constexpr (FEW) {
+    const int blocks = (int)gridDim.x / a.nkv;            // of a key/value head
+    ti.b = a.tiles[2 * blockIdx.y];
+    q_off_few = a.tiles[2 * blockIdx.y + 1];
+    ti.tok0 = a.cu_tokens[ti.b];
+    ti.lb = a.len_before[ti.b];
+    ti.slot = a.slots[ti.b];
+    queries = min(GROUPS * BQ, a.cu_tokens[ti.b + 1] - ti.tok0 - q_off_few);
+    row0 = (int)blockIdx.x % blocks * BQ;
+    const int rows = min(BQ, queries * heads_per_kv - row0);
+    if (rows <= 0) return;                                // (all blocks of a cluster alike)
+    // the rows' first and last query: all of the tile's where the rows are not one head's
+    const bool one_head = row0 / queries == (row0 + rows - 1) / queries;
+    const int q_first = one_head ? row0 % queries : 0, q_last = one_head ? (row0 + rows - 1) % queries : queries - 1;
+    mode = SPLIT;
+    for (int g = 0; g < GROUPS; ++g) {
+      ti.nq[g] = rows;
+      ti.pos0[g] = ti.lb + q_off_few + q_first;
+      ti.n_tiles[g] = 0;                                  // (SPLIT: by n_max)
+    }
+    ti.k_begin = mask_first(ti.pos0[0], a.window, a.chunked) / TK * TK;
+    ti.n_max = (ti.lb + q_off_few + q_last + 1 - ti.k_begin + TK - 1) / TK;
+    // this block's run of the key tiles (the last blocks may find none left)
+    const int run = (ti.n_max + parts - 1) / parts, t0 = min((int)blockIdx.z * run, ti.n_max);
+    ti.k_begin += t0 * TK;
+    ti.n_max = min(run, ti.n_max - t0);
+  } else {
     const int tile_id = (int)blockIdx.y;
     ti.b = a.tiles[2 * tile_id];
     const int q_off = a.tiles[2 * tile_id + 1];
@@ -344,15 +401,20 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  // (a cluster's blocks come together: a block of a later kernel must not take tensor memory ahead of one of theirs and then wait for it)
+  if (FEW) pdl_launch_dependents();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base_slot;
   volatile int* abortp = &abort_flag;
   pdl_wait();
   if (tid == 0) LLG_STAMP(5, 1, 0, blockIdx.x + gridDim.x * blockIdx.y);
 
-  const int h = blockIdx.x, kvh = h / (a.nh / a.nkv);
-  const int k_end = ti.pos0[0] + (ti.nq[1] > 0 ? g_step + ti.nq[1] : ti.nq[0]);   // keys past it are never copied
-  const int q_tok0 = ti.tok0 + ti.pos0[0] - ti.lb;                              // first token of the first query tile
+  const int h = blockIdx.x, kvh = FEW ? (int)blockIdx.x / ((int)gridDim.x / a.nkv) : h / heads_per_kv;
+  const int k_end = FEW ? ti.lb + q_off_few + queries : ti.pos0[0] + (ti.nq[1] > 0 ? g_step + ti.nq[1] : ti.nq[0]);   // keys past it are never copied
+  const int q_tok0 = FEW ? ti.tok0 + q_off_few : ti.tok0 + ti.pos0[0] - ti.lb;  // first token of the first query tile
+  // FEW: a row's query among the tile's, and its head
+  auto row_query = [&](int row) { return (row0 + row) % queries; };
+  auto row_head = [&](int row) { return kvh * heads_per_kv + (row0 + row) / queries; };
 
   // queries: thread r of group g copies its part of tile g; the issuing lane waits for all of them,
   // the copying warps start on the keys and values meanwhile
@@ -363,7 +425,9 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
     const int head = h + (mode == TWO_HEADS ? g : 0);
     for (int row = r / CPR + (one_q ? g * ROWS : 0); row < BQ; row += one_q ? GROUPS * ROWS : ROWS) {
       const bool valid = row < ti.nq[g];
-      const bf16* src = (const bf16*)a.q + ((long long)(q_tok0 + g * g_step + (valid ? row : 0)) * a.nh + head) * HD + ch * 8;
+      const int at = valid ? row : 0;
+      const bf16* src = (const bf16*)a.q + ch * 8 +
+                        (FEW ? (long long)(q_tok0 + row_query(at)) * a.nh + row_head(at) : (long long)(q_tok0 + g * g_step + at) * a.nh + head) * HD;
       cp_async16(smem_u32(Qs + (one_q ? 0 : g * Q_BYTES)) + (uint32_t)((ch >> 3) * (BQ * 128)) + swz(row, ch & 7), src, valid);
     }
     cp_async_commit();
@@ -524,7 +588,9 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
     // and rounding a weight to bfloat16 gives the same bits whatever M was: how the keys are cut into tiles or
     // steps does not show in the rounded weights.
     const float sum_bound = 16384.0f;
-    const int qpos = pos0 + r;
+    const int qpos = FEW ? ti.lb + q_off_few + row_query(r) : pos0 + r;
+    // positions of the warp's first and last row, for the tiles that need no mask (FEW: of the block's)
+    const int warp_first = FEW ? pos0 : pos0 + gw * 32, warp_last = FEW ? ti.lb + q_off_few + queries - 1 : pos0 + gw * 32 + 31;
     float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     for (int j = 0; j < n_tiles; ++j) {
@@ -551,7 +617,7 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
           sv[48 + c] = __uint_as_float(r3_[c]);
         }
       }
-      const bool need_mask = (kt + TK - 1 > pos0 + gw * 32) || (a.window > 0 && kt < mask_first(pos0 + gw * 32 + 31, a.window, a.chunked));
+      const bool need_mask = (kt + TK - 1 > warp_first) || (a.window > 0 && kt < mask_first(warp_last, a.window, a.chunked));
       if (need_mask) {
 #pragma unroll
         for (int c = 0; c < TK; ++c) {
@@ -680,6 +746,59 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
           *reinterpret_cast<uint4*>(dst + c0) = v;
         }
       }
+    } else if (FEW) {
+      // the two groups meet, as above: every thread joins a half of its row's two accumulators and writes them out, or, where the
+      // keys are in parts, leaves them where queries, keys and values were (all products have read those): four columns of all rows
+      // after four columns
+      split_share[g][0][r] = m_run;
+      split_share[g][1][r] = l_run;
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      asm volatile("bar.sync 1, %0;" ::"n"(WORKERS) : "memory");
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const bool whole = warp_all(!*abortp);
+      const float m0 = split_share[0][0][r], m1 = split_share[1][0][r], m = fmaxf(m0, m1);
+      float w0 = m0 == -INFINITY ? 0.f : fast_exp2(m0 - m), w1 = m1 == -INFINITY ? 0.f : fast_exp2(m1 - m);
+      float l = split_share[0][1][r] * w0 + split_share[1][1][r] * w1;
+      if (g == 0) part_share[FEW ? r : 0] = make_float2(m, l);
+      const bool live = r < ti.nq[g];
+      const int head = live ? row_head(r) : 0, tok = q_tok0 + row_query(r);
+      if (parts == 1) {
+        if (a.has_sink) l += fast_exp2((a.sinks ? a.sinks[head] : a.sink_score) * LOG2E - m);
+        float inv = l > 0.f ? 1.0f / l : 0.f;
+        if (a.gate && live) inv *= a.gate[(long long)tok * a.nh + head];
+        w0 *= inv;
+        w1 *= inv;
+      }
+      const bool some0 = ti.n_max > 0, some1 = ti.n_max > 1;      // an accumulator that no tile went into holds anything
+      bf16* dst = (bf16*)a.out + ((long long)tok * a.nh + head) * HD;
+      const uint32_t row = tmem + O_COL + ((uint32_t)(gw * 32) << 16);
+#pragma unroll 1
+      for (int c0 = g * (HD / 2); c0 < (g + 1) * (HD / 2); c0 += 16) {
+        uint32_t r0_[16], r1_[16];
+        warp_whole();                                     // (the last columns' stores are those of the queries that there are)
+        if (whole) {                                      // uniform
+          tmem_ld16(row + c0, r0_);
+          tmem_ld16(row + G_COLS + c0, r1_);
+        }
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        float o[16];
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          o[c] = some0 ? w0 * __uint_as_float(r0_[c]) : 0.f;
+          if (some1) o[c] = fmaf(w1, __uint_as_float(r1_[c]), o[c]);
+        }
+        if (parts > 1) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            reinterpret_cast<float4*>(smem)[(c0 / 4 + q) * BQ + r] = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+        } else if (live && whole) {
+          uint4 v0, v1;
+          v0.x = pack_bf16(o[0], o[1]); v0.y = pack_bf16(o[2], o[3]); v0.z = pack_bf16(o[4], o[5]); v0.w = pack_bf16(o[6], o[7]);
+          v1.x = pack_bf16(o[8], o[9]); v1.y = pack_bf16(o[10], o[11]); v1.z = pack_bf16(o[12], o[13]); v1.w = pack_bf16(o[14], o[15]);
+          *reinterpret_cast<uint4*>(dst + c0) = v0;
+          *reinterpret_cast<uint4*>(dst + c0 + 8) = v1;
+        }
+      }
     } else if (split) {
       // the two groups meet, as above: every thread joins a half of its row's two accumulators
       split_share[g][0][r] = m_run;
@@ -747,6 +866,53 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
     }
   }
 
+  if (FEW && parts > 1) {
+    // every block of the cluster has left its accumulators and its rows' maxima and sums; this one joins some of the columns
+    __syncwarp();
+    cluster_barrier();
+    const int g = tid / BQ, r = tid % BQ;
+    if (tid < WORKERS && r < ti.nq[0]) {
+      const uint32_t ml = smem_u32(&part_share[FEW ? r : 0]), acc = smem_u32(smem) + (uint32_t)r * 16;
+      float w[MAX_PARTS], m = -INFINITY, l = 0.f;
+      float2 mls[MAX_PARTS];
+#pragma unroll
+      for (int p = 0; p < MAX_PARTS; ++p) {
+        mls[p] = p < parts ? peer_ld2(peer_smem(ml, p)) : make_float2(-INFINITY, 0.f);
+        m = fmaxf(m, mls[p].x);
+      }
+#pragma unroll
+      for (int p = 0; p < MAX_PARTS; ++p) {
+        w[p] = mls[p].x == -INFINITY ? 0.f : fast_exp2(mls[p].x - m);
+        l = fmaf(mls[p].y, w[p], l);
+      }
+      const int head = row_head(r), tok = q_tok0 + row_query(r);
+      if (a.has_sink) l += fast_exp2((a.sinks ? a.sinks[head] : a.sink_score) * LOG2E - m);
+      float inv = l > 0.f ? 1.0f / l : 0.f;
+      if (a.gate) inv *= a.gate[(long long)tok * a.nh + head];
+      bf16* dst = (bf16*)a.out + ((long long)tok * a.nh + head) * HD;
+      // runs of eight columns, the row's two threads in turn
+      for (int c8 = (int)blockIdx.z * (HD / 8 / parts) + g; c8 < ((int)blockIdx.z + 1) * (HD / 8 / parts); c8 += GROUPS) {
+        float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int p = 0; p < MAX_PARTS; ++p) {
+          if (p < parts) {
+            const uint32_t from = peer_smem(acc + (uint32_t)(2 * c8 * BQ) * 16, p);
+            const float4 u = peer_ld4(from), v = peer_ld4(from + BQ * 16);
+            o[0] = fmaf(w[p], u.x, o[0]); o[1] = fmaf(w[p], u.y, o[1]); o[2] = fmaf(w[p], u.z, o[2]); o[3] = fmaf(w[p], u.w, o[3]);
+            o[4] = fmaf(w[p], v.x, o[4]); o[5] = fmaf(w[p], v.y, o[5]); o[6] = fmaf(w[p], v.z, o[6]); o[7] = fmaf(w[p], v.w, o[7]);
+          }
+        }
+        uint4 v;
+        v.x = pack_bf16(o[0] * inv, o[1] * inv);
+        v.y = pack_bf16(o[2] * inv, o[3] * inv);
+        v.z = pack_bf16(o[4] * inv, o[5] * inv);
+        v.w = pack_bf16(o[6] * inv, o[7] * inv);
+        *reinterpret_cast<uint4*>(dst + 8 * c8) = v;
+      }
+    }
+    __syncwarp();
+    cluster_barrier();                                      // nobody leaves while another block reads its shared memory
+  }
   // every role comes here, also after a wait that ran out: copies in flight have been waited for above
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -815,13 +981,56 @@ bool kv_map(const void* base, long long rows, int nkv, int hd, CUtensorMap* resu
   return true;
 }
 
-template <int HD, bool MAPS>
-int launch(const PrefillArgs& a, cudaStream_t stream) {
+// Whether a step takes the FEW instance, and in what form: `parts` blocks that share a tile's keys (0: the other instance), `blocks` of 128 rows a
+// key/value head.  From the tiles' keys and queries on the host (a.host_tiles; without them the other instance): the form whose blocks, spread over the
+// multiprocessors, end soonest by the measured times below (us: a block, a key tile of a SPLIT block and of a PLAIN one, what parts add).  Parts only
+// where all clusters are resident at once: in two rounds of them a step takes longer than with whole keys (96 blocks of 1,399 to 2,813
+// keys: 39 us, in two parts 45; 16 of 810: 16 us, in four parts 13, in eight 25, as not quite sixteen clusters of eight fit).
+// Measured, heads of 128, 32 query and 8 key/value heads: 83 queries behind 4,000 keys 43 us in the other instance, 23 in four parts; 5 behind
+// 6,000 (40 heads) 58 and 18 in eight; 300 behind 6,000 119 and 69 whole, behind 1,000 39 and 25; two of 200 behind 3,000 and 2,000 73 and
+// 46; a prompt of 300 18 and 14, of 2,048 69 and 75; four prompts of 1,100 (heads of 64) 100 and 110.
+struct FewForm { int parts, blocks; };
+constexpr float BLOCK_US = 7.0f, SPLIT_TILE_US = 0.57f, PLAIN_TILE_US = 1.15f, JOIN_US = 4.5f;
+FewForm few_form(const PrefillArgs& a, int sms) {
+  const int per_kv = a.nh / a.nkv;
+  FewForm best{0, 0};
+  if (!a.host_tiles || (long long)a.nh * a.n_tiles > 8LL * sms) return best;
+  float best_us = 0.f;
+  int most = 0;
+  for (int parts = 0; parts <= MAX_PARTS; parts = parts ? 2 * parts : 1) {
+    float all = 0.f, longest = 0.f;
+    long long blocks = 0;
+    for (int t = 0; t < a.n_tiles; ++t) {
+      const int end = a.host_tiles[2 * t], queries = a.host_tiles[2 * t + 1], pos0 = end - queries;
+      const int first = a.window <= 0 ? 0 : a.chunked ? pos0 / a.window * a.window : (pos0 - a.window + 1 > 0 ? pos0 - a.window + 1 : 0);
+      const int tiles = (end - first / TK * TK + TK - 1) / TK, n = (queries * per_kv + BQ - 1) / BQ;
+      const long long same = parts ? (long long)parts * n * a.nkv : a.nh;
+      const float us = BLOCK_US + (parts > 1 ? JOIN_US : 0.f) +
+                       (parts ? (tiles + parts - 1) / parts * SPLIT_TILE_US : tiles * (queries > BQ ? PLAIN_TILE_US : SPLIT_TILE_US));
+      all += us * same;
+      blocks += same;
+      if (us > longest) longest = us;
+      if (n > most) most = n;
+    }
+    if (parts > 1 && blocks > (parts == 2 ? sms - sms / 16 : parts == 4 ? sms - sms / 7 : sms - sms * 3 / 10)) break;
+    const float us = blocks <= sms ? longest : fmaxf(longest, all / sms) + 0.3f * longest;
+    if (parts == 0 || us < 0.95f * best_us) {
+      best.parts = parts;
+      best_us = us;
+    }
+  }
+  best.blocks = most;
+  return best;
+}
+
+template <int HD, bool MAPS, bool FEW>
+int launch(const PrefillArgs& a, FewForm form, cudaStream_t stream) {
   constexpr int KVB = (HD / 64) * TK * 128;
-  constexpr int smem = (MAPS ? 1 : GROUPS) * (HD / 64) * BQ * 128 + (KST + VST) * KVB;
+  constexpr int smem = (MAPS || FEW ? 1 : GROUPS) * (HD / 64) * BQ * 128 + (KST + VST) * KVB;
+  static_assert(!FEW || BQ * HD * 4 <= smem, "a block's accumulators take the place of its queries, keys and values");
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<HD, MAPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<HD, MAPS, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return llg_fail("attn_prefill_tc: shared memory %d: %s", smem, cudaGetErrorString(e));
     configured = true;
   }
@@ -830,8 +1039,26 @@ int launch(const PrefillArgs& a, cudaStream_t stream) {
   if (!kv_map(a.k_pages, page_rows, 0, HD, &mkp) || !kv_map(a.v_pages, page_rows, 0, HD, &mvp) ||
       !kv_map(a.k_new, a.n_tokens, a.nkv, HD, &mkn) || !kv_map(a.v_new, a.n_tokens, a.nkv, HD, &mvn))
     return llg_fail("attn_prefill_tc: cuTensorMapEncodeTiled failed or is not available");
-  cudaError_t le = llg_launch(attn_prefill_tc_kernel<HD, MAPS>, dim3(a.nh, a.n_tiles), dim3(THREADS), (size_t)smem, stream, mkp, mvp, mkn,
-                              mvn, a);
+  cudaError_t le;
+  if (FEW) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(a.nkv * form.blocks), a.n_tiles, form.parts);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = form.parts;
+    cfg.attrs = llg_pdl_enabled() ? attr : attr + 1;
+    cfg.numAttrs = (llg_pdl_enabled() ? 1 : 0) + (form.parts > 1 ? 1 : 0);
+    le = cudaLaunchKernelEx(&cfg, attn_prefill_tc_kernel<HD, MAPS, FEW>, mkp, mvp, mkn, mvn, a);
+  } else {
+    le = llg_launch(attn_prefill_tc_kernel<HD, MAPS, FEW>, dim3(a.nh, a.n_tiles), dim3(THREADS), (size_t)smem, stream, mkp, mvp, mkn, mvn, a);
+  }
   if (le != cudaSuccess) return llg_fail("attn_prefill_tc: launch: %s", cudaGetErrorString(le));
   return llg_check_launch("attn_prefill_tc");
 }
@@ -840,6 +1067,10 @@ int launch(const PrefillArgs& a, cudaStream_t stream) {
 
 // 1 when this kernel takes the head size (bfloat16 only): 64 or 128.
 LLG_API int llg_attn_tc_supported(int hd) { return hd == 64 || hd == 128; }
+
+// Blocks that share a tile's keys for these sizes (n_tiles, nh, nkv, window, chunked and host_tiles of `args`) on a GPU of `sms` multiprocessors;
+// 0 where the step takes the instance for long prompts.
+LLG_API int llg_attn_prefill_parts(const PrefillArgs* args, int sms) { return few_form(*args, sms).parts; }
 
 LLG_API int llg_attn_prefill_tc(const PrefillArgs* args, cudaStream_t stream) {
   const PrefillArgs& a = *args;
@@ -858,9 +1089,11 @@ LLG_API int llg_attn_prefill_tc(const PrefillArgs* args, cudaStream_t stream) {
   LLG_REQUIRE(a.maps == 0 || a.maps == 2, "attn_prefill_tc: %d maps (0 or 2)", a.maps);
   if (a.maps == 2) {
     LLG_REQUIRE(!a.has_sink && !a.gate && a.map_eps > 0.f, "attn_prefill_tc: two maps go with neither a sink nor gates");
-    return a.hd == 64 ? launch<64, true>(a, stream) : launch<128, true>(a, stream);
+    return a.hd == 64 ? launch<64, true, false>(a, {}, stream) : launch<128, true, false>(a, {}, stream);
   }
-  return a.hd == 64 ? launch<64, false>(a, stream) : launch<128, false>(a, stream);
+  const FewForm form = few_form(a, llg_sm_count());
+  if (form.parts > 0) return a.hd == 64 ? launch<64, false, true>(a, form, stream) : launch<128, false, true>(a, form, stream);
+  return a.hd == 64 ? launch<64, false, false>(a, {}, stream) : launch<128, false, false>(a, {}, stream);
 }
 
 // Error code recorded when a wait ran out (0 = none); clears it.  Synchronises the device.

@@ -94,6 +94,7 @@ struct RunnerStep {
   const int* len_before;
   const int* tiles;                         // prompt steps: the query tiles of the attention kernel in use
   int n_tiles;
+  const int* host_tiles;                    // the tiles' sizes in host memory (PrefillArgs)
   int max_len_after;
   int prefill_kind;                         // 0 CUDA cores, 1 mma.sync, 2 tcgen05
   int decode_kind;                          // 0 CUDA cores, 1 mma.sync, 2 TMA
@@ -306,6 +307,7 @@ int run_block(const DenseLayer& L, const RunnerStep& s, const float* pending, in
     a.window = L.window;
     a.n_tokens = n;
     a.n_pages = L.n_pages;
+    a.host_tiles = s.host_tiles;
     int rc;
     const char* (*err)();
     if (s.prefill_kind == 2) {

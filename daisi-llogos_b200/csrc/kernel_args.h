@@ -137,6 +137,9 @@ struct PrefillArgs {
   // the head and multiplied by map_scale.
   int maps;
   float map_lambda, map_eps, map_scale;
+  // null, or in HOST memory [n_tiles][2]: how many keys a tile's last query sees (the sequence's length there) and the tile's queries.
+  // Read at the launch only (attention_tc.cu chooses by it how many blocks share a tile's keys).
+  const int* host_tiles;
 };
 
 // Attention of one new token per sequence, split kernels (attention_simt.cu, attention_mma.cu).

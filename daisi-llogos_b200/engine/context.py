@@ -99,4 +99,6 @@ class StepContext:
             else:
                 dev.copy_(torch.from_numpy(host))
             tiles = self.extras[key] = dev.view(-1, 2)
+            # what the launch may read of them without the device: a tile's last key's place and its queries
+            tiles.host_sizes = np.asarray([(lb[b] + min(counts[b], q0 + tq), min(counts[b] - q0, tq)) for b, q0 in order], dtype=np.int32)
         return tiles

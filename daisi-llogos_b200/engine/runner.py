@@ -56,7 +56,7 @@ class _RunnerStep(Structure):
         ("n_tokens", c_int), ("n_seqs", c_int), ("decode", c_int), ("dtype", c_int),
         ("hidden", c_int), ("nh", c_int), ("nkv", c_int), ("hd", c_int), ("inter", c_int),
         ("positions", c_void_p), ("seq_of_token", c_void_p), ("slots", c_void_p), ("cu_tokens", c_void_p),
-        ("len_before", c_void_p), ("tiles", c_void_p), ("n_tiles", c_int), ("max_len_after", c_int),
+        ("len_before", c_void_p), ("tiles", c_void_p), ("n_tiles", c_int), ("host_tiles", c_void_p), ("max_len_after", c_int),
         ("prefill_kind", c_int), ("decode_kind", c_int), ("decode_splits", c_int), ("decode_balance", c_int),
         ("tc_qkv", c_int), ("tc_o", c_int), ("tc_gate_up", c_int), ("tc_down", c_int),
         ("splits_qkv", c_int), ("splits_o", c_int), ("splits_down", c_int), ("fused_qkv", c_int),
@@ -255,13 +255,13 @@ class BlockRunner:
             s.attn_scratch = ctx.buffer("attn.scratch", (max(1, plan.scratch_floats),), torch.float32).data_ptr()
             s.attn_counters = (ctx.buffer("attn.counters", (plan.n_counters,), torch.int32, zero=True).data_ptr()
                                if plan.n_counters else None)
-            s.tiles, s.n_tiles, s.k_new, s.v_new = None, 0, None, None
+            s.tiles, s.n_tiles, s.host_tiles, s.k_new, s.v_new = None, 0, None, None, None
         else:
             s.k_new = ctx.buffer("attn.k_new", (n, nkv, hd)).data_ptr()
             s.v_new = ctx.buffer("attn.v_new", (n, nkv, hd)).data_ptr()
             tq = ops.prefill_tile_queries(dtype, hd)
             tiles = ctx.query_tiles(tq)
-            s.tiles, s.n_tiles = tiles.data_ptr(), tiles.shape[0]
+            s.tiles, s.n_tiles, s.host_tiles = tiles.data_ptr(), tiles.shape[0], ops.tile_sizes_ptr(tiles)
             s.prefill_kind = 2 if ops._use_tc_attn(dtype, hd) else 1 if ops._use_mma(dtype, hd) else 0
         need = ["add_rmsnorm"] + (["gemm_tc_qkv"] if s.fused_qkv else ["qk_prep"])
         need.append("gemm_tc" if (s.tc_qkv or s.tc_o or s.tc_down or (s.tc_gate_up and bf16)) else "gemm_simt")

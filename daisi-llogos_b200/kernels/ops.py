@@ -159,6 +159,7 @@ class _PrefillArgs(Structure):
         ("vd", c_int), ("has_sink", c_int), ("sink_score", c_float), ("gate", c_void_p),
         ("sinks", c_void_p), ("chunked", c_int), ("softcap", c_float), ("head_mix", c_void_p),
         ("out_f32", c_int), ("maps", c_int), ("map_lambda", c_float), ("map_eps", c_float), ("map_scale", c_float),
+        ("host_tiles", c_void_p),
     ]
 
 
@@ -468,6 +469,7 @@ def _load_lib(name: str):
     elif name == "attention_tc":
         lib.llg_attn_tc_supported.argtypes = [c_int]
         lib.llg_attn_prefill_tc.argtypes = [POINTER(_PrefillArgs), c_void_p]
+        lib.llg_attn_prefill_parts.argtypes = [POINTER(_PrefillArgs), c_int]
         lib.llg_attn_tc_status.restype = c_int
     elif name == "attention_decode_tma":
         lib.llg_attn_decode_tma_supported.argtypes = [c_int, c_int, c_int, c_int]
@@ -1904,12 +1906,28 @@ def attn_tc_status() -> int:
     return _lib("attention_tc").llg_attn_tc_status()
 
 
+def tile_sizes_ptr(tiles: torch.Tensor) -> Optional[int]:
+    """Address of the sizes that ``StepContext.query_tiles`` leaves beside its tiles (``PrefillArgs.host_tiles``), or ``None``."""
+    sizes = getattr(tiles, "host_sizes", None)
+    return None if sizes is None else sizes.ctypes.data
+
+
+def attn_prefill_parts(tile_sizes, n_heads: int, n_kv_heads: int, window: int, sms: int) -> int:
+    """Blocks that the tcgen05 prompt attention lets share a tile's keys on a GPU of ``sms`` multiprocessors (0: the instance for long
+    prompts); ``tile_sizes``: int32 ``[n_tiles, 2]`` on the host (``PrefillArgs.host_tiles``)."""
+    a = _PrefillArgs()
+    a.n_tiles, a.nh, a.nkv, a.window = len(tile_sizes), n_heads, n_kv_heads, int(window)
+    a.host_tiles = tile_sizes.ctypes.data
+    return _lib("attention_tc").llg_attn_prefill_parts(byref(a), sms)
+
+
 def attn_prefill(q, k_new, v_new, k_pages, v_pages, page_table, ring_pages, tiles, cu_tokens, len_before,
                  slots, out, *, scale: float, window: int, tile_queries: int,
                  form: AttentionForm = PLAIN_ATTENTION, gate: Optional[torch.Tensor] = None) -> None:
     """Causal attention for a step with several tokens per sequence.
 
-    ``tiles`` is ``[n_tiles, 2]`` (sequence index, first query among its step tokens) cut every
+    ``tiles`` is ``[n_tiles, 2]`` (sequence index, first query among its step tokens; as ``StepContext.query_tiles`` makes it, with
+    the tiles' sizes on the host beside it) cut every
     ``tile_queries`` queries, which must be ``prefill_tile_queries(q.dtype, head_dim)``.  bfloat16 runs on
     the tensor cores: head sizes 64 and 128 with tcgen05 (csrc/attention_tc.cu), other multiples of 16 up
     to 128 with mma.sync (csrc/attention_mma.cu); everything else on the CUDA cores
@@ -1943,6 +1961,7 @@ def attn_prefill(q, k_new, v_new, k_pages, v_pages, page_table, ring_pages, tile
     a.scale, a.window = float(scale), int(window)
     a.n_tokens, a.n_pages = k_new.shape[0], k_pages.shape[0]
     _set_form(a, form, hd, gate)
+    a.host_tiles = tile_sizes_ptr(tiles)
     if own_maps:
         a.out_f32, a.maps, a.map_lambda, a.map_eps, a.map_scale = 0, 2, form.maps.lam, form.maps.eps, form.maps.scale
     if mix_mma:

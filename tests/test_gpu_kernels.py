@@ -4,6 +4,7 @@ numbers of heads and groups."""
 import importlib
 import math
 
+import numpy as np
 import pytest
 import torch
 
@@ -480,6 +481,56 @@ def test_attn_prefill_of_few_queries_per_sequence(ops, hd, nh, nkv, before, coun
             ref = ref * (share * gate[int(cu[b]):int(cu[b + 1])].double())[:, :, None]
         ref = ref.reshape(counts[b], -1)
         check(out[int(cu[b]):int(cu[b + 1])], ref, dtype, ("sequence", b))
+
+
+@pytest.mark.parametrize("before,counts,nh,nkv,window,parts", [
+    ([3000], [5], 8, 2, 0, 8),                            # one list of twenty rows
+    ([1200], [20], 4, 4, 0, 8),                           # twenty key tiles: the last block of a cluster finds none left
+    ([1000, 0], [200, 40], 6, 2, 0, 8),                   # rows of one head and of several, a tile of fewer blocks, one of one key tile
+    ([1400, 64, 700, 0], [83, 3, 130, 70], 32, 8, 0, 1),
+    ([1400, 64, 700, 0], [83, 3, 130, 70], 16, 4, 0, 2),
+    ([1000], [83], 32, 8, 0, 4),
+    ([1500], [150], 4, 1, 900, 8),                        # a window: parts that some rows see nothing of
+    ([300], [260], 16, 2, 0, 1),                          # two tiles of a sequence
+    ([0] * 5, [48, 49, 11, 51, 34], 32, 8, 0, 1),         # one key tile each: the second group has none
+    ([100], [20], 4, 4, 0, 0),                            # the instance for prompts
+], ids=["rows", "none left", "several heads", "ragged", "two parts", "four parts", "window", "two tiles", "short", "prompts"])
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("sinks", [False, True], ids=["", "sinks and a gate"])
+def test_attn_prefill_of_few_long_sequences(ops, hd, before, counts, nh, nkv, window, parts, sinks):
+    """Few blocks and many keys: the heads' queries in one list, and the blocks of a cluster take a run of a tile's keys each."""
+    dtype, scale = torch.bfloat16, 1 / math.sqrt(hd)
+    total = [a + c for a, c in zip(before, counts)]
+    ring = 64 if window == 0 else (window + 63) // 64 + 1
+    kp, vp, table, slots, ks, vs = _paged(nkv, hd, dtype, total, 51, ring, 160)
+    for b, n in enumerate(before):                       # the cache as it was before the step
+        for p in range(max(0, n - ring * 64), n):
+            pg = int(table[slots[b], (p // 64) % ring])
+            kp[pg, :, p % 64], vp[pg, :, p % 64] = ks[b][p], vs[b][p]
+    cu = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32)
+    q = rnd((int(cu[-1]), nh, hd), 52, dtype)
+    k_new, v_new = (torch.cat([t[b][before[b]:] for b in range(len(counts))]) for t in (ks, vs))
+    sink = 3.0 * rnd((nh,), 53) if sinks else None
+    gate = torch.rand((int(cu[-1]), nh), generator=torch.Generator().manual_seed(54)) if sinks else None
+    form = ops.AttentionForm(sinks=sink.to(DEV), gated=True) if sinks else ops.PLAIN_ATTENTION
+    tq = ops.prefill_tile_queries(dtype, hd, form)
+    order = [(b, q0) for b, c in enumerate(counts) for q0 in range(0, c, tq)]
+    tiles = torch.tensor(order, dtype=torch.int32, device=DEV)
+    tiles.host_sizes = np.asarray([(before[b] + min(counts[b], q0 + tq), min(counts[b] - q0, tq)) for b, q0 in order], dtype=np.int32)
+    assert ops.attn_prefill_parts(tiles.host_sizes, nh, nkv, window, 148) == parts
+    out = torch.full((int(cu[-1]), nh * hd), float("nan"), dtype=dtype, device=DEV)
+    d = lambda t: t.to(DEV)
+    ops.attn_prefill(d(q), d(k_new), d(v_new), d(kp), d(vp), d(table), ring, tiles, d(cu), d(torch.tensor(before, dtype=torch.int32)),
+                     d(slots), out, scale=scale, window=window, tile_queries=tq, form=form, gate=d(gate) if sinks else None)
+    assert ops.attn_tc_status() == 0
+    for b in range(len(counts)):
+        qq = torch.zeros(total[b], nh, hd, dtype=dtype)
+        qq[before[b]:] = q[int(cu[b]):int(cu[b + 1])]
+        ref = P.attention(qq, ks[b], vs[b], scale, window)[before[b]:]
+        if sinks:
+            share = torch.sigmoid(_log_sum(qq, ks[b], scale, window)[before[b]:] - sink.double())
+            ref = ref * (share * gate[int(cu[b]):int(cu[b + 1])].double())[:, :, None]
+        check(out[int(cu[b]):int(cu[b + 1])], ref.reshape(counts[b], -1), dtype, ("sequence", b))
 
 
 @pytest.mark.parametrize("tc", [True, False], ids=["tcgen05", "mma"])
