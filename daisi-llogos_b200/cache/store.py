@@ -21,6 +21,7 @@ from typing import Dict, List, Optional, Sequence, Tuple
 
 import torch
 
+from ..kernels import ops as kernel_ops
 from ..parts.base import KvNeed, MultiNeed, StateNeed
 from .slots import CacheError, FreeList, SlotTable
 
@@ -199,6 +200,8 @@ class SequenceCache:
                 self.state[unit] = torch.zeros((n_slots + 1, *need.shape), dtype=need.dtype, device=device)
             else:
                 raise TypeError(f"cache unit {unit}: unknown need {need!r}")
+        # on the GPU a slot's state is zeroed by one launch for all units
+        self._state_rows = kernel_ops.SlotRows(self.state.values()) if self.state and torch.device(device).type == "cuda" else None
         for need, units in by_need.items():
             g = KvGroup(need, units, self.n_pages, n_slots, pages_for(self.max_seq_len), dtype, device)
             self.kv_groups.append(g)
@@ -210,8 +213,11 @@ class SequenceCache:
         """A fresh slot: length 0, no pages, state zeroed."""
         slot = self.slots.acquire()
         self._longest.pop(slot, None)
-        for t in self.state.values():
-            t[slot].zero_()
+        if self._state_rows is not None:
+            self._state_rows.zero(slot)
+        else:
+            for t in self.state.values():
+                t[slot].zero_()
         return slot
 
     def release(self, slot: int) -> None:

@@ -969,6 +969,37 @@ LLG_API int llg_zero_rows(void* base, const int* rows, int n_rows, long long row
   return llg_check_launch("zero_rows");
 }
 
+// A slot's rows of all of a cache's state tensors, in one launch: a sequence that starts has one launch to wait for, not one a tensor
+// (what a tensor cost was the host's time for a launch, 7 to 9 us, the GPU idle).
+// Rows are blockIdx.y, ZERO_BLOCKS blocks share a row; 16 bytes a store where the row lies on 16 bytes.
+constexpr int ZERO_ROWS = 32, ZERO_BLOCKS = 16;
+struct ZeroRows {
+  unsigned char* row[ZERO_ROWS];
+  long long bytes[ZERO_ROWS];
+};
+__global__ void __launch_bounds__(256) zero_slot_kernel(ZeroRows a) {
+  unsigned char* p = a.row[blockIdx.y];
+  const long long bytes = a.bytes[blockIdx.y], at = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)ZERO_BLOCKS * blockDim.x;
+  const long long wide = ((uintptr_t)p & 15u) == 0 ? bytes / 16 : 0;
+  for (long long i = at; i < wide; i += step) reinterpret_cast<uint4*>(p)[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (long long i = wide * 16 + at; i < bytes; i += step) p[i] = 0;
+}
+
+// Zeroes row `slot` of n tensors: base[i] is tensor i's first row, row_bytes[i] its rows' size.
+LLG_API int llg_zero_slot(void* const* base, const long long* row_bytes, int n, int slot, cudaStream_t stream) {
+  LLG_REQUIRE(n >= 0 && slot >= 0, "zero_slot: %d tensors, slot %d", n, slot);
+  for (int i0 = 0; i0 < n; i0 += ZERO_ROWS) {
+    ZeroRows a;
+    const int m = n - i0 < ZERO_ROWS ? n - i0 : ZERO_ROWS;
+    for (int i = 0; i < m; ++i) {
+      a.row[i] = (unsigned char*)base[i0 + i] + slot * row_bytes[i0 + i];
+      a.bytes[i] = row_bytes[i0 + i];
+    }
+    zero_slot_kernel<<<dim3(ZERO_BLOCKS, m), 256, 0, stream>>>(a);
+  }
+  return llg_check_launch("zero_slot");
+}
+
 // ---- residual in several streams (hyper-connections) ----------------------------------
 
 // See HyperNormArgs in kernel_args.h.  One block per output row; the read-out u stays in shared memory between the

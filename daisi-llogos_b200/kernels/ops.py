@@ -420,6 +420,7 @@ def _load_lib(name: str):
         lib.llg_scatter_i32.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_void_p]
         lib.llg_gather_i32.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_void_p]
         lib.llg_zero_rows.argtypes = [c_void_p, c_void_p, c_int, c_longlong, c_void_p]
+        lib.llg_zero_slot.argtypes = [c_void_p, c_void_p, c_int, c_int, c_void_p]
         lib.llg_hc_add_rmsnorm.argtypes = [POINTER(_HyperNormArgs), c_void_p]
         lib.llg_qkv_row_prep.argtypes = [POINTER(_QkvRowPrepArgs), c_int, c_void_p]
         lib.llg_act_rows.argtypes = [c_void_p, c_int, c_int, c_longlong, c_void_p, c_int, c_longlong, c_int, c_void_p]
@@ -1745,6 +1746,26 @@ def zero_rows(base: torch.Tensor, rows: torch.Tensor) -> None:
     lib = _lib("elementwise")
     row_bytes = (base.numel() // base.shape[0]) * base.element_size() if base.shape[0] else 0
     _check(lib, lib.llg_zero_rows(_ptr(base), _ptr(rows, torch.int32), rows.numel(), row_bytes, _stream()))
+
+
+class SlotRows:
+    """Tensors ``[n_slots, ...]`` whose rows of one slot are zeroed together (``zero``): one launch for all of them."""
+
+    def __init__(self, tensors):
+        self.tensors = list(tensors)                  # kept alive: the addresses below are theirs
+        n = len(self.tensors)
+        self.n_slots = min((t.shape[0] for t in self.tensors), default=0)
+        self.base = (c_void_p * n)(*[_ptr(t) for t in self.tensors])
+        self.row_bytes = (c_longlong * n)(*[t[0].numel() * t.element_size() for t in self.tensors])
+
+    def zero(self, slot: int) -> None:
+        if not self.tensors:
+            return
+        if not 0 <= slot < self.n_slots:
+            raise KernelError(f"SlotRows: slot {slot} of {self.n_slots}")
+        lib = _lib("elementwise")
+        with torch.cuda.device(self.tensors[0].device):
+            _check(lib, lib.llg_zero_slot(self.base, self.row_bytes, len(self.tensors), slot, _stream()))
 
 
 def _use_mma(dtype: torch.dtype, head_dim: int) -> bool:

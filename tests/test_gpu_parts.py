@@ -827,3 +827,15 @@ def test_toy_architecture_with_a_configuration_and_a_norm_of_its_own(llogos, tmp
     finally:
         Pt.unregister_part("norm", "toy_mean_variance")
         reg._ARCHITECTURES.pop("ToyOwnConfigLM", None)
+
+
+def test_a_slots_rows_are_zeroed_together(ops):
+    """More tensors than a launch takes, rows of one byte, of no whole 16 bytes and of many: the slot's rows and no others."""
+    tensors = [torch.full((3, n), 1, dtype=dt, device=DEV) for n in (1, 5, 16, 1000, 70001) for dt in (torch.float32, torch.bfloat16, torch.int32)]
+    tensors += [torch.full((4, 2, 3), 1, dtype=torch.uint8, device=DEV) for _ in range(25)]
+    rows = ops.SlotRows(tensors)
+    rows.zero(1)
+    for t in tensors:
+        assert not bool(t[1].any()) and bool((t[0] == 1).all()) and bool((t[2:] == 1).all())
+    with pytest.raises(ops.KernelError):
+        rows.zero(3)
