@@ -682,7 +682,7 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
         ok = warp_all(added);
         if (!ok) break;                                // uniform
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (rescale_now) {
+        if (rescale_now) {                             // uniform: rescale is one answer for the warp
 #pragma unroll
           for (int c0 = 0; c0 < HD; c0 += 16) {        // uniform
             uint32_t rr[16];
