@@ -172,26 +172,24 @@ __global__ void __launch_bounds__(128) attn_prefill_kernel(PrefillArgs a) {
 
 // GC: query heads of one key/value head handled per pass (4 or 8: the smaller where it takes them all).  MAXD: value elements a
 // lane holds, 32 apart; with the head's own size instead of the largest the accumulators leave registers for rows in flight.
-// Bound by latency: a warp owns a tile of 32 keys.  Heads of at most 64 float32 elements (WHOLE): all key and value rows of the warp's first
-// tile are asked for before the kernel waits for the one ahead (lengths, page table and the rows of older tokens are no result of it; the
-// newest token's row is, and comes after the wait), so that one trip to memory, most of it hidden, stands before the arithmetic.
-// The others read ROWS key rows, then value rows, at a time.  Three sequences of 10 to 35 keys, 32 heads of 64: 4 us less a layer of a step.
+// Bound by latency: a warp owns a tile of 32 keys and reads ROWS key rows (then value rows) at a time before it uses the first,
+// where one row at a time cost a trip to memory each.  3 sequences of about 100 keys, 32 heads of 64: 68 us before, 12 now.
 template <typename T, int MAXD, int GC>
 __global__ void __launch_bounds__(128) attn_decode_kernel(DecodeArgs a) {
-  constexpr bool WHOLE = MAXD <= 2 && sizeof(T) == 4;      // (two bytes an element: the conversions take the registers that this wants)
   constexpr int ROWS = MAXD <= 2 ? 16 : MAXD <= 4 ? 8 : 4;
-  extern __shared__ __align__(16) float sm[];
+  extern __shared__ float sm[];
   pdl_launch_dependents();
+  pdl_wait();
   const int hd = a.hd, vd = a.vd > 0 ? a.vd : a.hd;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
   const int G = a.nh / a.nkv;
-  float* Qs = sm;                                   // [hd][GC]
+  float* Qs = sm;                                   // [GC][hd]
   float* Kt = Qs + GC * hd + warp * (KT * (hd + 1) + GC * KT);   // per warp: [KT][hd + 1]
   float* Pw = Kt + KT * (hd + 1);                   // per warp: [GC][KT]
   float* merge = Qs + GC * hd;                      // reused after the key loop: [4][GC][vd + 2]
 
-  const int len = a.len_before[b] + 1, newest = len - 1;
+  const int len = a.len_before[b] + 1;
   const int slot = a.slots[b];
   const int lo = mask_first(len - 1, a.window, a.chunked);
   const int t0 = lo / KT, t_end = (len + KT - 1) / KT;
@@ -200,32 +198,13 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(DecodeArgs a) {
   const int my1 = min(t_end, my0 + per_split);
   const T* kp_base = (const T*)a.k_pages;
   const T* vp_base = (const T*)a.v_pages;
-  // the rows of a tile but the newest token's: row u, elements lane + 32 dd
-  T kr[WHOLE ? KT : 1][MAXD], vr[WHOLE ? KT : 1][MAXD];
-  auto fetch = [&](int t) {
-    const int kp = t * KT + lane;
-    const bool old = kp >= lo && kp < newest;
-    const long long row = old ? kv_row(a.page_table, a.table_width, a.ring_pages, slot, kp, kvh, a.nkv) : -1;
-#pragma unroll
-    for (int u = 0; u < (WHOLE ? KT : 1); ++u) {
-      const long long rj = __shfl_sync(0xffffffffu, row, u);
-#pragma unroll
-      for (int dd = 0; dd < MAXD; ++dd) {
-        const int d = lane + 32 * dd;
-        kr[u][dd] = rj >= 0 && d < hd ? kp_base[rj * hd + d] : from_f32<T>(0.f);
-        vr[u][dd] = rj >= 0 && d < vd ? vp_base[rj * vd + d] : from_f32<T>(0.f);
-      }
-    }
-  };
-  if (WHOLE && my0 + warp < my1) fetch(my0 + warp);
-  pdl_wait();
 
   for (int g0 = 0; g0 < G; g0 += GC) {
     const int ng = min(GC, G - g0);
     __syncthreads();
     for (int idx = tid; idx < GC * hd; idx += 128) {
       const int g = idx / hd, d = idx % hd;
-      Qs[d * GC + g] = g < ng ? to_f32(((const T*)a.q)[((long long)b * a.nh + kvh * G + g0 + g) * hd + d]) : 0.f;
+      Qs[idx] = g < ng ? to_f32(((const T*)a.q)[((long long)b * a.nh + kvh * G + g0 + g) * hd + d]) : 0.f;
     }
     __syncthreads();
     float m[GC], l[GC], acc[GC][MAXD];
@@ -239,61 +218,28 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(DecodeArgs a) {
     for (int t = my0 + warp; t < my1; t += 4) {
       const int kp = t * KT + lane;
       const bool valid = kp >= lo && kp < len;
-      const int fresh = newest - t * KT;                // the newest token's row, if this tile has it
-      const bool has_fresh = fresh < KT;
-      long long row = 0;
-      float vn[MAXD];                                   // WHOLE: its values
-      if (WHOLE) {
-        if (t != my0 + warp || g0 > 0) fetch(t);
-        float kn[MAXD];
-        if (has_fresh) {
-          const long long rn = kv_row(a.page_table, a.table_width, a.ring_pages, slot, newest, kvh, a.nkv);
-#pragma unroll
-          for (int dd = 0; dd < MAXD; ++dd) {
-            const int d = lane + 32 * dd;
-            kn[dd] = d < hd ? to_f32(kp_base[rn * hd + d]) : 0.f;
-            vn[dd] = d < vd ? to_f32(vp_base[rn * vd + d]) : 0.f;
-          }
-        }
-        __syncwarp();
-#pragma unroll
-        for (int u = 0; u < (WHOLE ? KT : 1); ++u)
-#pragma unroll
-          for (int dd = 0; dd < MAXD; ++dd) {
-            const int d = lane + 32 * dd;
-            if (d < hd) Kt[u * (hd + 1) + d] = to_f32(kr[u][dd]);
-          }
-        if (has_fresh) {
-#pragma unroll
-          for (int dd = 0; dd < MAXD; ++dd) {
-            const int d = lane + 32 * dd;
-            if (d < hd) Kt[fresh * (hd + 1) + d] = kn[dd];
-          }
-        }
-      } else {
-        row = valid ? kv_row(a.page_table, a.table_width, a.ring_pages, slot, kp, kvh, a.nkv) : 0;
-        __syncwarp();
+      const long long row = valid ? kv_row(a.page_table, a.table_width, a.ring_pages, slot, kp, kvh, a.nkv) : 0;
+      __syncwarp();
 #pragma unroll 1
-        for (int j0 = 0; j0 < KT; j0 += ROWS) {
-          float k8[ROWS][MAXD];
+      for (int j0 = 0; j0 < KT; j0 += ROWS) {
+        float kr[ROWS][MAXD];
 #pragma unroll
-          for (int u = 0; u < ROWS; ++u) {
-            const long long rj = __shfl_sync(0xffffffffu, row, j0 + u);
-            const bool vj = __shfl_sync(0xffffffffu, (int)valid, j0 + u);
+        for (int u = 0; u < ROWS; ++u) {
+          const long long rj = __shfl_sync(0xffffffffu, row, j0 + u);
+          const bool vj = __shfl_sync(0xffffffffu, (int)valid, j0 + u);
 #pragma unroll
-            for (int dd = 0; dd < MAXD; ++dd) {
-              const int d = lane + 32 * dd;
-              k8[u][dd] = vj && d < hd ? to_f32(kp_base[rj * hd + d]) : 0.f;
-            }
+          for (int dd = 0; dd < MAXD; ++dd) {
+            const int d = lane + 32 * dd;
+            kr[u][dd] = vj && d < hd ? to_f32(kp_base[rj * hd + d]) : 0.f;
           }
-#pragma unroll
-          for (int u = 0; u < ROWS; ++u)
-#pragma unroll
-            for (int dd = 0; dd < MAXD; ++dd) {
-              const int d = lane + 32 * dd;
-              if (d < hd) Kt[(j0 + u) * (hd + 1) + d] = k8[u][dd];
-            }
         }
+#pragma unroll
+        for (int u = 0; u < ROWS; ++u)
+#pragma unroll
+          for (int dd = 0; dd < MAXD; ++dd) {
+            const int d = lane + 32 * dd;
+            if (d < hd) Kt[(j0 + u) * (hd + 1) + d] = kr[u][dd];
+          }
       }
       __syncwarp();
       const float* krow = Kt + lane * (hd + 1);
@@ -304,83 +250,47 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(DecodeArgs a) {
       for (int d = 0; d < hd; ++d) {
         const float kd = krow[d];
 #pragma unroll
-        for (int g4 = 0; g4 < GC; g4 += 4) {            // rows of absent heads are zero
-          const float4 q = *reinterpret_cast<const float4*>(Qs + d * GC + g4);
-          dot[g4] = fmaf(q.x, kd, dot[g4]);
-          dot[g4 + 1] = fmaf(q.y, kd, dot[g4 + 1]);
-          dot[g4 + 2] = fmaf(q.z, kd, dot[g4 + 2]);
-          dot[g4 + 3] = fmaf(q.w, kd, dot[g4 + 3]);
-        }
-      }
-      // (absent heads go along: without a branch the heads' chains of exchanges overlap)
-      float top[GC], sum[GC];
-#pragma unroll
-      for (int g = 0; g < GC; ++g) {
-        dot[g] = valid ? dot[g] * a.scale : -INFINITY;
-        top[g] = warp_max(dot[g]);
+        for (int g = 0; g < GC; ++g) dot[g] = fmaf(Qs[g * hd + d], kd, dot[g]);      // rows of absent heads are zero
       }
 #pragma unroll
       for (int g = 0; g < GC; ++g) {
-        const float m_new = fmaxf(m[g], top[g]);
+        if (g >= ng) break;
+        const float s = valid ? dot[g] * a.scale : -INFINITY;
+        const float m_new = fmaxf(m[g], warp_max(s));
         float corr = 1.f, p = 0.f;
         if (m_new != -INFINITY) {
           corr = expf(m[g] - m_new);
-          p = valid ? expf(dot[g] - m_new) : 0.f;
+          p = valid ? expf(s - m_new) : 0.f;
         }
-        l[g] *= corr;
-        sum[g] = p;
+        l[g] = l[g] * corr + warp_sum(p);
         m[g] = m_new;
         Pw[g * KT + lane] = p;
 #pragma unroll
         for (int dd = 0; dd < MAXD; ++dd) acc[g][dd] *= corr;
       }
-#pragma unroll
-      for (int g = 0; g < GC; ++g) l[g] += warp_sum(sum[g]);
       __syncwarp();
-      if (WHOLE) {
-#pragma unroll
-        for (int u0 = 0; u0 < (WHOLE ? KT : 4); u0 += 4)
-#pragma unroll
-          for (int g = 0; g < GC; ++g) {
-            const float4 p4 = *reinterpret_cast<const float4*>(Pw + g * KT + u0);
-            const float p[4] = {p4.x, p4.y, p4.z, p4.w};
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-              for (int dd = 0; dd < MAXD; ++dd) acc[g][dd] = fmaf(p[u], to_f32(vr[WHOLE ? u0 + u : 0][dd]), acc[g][dd]);
-          }
-        if (has_fresh) {
-#pragma unroll
-          for (int g = 0; g < GC; ++g) {
-            const float p = Pw[g * KT + fresh];
-#pragma unroll
-            for (int dd = 0; dd < MAXD; ++dd) acc[g][dd] = fmaf(p, vn[dd], acc[g][dd]);
-          }
-        }
-      } else {
 #pragma unroll 1
-        for (int j0 = 0; j0 < KT; j0 += ROWS) {
-          float v8[ROWS][MAXD];
+      for (int j0 = 0; j0 < KT; j0 += ROWS) {
+        float vr[ROWS][MAXD];
 #pragma unroll
-          for (int u = 0; u < ROWS; ++u) {
-            const bool vj = __shfl_sync(0xffffffffu, (int)valid, j0 + u);
-            const long long rj = __shfl_sync(0xffffffffu, row, j0 + u);
+        for (int u = 0; u < ROWS; ++u) {
+          const bool vj = __shfl_sync(0xffffffffu, (int)valid, j0 + u);
+          const long long rj = __shfl_sync(0xffffffffu, row, j0 + u);
 #pragma unroll
-            for (int dd = 0; dd < MAXD; ++dd) {
-              const int d = lane + 32 * dd;
-              v8[u][dd] = vj && d < vd ? to_f32(vp_base[rj * vd + d]) : 0.f;
-            }
+          for (int dd = 0; dd < MAXD; ++dd) {
+            const int d = lane + 32 * dd;
+            vr[u][dd] = vj && d < vd ? to_f32(vp_base[rj * vd + d]) : 0.f;
           }
-#pragma unroll
-          for (int u = 0; u < ROWS; ++u)
-#pragma unroll
-            for (int g = 0; g < GC; ++g)
-              if (g < ng) {
-                const float p = Pw[g * KT + j0 + u];      // 0 for a key that the query does not see
-#pragma unroll
-                for (int dd = 0; dd < MAXD; ++dd) acc[g][dd] = fmaf(p, v8[u][dd], acc[g][dd]);
-              }
         }
+#pragma unroll
+        for (int u = 0; u < ROWS; ++u)
+#pragma unroll
+          for (int g = 0; g < GC; ++g)
+            if (g < ng) {
+              const float p = Pw[g * KT + j0 + u];      // 0 for a key that the query does not see
+#pragma unroll
+              for (int dd = 0; dd < MAXD; ++dd) acc[g][dd] = fmaf(p, vr[u][dd], acc[g][dd]);
+            }
       }
     }
     // join the four warps
