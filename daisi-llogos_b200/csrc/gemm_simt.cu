@@ -354,11 +354,13 @@ int launch_tile(const float* x, const float* w, float* out, int n, int o, int k,
 // of eight more (42 us at 64 x 2,048 x 2,048).  Of the twelve forms, timed at 36 to 600 rows of a 1B model's four matrices, it takes the
 // fastest or one within 15 % of it.
 struct TileForm { int rows, ranks; };
+constexpr int MAX_ROW_TILES = 65535;
 TileForm tile_form(int n, int o, int k, long long sms) {
   const int steps = (k + TK - 1) / TK;
   TileForm best{64, 1};
   double best_cost = 0;
   for (int rows = 64; rows >= 40; rows -= 8) {
+    if ((n + rows - 1) / rows > MAX_ROW_TILES) break;    // a grid's y: lower tiles would be more than it takes
     const long long tiles = (long long)((n + rows - 1) / rows) * ((o + TF - 1) / TF);
     for (int s = 1; s <= 4; s *= 2) {
       if (s > 1 && steps < 2 * s) break;
@@ -394,7 +396,7 @@ LLG_API int llg_gemm_simt(const void* x, int x_dtype, const void* w, int w_dtype
   LLG_REQUIRE(n >= 0 && o > 0 && k > 0, "gemm_simt: bad sizes n=%d o=%d k=%d", n, o, k);
   if (n == 0) return 0;
   dim3 grid((o + BN - 1) / BN, (n + BM - 1) / BM);
-  LLG_REQUIRE(grid.y <= 65535, "gemm_simt: %d rows need more than 65535 row blocks", n);
+  LLG_REQUIRE(grid.y <= MAX_ROW_TILES, "gemm_simt: %d rows need more than 65535 row blocks", n);
   const RowScale rs = scale ? *scale : RowScale{nullptr, 0, 0.f, 0.f};
   if (x_dtype == LLG_F32 && w_dtype == LLG_F32 && out_dtype == LLG_F32 && k % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15u) == 0) {
     const float *xf = (const float*)x, *wf = (const float*)w;
@@ -431,7 +433,7 @@ LLG_API int llg_gemm_simt_tile(const float* x, const float* w, float* out, int n
                                cudaStream_t stream) {
   LLG_REQUIRE(n > 0 && o > 0 && k > 0 && k % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15u) == 0, "gemm_simt_tile: n=%d o=%d k=%d", n, o, k);
   LLG_REQUIRE((rows == 40 || rows == 48 || rows == 56 || rows == 64) && (ranks == 1 || ranks == 2 || ranks == 4) &&
-                  (ranks == 1 || (k + TK - 1) / TK >= 2 * ranks) && (n + rows - 1) / rows <= 65535,
+                  (ranks == 1 || (k + TK - 1) / TK >= 2 * ranks) && (n + rows - 1) / rows <= MAX_ROW_TILES,
               "gemm_simt_tile: tiles of %d rows, %d blocks", rows, ranks);
   return run_tile(x, w, out, n, o, k, TileForm{rows, ranks}, scale ? *scale : RowScale{nullptr, 0, 0.f, 0.f}, stream);
 }

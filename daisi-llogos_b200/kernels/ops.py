@@ -721,6 +721,12 @@ def gemm_simt_tile(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, rows: in
                                        _scale_ref(row_scale, n), _stream()))
 
 
+def gemm_simt_form(n: int, o: int, k: int, sms: int):
+    """``(rows, ranks)`` that ``gemm_simt`` takes for a float32 product in tiles on a GPU of ``sms`` multiprocessors (``gemm_simt_tile``)."""
+    form = _lib("gemm_simt").llg_gemm_simt_form(n, o, k, sms)
+    return form % 1000, form // 1000
+
+
 def gemm_tc_status() -> int:
     """Error code a tensor-core product recorded when a wait ran out (0 = none); synchronises."""
     lib = _lib("gemm_tc")

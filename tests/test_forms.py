@@ -1,0 +1,30 @@
+"""Which form of a kernel a size takes: rules that run on the host, asked through the libraries themselves."""
+import importlib
+import random
+
+import pytest
+
+SMS = 148
+
+
+@pytest.fixture(scope="module")
+def ops():
+    return importlib.import_module("daisi-llogos_b200.kernels.ops")
+
+
+@pytest.mark.parametrize("n,o,k", [(2621441, 128, 128), (2680889, 128, 128), (3343748, 100, 4), (3905846, 100, 128), (3987930, 128, 512),
+                                   (64 * 65535, 128, 128)])
+def test_float32_tiles_of_very_many_rows_fit_a_grid(ops, n, o, k):
+    """64 rows a tile always fit up to 64 x 65,535 rows, the most that a product takes; lower tiles do not."""
+    rows, _ = ops.gemm_simt_form(n, o, k, SMS)
+    assert -(-n // rows) <= 65535
+
+
+def test_float32_tiles_of_any_size(ops):
+    rng = random.Random(5)
+    for _ in range(20000):
+        n, o, k = (int(2 ** rng.uniform(low, high)) for low, high in ((5.1, 21.99), (0, 17), (0, 14)))
+        k = 4 * k
+        rows, ranks = ops.gemm_simt_form(n, o, k, rng.choice((1, 16, 132, SMS)))
+        assert rows in (40, 48, 56, 64) and ranks in (1, 2, 4) and -(-n // rows) <= 65535
+        assert ranks == 1 or -(-k // 32) >= 2 * ranks           # every block of a tile has two steps or more, but for the last one's rest
