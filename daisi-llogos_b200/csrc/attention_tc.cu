@@ -401,7 +401,8 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  // (a cluster's blocks come together: a block of a later kernel must not take tensor memory ahead of one of theirs and then wait for it)
+  // (a cluster's blocks come together: a block of a later kernel must not take tensor memory ahead of one of theirs and then wait for it; nor
+  // may another cluster's block, see block_smem)
   if (FEW) pdl_launch_dependents();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base_slot;
@@ -1023,15 +1024,25 @@ FewForm few_form(const PrefillArgs& a, int sms) {
   return best;
 }
 
+// Shared memory of a block: queries, keys and values.  The blocks of a cluster wait for one another while each holds all of its multiprocessor's
+// tensor memory, so no two such blocks may share a multiprocessor (each could wait for ever for what the other's cluster holds, and
+// tcgen05.alloc and the cluster's barrier have no limit): they ask for more than half of its 228 KB.  (The pair products, the other kernel
+// whose blocks wait for one another with tensor memory in hand, take more than half too.)
+constexpr int ALONE_SMEM = 120 * 1024;
+constexpr int block_smem(int hd, int q_tiles, int parts) {
+  const int tiles = hd / 64 * 128 * (q_tiles * BQ + (KST + VST) * TK);
+  return parts > 1 && tiles < ALONE_SMEM ? ALONE_SMEM : tiles;
+}
+
 template <int HD, bool MAPS, bool FEW>
 int launch(const PrefillArgs& a, FewForm form, cudaStream_t stream) {
-  constexpr int KVB = (HD / 64) * TK * 128;
-  constexpr int smem = (MAPS || FEW ? 1 : GROUPS) * (HD / 64) * BQ * 128 + (KST + VST) * KVB;
-  static_assert(!FEW || BQ * HD * 4 <= smem, "a block's accumulators take the place of its queries, keys and values");
+  constexpr int Q_TILES = MAPS || FEW ? 1 : GROUPS, MOST_SMEM = block_smem(HD, Q_TILES, FEW ? MAX_PARTS : 1);
+  static_assert(!FEW || BQ * HD * 4 <= block_smem(HD, Q_TILES, 1), "a block's accumulators take the place of its queries, keys and values");
+  const int smem = block_smem(HD, Q_TILES, form.parts);
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<HD, MAPS, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return llg_fail("attn_prefill_tc: shared memory %d: %s", smem, cudaGetErrorString(e));
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<HD, MAPS, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST_SMEM);
+    if (e != cudaSuccess) return llg_fail("attn_prefill_tc: shared memory %d: %s", MOST_SMEM, cudaGetErrorString(e));
     configured = true;
   }
   CUtensorMap mkp, mvp, mkn, mvn;
@@ -1071,6 +1082,9 @@ LLG_API int llg_attn_tc_supported(int hd) { return hd == 64 || hd == 128; }
 // Blocks that share a tile's keys for these sizes (n_tiles, nh, nkv, window, chunked and host_tiles of `args`) on a GPU of `sms` multiprocessors;
 // 0 where the step takes the instance for long prompts.
 LLG_API int llg_attn_prefill_parts(const PrefillArgs* args, int sms) { return few_form(*args, sms).parts; }
+
+// Bytes of shared memory that such a block asks for.
+LLG_API int llg_attn_prefill_few_smem(int hd, int parts) { return block_smem(hd, 1, parts); }
 
 LLG_API int llg_attn_prefill_tc(const PrefillArgs* args, cudaStream_t stream) {
   const PrefillArgs& a = *args;

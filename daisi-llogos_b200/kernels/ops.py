@@ -471,6 +471,7 @@ def _load_lib(name: str):
         lib.llg_attn_tc_supported.argtypes = [c_int]
         lib.llg_attn_prefill_tc.argtypes = [POINTER(_PrefillArgs), c_void_p]
         lib.llg_attn_prefill_parts.argtypes = [POINTER(_PrefillArgs), c_int]
+        lib.llg_attn_prefill_few_smem.argtypes = [c_int, c_int]
         lib.llg_attn_tc_status.restype = c_int
     elif name == "attention_decode_tma":
         lib.llg_attn_decode_tma_supported.argtypes = [c_int, c_int, c_int, c_int]

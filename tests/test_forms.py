@@ -28,3 +28,12 @@ def test_float32_tiles_of_any_size(ops):
         rows, ranks = ops.gemm_simt_form(n, o, k, rng.choice((1, 16, 132, SMS)))
         assert rows in (40, 48, 56, 64) and ranks in (1, 2, 4) and -(-n // rows) <= 65535
         assert ranks == 1 or -(-k // 32) >= 2 * ranks           # every block of a tile has two steps or more, but for the last one's rest
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("parts", [2, 4, 8])
+def test_blocks_that_share_a_tiles_keys_have_a_multiprocessor_each(ops, hd, parts):
+    """Blocks of a cluster wait for one another with all of a multiprocessor's tensor memory in hand: two must not fit on one (228 KB of
+    shared memory, 1 KB of it the system's for every block; at most 227 KB for a block)."""
+    need = ops._lib("attention_tc").llg_attn_prefill_few_smem(hd, parts)
+    assert 2 * (need + 1024) > 228 * 1024 and need <= 227 * 1024
