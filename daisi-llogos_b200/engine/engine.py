@@ -14,6 +14,7 @@ the cache.
 """
 from __future__ import annotations
 
+from types import SimpleNamespace
 from typing import Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -124,6 +125,8 @@ class Engine:
         if self.device.type == "cuda":
             from .runner import BlockRunner
             self._runner = BlockRunner.build(model, self.cache)
+            if self._runner is not None and self.cache.max_seq_len > 0:
+                self._load_decode_kernels()
         self.vocab = model.spec.vocab_size
         self.use_graphs = use_graphs and self.device.type == "cuda"
         self._staging = _Staging(self.device)
@@ -131,6 +134,29 @@ class Engine:
         self._workspace = Workspace(self.device)
         self._decode: Dict[Tuple[int, int], _DecodeState] = {}     # (batch size, length bound) -> buffers and graph
         self.graph_kernels = 0      # kernels inside CUDA graphs replayed by step(), for reporting
+
+    def _load_decode_kernels(self) -> None:
+        """A decode step of two layers on the padding slot.  The driver loads a kernel when it is first launched, behind the kernels loaded
+        before it, and a step of some hundred short kernels feels where they lie: loaded among a prompt's, one sequence of a 1B model took 805
+        to 820 us a step, by what else the process had run and how large a prompt kernel's code was (the decode kernels byte for byte the
+        same); loaded together 800 to 806.  Only where every part is the library's own: nobody else's code runs before its first step."""
+        model = self.model
+        own = __package__.rpartition(".")[0] + ".parts."
+        if not all(type(p).__module__.startswith(own) for p in (model.embedding, model.final_norm, model.head, *model.encodings.values())):
+            return
+        st = _DecodeState(1, self.device)
+        m = st.meta
+        m.copy_(torch.tensor([0, 0, 0, self.cache.pad_slot, 0, 1, 0], dtype=torch.int32))       # laid out as in _decode_step
+        ctx = StepContext(n_tokens=1, n_seqs=1, decode=True, counts=[1], max_count=1, token_ids=m[0:1], positions=m[1:2],
+                          seq_of_token=m[2:3], slots=m[3:4], cu_tokens=m[4:6], len_before=m[6:7], dtype=self.dtype,
+                          device=self.device, ops=self.ops, workspace=st.workspace,
+                          max_len_after=min(self.cache.max_seq_len, length_bucket(1)))
+        layers = SimpleNamespace(run=lambda c, residual: self._runner.run(c, residual, layers=2))
+        try:
+            with torch.cuda.device(self.device):
+                model.forward(ctx, self.cache, st.rows, layers)
+        except RuntimeError:
+            pass                                # a size that the kernels refuse: the step that meets it says so
 
     # ---- sequences -----------------------------------------------------------------------
     def open(self) -> int:

@@ -208,8 +208,8 @@ class BlockRunner:
         return cls(model, cache, layers, keep, dict(geom, fusable_rotation=fusable))
 
     # ---- one step ----------------------------------------------------------------------------
-    def run(self, ctx, residual: torch.Tensor) -> Branch:
-        """Runs every layer on the step's tokens; returns the last block's output, still to be added."""
+    def run(self, ctx, residual: torch.Tensor, layers: Optional[int] = None) -> Branch:
+        """Runs every layer (or the first ``layers``) on the step's tokens; returns the last block's output, still to be added."""
         g, s, dtype = self.g, self.step, self.model.dtype
         n, hidden, nh, nkv, hd, inter = ctx.n_tokens, g["hidden"], g["nh"], g["nkv"], g["hd"], g["inter"]
         qkv_dim, q_dim = (nh + 2 * nkv) * hd, nh * hd
@@ -279,7 +279,7 @@ class BlockRunner:
             _ensure(need)
             self._ensured.add(key)
         s.stream = ops._stream()
-        rc = self.lib.llg_runner_run(self.table, self.n_layers, byref(s), None, 0, byref(self._out_parts), byref(self._launches))
+        rc = self.lib.llg_runner_run(self.table, self.n_layers if layers is None else min(layers, self.n_layers), byref(s), None, 0, byref(self._out_parts), byref(self._launches))
         ops._launches += self._launches.value
         if rc != 0:
             raise ops.KernelError(self.lib.llg_last_error().decode("utf-8", "replace"))
