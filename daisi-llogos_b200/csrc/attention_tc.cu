@@ -996,6 +996,10 @@ FewForm few_form(const PrefillArgs& a, int sms) {
   const int per_kv = a.nh / a.nkv;
   FewForm best{0, 0};
   if (!a.host_tiles || (long long)a.nh * a.n_tiles > 8LL * sms) return best;
+  // the grid goes by the sizes on the host, the kernel's rows by the device's: sizes that are not the step's must not leave rows out
+  long long step_rows = 0;
+  for (int t = 0; t < a.n_tiles; ++t) step_rows += a.host_tiles[2 * t + 1];
+  if (step_rows != a.n_tokens) return best;
   float best_us = 0.f;
   int most = 0;
   for (int parts = 0; parts <= MAX_PARTS; parts = parts ? 2 * parts : 1) {
@@ -1079,7 +1083,7 @@ int launch(const PrefillArgs& a, FewForm form, cudaStream_t stream) {
 // 1 when this kernel takes the head size (bfloat16 only): 64 or 128.
 LLG_API int llg_attn_tc_supported(int hd) { return hd == 64 || hd == 128; }
 
-// Blocks that share a tile's keys for these sizes (n_tiles, nh, nkv, window, chunked and host_tiles of `args`) on a GPU of `sms` multiprocessors;
+// Blocks that share a tile's keys for these sizes (n_tiles, n_tokens, nh, nkv, window, chunked and host_tiles of `args`) on a GPU of `sms` multiprocessors;
 // 0 where the step takes the instance for long prompts.
 LLG_API int llg_attn_prefill_parts(const PrefillArgs* args, int sms) { return few_form(*args, sms).parts; }
 

@@ -302,3 +302,26 @@ def test_truncate_and_continue(llogos, setup, name):
         eng.truncate(slot, 100)
     eng.close(slot)
     eng.cache.audit()
+
+
+@pytest.mark.parametrize("tq", [16, 64, 256])
+@pytest.mark.parametrize("before,counts", [([0], [1]), ([70, 0, 5000, 300, 0], [83, 257, 1, 512, 16]), ([3, 3, 3], [16, 64, 256])])
+def test_query_tiles_and_their_sizes_on_the_host(before, counts, tq):
+    """Every query in one tile, the tiles that see the most keys first, and beside them, row by row, how many keys a tile's last query sees and
+    how many queries it has: a launch's grid goes by these."""
+    from importlib import import_module
+    C = import_module("daisi-llogos_b200.engine.context")
+    none = torch.zeros(0, dtype=torch.int32)
+    ctx = C.StepContext(n_tokens=sum(counts), n_seqs=len(counts), decode=False, counts=counts, max_count=max(counts), token_ids=none,
+                        positions=none, seq_of_token=none, slots=none, cu_tokens=none, len_before=none, device=torch.device("cpu"),
+                        workspace=C.Workspace(torch.device("cpu")), len_before_host=before)
+    tiles = ctx.query_tiles(tq)
+    seen = [[] for _ in counts]
+    assert tiles.host_sizes.dtype == "int32" and tiles.host_sizes.shape == tuple(tiles.shape)
+    for (b, q0), (keys, queries) in zip(tiles.tolist(), tiles.host_sizes.tolist()):
+        places = range(q0, min(q0 + tq, counts[b]))
+        assert queries == len(places) and keys == before[b] + places[-1] + 1
+        seen[b] += places
+    assert [sorted(s) for s in seen] == [list(range(c)) for c in counts]
+    keys = tiles.host_sizes[:, 0].tolist()
+    assert keys == sorted(keys, reverse=True) and ctx.query_tiles(tq) is tiles

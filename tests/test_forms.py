@@ -2,6 +2,7 @@
 import importlib
 import random
 
+import numpy as np
 import pytest
 
 SMS = 148
@@ -37,3 +38,12 @@ def test_blocks_that_share_a_tiles_keys_have_a_multiprocessor_each(ops, hd, part
     shared memory, 1 KB of it the system's for every block; at most 227 KB for a block)."""
     need = ops._lib("attention_tc").llg_attn_prefill_few_smem(hd, parts)
     assert 2 * (need + 1024) > 228 * 1024 and need <= 227 * 1024
+
+
+def test_prompt_attention_goes_by_host_sizes_only_where_they_are_the_steps(ops):
+    """The form for few long sequences has a grid made for the sizes on the host: with sizes that understate the step's queries rows would
+    stay unwritten, so it is not taken (0: the other instance, which asks the device alone)."""
+    sizes = np.asarray([(1083, 83), (900, 83)], dtype=np.int32)
+    assert ops.attn_prefill_parts(sizes, 16, 4, 0, SMS, n_tokens=166) == ops.attn_prefill_parts(sizes, 16, 4, 0, SMS) == 4
+    for n_tokens in (165, 167, 240):
+        assert ops.attn_prefill_parts(sizes, 16, 4, 0, SMS, n_tokens=n_tokens) == 0
