@@ -1940,12 +1940,13 @@ def tile_sizes_ptr(tiles: torch.Tensor) -> Optional[int]:
     return None if sizes is None else sizes.ctypes.data
 
 
-def attn_prefill_parts(tile_sizes, n_heads: int, n_kv_heads: int, window: int, sms: int, n_tokens: Optional[int] = None) -> int:
+def attn_prefill_parts(tile_sizes, n_heads: int, n_kv_heads: int, window: int, sms: int, n_tokens: Optional[int] = None,
+                       chunked: bool = False) -> int:
     """Blocks that the tcgen05 prompt attention lets share a tile's keys on a GPU of ``sms`` multiprocessors (0: the instance for long
     prompts); ``tile_sizes``: int32 ``[n_tiles, 2]`` on the host (``PrefillArgs.host_tiles``); ``n_tokens``: the step's (default: theirs)."""
     a = _PrefillArgs()
     a.n_tokens = int(tile_sizes[:, 1].sum()) if n_tokens is None else n_tokens
-    a.n_tiles, a.nh, a.nkv, a.window = len(tile_sizes), n_heads, n_kv_heads, int(window)
+    a.n_tiles, a.nh, a.nkv, a.window, a.chunked = len(tile_sizes), n_heads, n_kv_heads, int(window), int(chunked)
     a.host_tiles = tile_sizes.ctypes.data
     return _lib("attention_tc").llg_attn_prefill_parts(byref(a), sms)
 

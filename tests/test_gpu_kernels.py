@@ -113,12 +113,13 @@ def test_add_rmsnorm_of_many_rows(ops, dtype, hidden):
         check(out, P.rms_norm(total, w, eps), dtype, "normed")
 
 
-# float32 rows of 16 bytes: the weight stream up to 32 rows (chunks of 1, 2, 4 or 8 rows, the last one short; a warp's k with and
-# without a remainder), the tiles of 64 x 128 above, whose k one block, two (100 x 3,170: 50 tiles of eight steps) or four share, the
-# last of four with less than the others or with nothing (65 x 300: nine steps, three a block)
-@pytest.mark.parametrize("n,o,k", [(1, 5, 4), (2, 33, 132), (3, 64, 1000), (7, 301, 2048), (9, 20, 516), (16, 4100, 260), (17, 129, 4),
-                                   (25, 301, 2052), (32, 4100, 260), (33, 200, 132), (63, 129, 1036), (100, 3170, 252), (65, 300, 288),
-                                   (64, 128, 1036), (65, 257, 4104), (200, 300, 2052), (130, 24000, 64)])
+# float32 rows of 16 bytes: the weight stream up to 32 rows (chunks of 1, 2, 4 or 8 rows of which 3, 4, 5 or 6 may be there, the last chunk
+# short; a warp's k with and without a remainder), the tiles above, in the forms that test_forms.py lists for these sizes: 40 or 48 rows,
+# one block a tile or four, of which the last has less k than the others or none (65 x 300: nine steps, three a block).  Tiles of 56 and 64
+# rows and pairs of blocks: test_gemm_simt_tiles
+@pytest.mark.parametrize("n,o,k", [(1, 5, 4), (2, 33, 132), (3, 64, 1000), (4, 301, 1036), (5, 33, 132), (5, 301, 2052), (6, 129, 1000), (7, 301, 2048),
+                                   (9, 20, 516), (16, 4100, 260), (17, 129, 4), (25, 301, 2052), (32, 4100, 260), (33, 200, 132), (63, 129, 1036),
+                                   (100, 3170, 252), (65, 300, 288), (64, 128, 1036), (65, 257, 4104), (200, 300, 2052), (130, 24000, 64)])
 def test_gemm_simt_float32_rows(ops, n, o, k):
     x, w = rnd((n, k), 5), rnd((o, k), 6, torch.float32, 1.0 / math.sqrt(k))
     ss = rnd((n, 3), 7).abs() + 0.5
@@ -531,6 +532,51 @@ def test_attn_prefill_of_few_long_sequences(ops, hd, before, counts, nh, nkv, wi
             share = torch.sigmoid(_log_sum(qq, ks[b], scale, window)[before[b]:] - sink.double())
             ref = ref * (share * gate[int(cu[b]):int(cu[b + 1])].double())[:, :, None]
         check(out[int(cu[b]):int(cu[b + 1])], ref.reshape(counts[b], -1), dtype, ("sequence", b))
+
+
+@pytest.mark.parametrize("before,count,nh,nkv,parts", [(2990, 5, 8, 2, 8), (1900, 200, 8, 2, 4), (640, 300, 16, 2, 1)],
+                         ids=["eight parts", "across a chunk's end", "whole keys"])
+@pytest.mark.parametrize("shape", ["chunks", "slow", "steps"])
+@pytest.mark.parametrize("hd", [64, 128])
+def test_attn_prefill_of_few_long_sequences_chunks_and_rising_scores(ops, hd, shape, before, count, nh, nkv, parts):
+    """The form for few long sequences with chunks of 1,024 positions (rows of one block in two of them), and with scores that rise along the
+    keys: slowly, or by twenty units at three places, so that rows of some blocks of a cluster are rescaled in the middle and those of others not."""
+    dtype, total = torch.bfloat16, before + count
+    chunk = 1024 if shape == "chunks" else 0
+    g = torch.Generator().manual_seed(91 + hd)
+    u = torch.randn(hd, generator=g)
+    u = u / u.norm()
+    pos = torch.arange(total, dtype=torch.float32)
+    edges = 14.0 * (pos % 1024 == 1023) + 10.0 * (pos % 1024 == 0)       # the key that the next chunk must not see, the first that it must
+    rise = {"chunks": edges, "slow": pos * (40.0 / total), "steps": 20.0 * sum((pos >= f * total).float() for f in (0.2, 0.55, 0.9))}[shape]
+    k = (0.3 * torch.randn(total, nkv, hd, generator=g) + rise[:, None, None] * u).to(dtype)
+    v = torch.randn(total, nkv, hd, generator=g).to(dtype)
+    q = (0.3 * torch.randn(count, nh, hd, generator=g) + u).to(dtype)
+    pages = (total + 63) // 64
+    ring = chunk // 64 + 1 if chunk else pages
+    table = torch.zeros(3, ring, dtype=torch.int32)
+    table[1] = torch.randperm(ring, generator=g).int()
+    kp, vp = (torch.zeros(ring, nkv, 64, hd, dtype=dtype) for _ in range(2))
+    for p_ in range(max(0, before - (ring - 1) * 64), before):
+        at = int(table[1, p_ // 64 % ring])
+        kp[at, :, p_ % 64], vp[at, :, p_ % 64] = k[p_], v[p_]
+    form = ops.AttentionForm(chunked=True) if chunk else ops.PLAIN_ATTENTION
+    tq = ops.prefill_tile_queries(dtype, hd, form)
+    starts = list(range(0, count, tq))[::-1]
+    d = lambda t: t.to(DEV)
+    tiles = torch.tensor([(0, q0) for q0 in starts], dtype=torch.int32, device=DEV)
+    tiles.host_sizes = np.asarray([(before + min(count, q0 + tq), min(count - q0, tq)) for q0 in starts], dtype=np.int32)
+    assert ops.attn_prefill_parts(tiles.host_sizes, nh, nkv, chunk, 148, chunked=bool(chunk)) == parts
+    out = torch.full((count, nh * hd), float("nan"), dtype=dtype, device=DEV)
+    ops.attn_prefill(d(q), d(k[before:].contiguous()), d(v[before:].contiguous()), d(kp), d(vp), d(table), ring, tiles,
+                     d(torch.tensor([0, count], dtype=torch.int32)), d(torch.tensor([before], dtype=torch.int32)),
+                     d(torch.tensor([1], dtype=torch.int32)), out, scale=1.0, window=chunk, tile_queries=tq, form=form)
+    assert ops.attn_tc_status() == 0
+    at, keys = before + torch.arange(count)[:, None], torch.arange(total)[None, :]
+    hidden = (keys > at) | (keys < (at // chunk * chunk if chunk else 0))
+    s = torch.einsum("ihd,jhd->hij", q.double(), k.double().repeat_interleave(nh // nkv, 1)).masked_fill(hidden, -math.inf)
+    ref = torch.einsum("hij,jhd->ihd", s.softmax(-1), v.double().repeat_interleave(nh // nkv, 1))
+    check(out, ref.reshape(count, -1), dtype, shape)
 
 
 @pytest.mark.parametrize("tc", [True, False], ids=["tcgen05", "mma"])
