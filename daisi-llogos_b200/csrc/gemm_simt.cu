@@ -92,10 +92,11 @@ __device__ __forceinline__ float both(pair_t v) { return __uint_as_float((unsign
 // feature group share k.  Bound by the weight stream: a float4 of weights is used for NR products of four, and the rows'
 // float4s come from the first-level cache once per F features, so F x NR = 32 keeps the CUDA cores and that cache below
 // half of what the memory's rate asks of them.  The weights of the first group do not wait for the kernel before.
-// 16,384 x 2,048: 23.5 us for one row (5.7 TB/s), 28.4 for three (4.7), 36.5 for eight (3.7; there the cores bound it); 128,256 x
-// 2,048 at three rows 169 us (6.2 TB/s).  gemm_tn_kernel, which took these before, pays for 64 rows: 618 us on average over a 1B
+// 16,384 x 2,048: 23.3 us for one row (5.8 TB/s), 26.7 for three (5.0), 35.9 for eight (3.7; there the cores bound it); 128,256 x
+// 2,048 at three rows 163 us (6.4 TB/s).  gemm_tn_kernel, which took these before, pays for 64 rows: 618 us on average over a 1B
 // model's products.
-// LIVE of the NR rows are there (the rest of the sums stay zero).
+// LIVE of the NR rows are there (the rest of the sums stay zero): three rows 27.9 us with the fourth's multiply-adds, 26.7 without, six 35.9
+// with those of eight and 33.1.
 template <int NR, int F, int LIVE>
 __global__ void __launch_bounds__(256, 2) gemv_rows_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                         float* __restrict__ out, int n, int o, int k, int wk, RowScale scale) {
@@ -177,9 +178,9 @@ __global__ void __launch_bounds__(256, 2) gemv_rows_kernel(const float* __restri
 }
 
 // More rows (a prompt step): tiles of up to 64 rows x 128 features, 256 threads with up to 8 x 4 sums each.  Both operands arrive by
-// cp.async as they lie in memory, 32 k of a row at a time, in a ring of three stages: a stage is 24 KB, so that one block a
+// cp.async as they lie in memory, 32 k of a row at a time, in a ring of three stages: a stage is 24 to 27 KB, so that one block a
 // multiprocessor already has the bytes in flight that the memory's latency asks for (with the next stage in registers and
-// half as much a step a block waited 2 us a step: 100 x 2,048 x 2,048 81.5 us before, 38.6 now).  Rows are padded to 36 floats: 16-byte
+// half as much a step a block waited 2 us a step: 100 x 2,048 x 2,048 81.5 us before, 38.6 in tiles of 64 rows, 34.3 in tiles of 56).  Rows are padded to 36 floats: 16-byte
 // reads of consecutive rows at one k fall into different banks.  A thread takes four k at a time, 12 reads for 128
 // multiply-adds.  From 300 rows on the multiply-add pipes (two thirds busy) and the 16-byte shared reads bound it: 38 TFLOP/s.  Where a shape has few tiles, the blocks of a cluster
 // share the tile's k and add their sums through distributed shared memory, in the order of the ranks.
@@ -349,10 +350,12 @@ int launch_tile(const float* x, const float* w, float* out, int n, int o, int k,
 }
 
 // Rows of a tile (40, 48, 56 or 64) and the blocks that share a tile's k: the multiprocessor with the most blocks has their steps to do, each as
-// long as the tile has rows (two blocks a multiprocessor take as long as one with twice the steps, to 5 %), and every block a fixed
-// cost.  Clusters of four leave some multiprocessors out (288 blocks, 100 x 3,072 x 2,048: 68 us, where 144 in clusters of two take 51), clusters
-// of eight more (42 us at 64 x 2,048 x 2,048).  Of the twelve forms, timed at 36 to 600 rows of a 1B model's four matrices, it takes the
-// fastest or one within 15 % of it.
+// long as the tile has rows and four more, for its features (two blocks a multiprocessor take as long as one with twice the steps, to 5 %),
+// and every block a fixed cost.  Clusters of four leave some multiprocessors out (288 blocks, 100 x 3,072 x 2,048: 68 us, where 144 in
+// clusters of two take 51), clusters of eight more (42 us at 64 x 2,048 x 2,048).  Of the twelve forms, timed at 309 sizes (33 to 2,048
+// rows, twelve matrices from 1,000 x 1,024 to 128,256 x 2,048), it takes 1.1 % more than the fastest on average and 21 % at worst, and nowhere
+// more than tiles of 64 rows alone, which take 25 % more on average; with steps as long as the rows alone it took lower tiles where those of 64
+// were 2 to 8 % faster (300 x 4,096 x 4,096: 339 us in tiles of 40, 319 in tiles of 64, four blocks each).
 struct TileForm { int rows, ranks; };
 constexpr int MAX_ROW_TILES = 65535;
 TileForm tile_form(int n, int o, int k, long long sms) {
@@ -365,7 +368,7 @@ TileForm tile_form(int n, int o, int k, long long sms) {
     for (int s = 1; s <= 4; s *= 2) {
       if (s > 1 && steps < 2 * s) break;
       const long long places = s == 4 ? sms - sms / 14 : sms, per_sm = (tiles * s + places - 1) / places;
-      const double cost = rows / 64.0 * (per_sm == 1 ? 1.0 : 0.95 * per_sm) * ((steps + s - 1) / s) + 3.0 + (s > 1 ? 2.0 : 0.0);
+      const double cost = (rows + 4) / 68.0 * (per_sm == 1 ? 1.0 : 0.95 * per_sm) * ((steps + s - 1) / s) + 3.0 + (s > 1 ? 2.0 : 0.0);
       if (best_cost == 0 || cost < best_cost * 0.999) {
         best_cost = cost;
         best = {rows, s};
@@ -384,8 +387,9 @@ int run_tile(const float* x, const float* w, float* out, int n, int o, int k, Ti
   }
 }
 
-// Rows up to which the weight stream is taken: at 32 rows of 2,048 x 2,048 it takes 21 us and the tiles 38, at 40 rows 27 and 38, but
-// at 2,048 x 16,384 the tiles are even from 40 on (142 us both).
+// Rows up to which the weight stream is taken: its time rises with every eight rows, that of tiles of 40 does not.  At 24 and 32 rows 80 and
+// 94 us at 16,384 x 2,048, where the tiles take 95; 43 and 55 (96) at 2,048 x 8,192; 18.5 and 23 (27) at 3,072 x 2,048; 13.7 and 17.6 (26.8)
+// at 2,048 x 2,048.  Even at 32 for the widest, which is the most of a model's time.
 constexpr int GEMV_ROWS_MAX = 32;
 
 }  // namespace
