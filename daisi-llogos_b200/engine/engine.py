@@ -93,6 +93,9 @@ class _DecodeState:
         self.eager_runs = 0
 
 
+_DECODE_KERNELS_LOADED = set()       # (device, dtype, sizes) of models; see Engine._load_decode_kernels
+
+
 class Engine:
     """A model, its cache and the step function.
 
@@ -139,8 +142,13 @@ class Engine:
         """A decode step of two layers on the padding slot.  The driver loads a kernel when it is first launched, behind the kernels loaded
         before it, and a step of some hundred short kernels feels where they lie: loaded among a prompt's, one sequence of a 1B model took 805
         to 820 us a step, by what else the process had run and how large a prompt kernel's code was (the decode kernels byte for byte the
-        same); loaded together 800 to 806.  Only where every part is the library's own: nobody else's code runs before its first step."""
+        same); loaded together 800 to 806.  Once a process for a device and a model's sizes (0.4 ms).  Only where every part is the library's
+        own: nobody else's code runs before its first step."""
         model = self.model
+        sizes = (torch.cuda.current_device() if self.device.index is None else self.device.index, self.dtype, model.spec.vocab_size,
+                 *sorted(self._runner.g.items()))
+        if sizes in _DECODE_KERNELS_LOADED:
+            return
         own = __package__.rpartition(".")[0] + ".parts."
         if not all(type(p).__module__.startswith(own) for p in (model.embedding, model.final_norm, model.head, *model.encodings.values())):
             return
@@ -155,6 +163,7 @@ class Engine:
         try:
             with torch.cuda.device(self.device):
                 model.forward(ctx, self.cache, st.rows, layers)
+            _DECODE_KERNELS_LOADED.add(sizes)
         except RuntimeError:
             pass                                # a size that the kernels refuse: the step that meets it says so
 
