@@ -25,11 +25,12 @@
 // 2^14, warp by warp and only when some row of the warp needs it; only then are the tile's maxima worked out.
 //
 // A key tile's time is a softmax warp's chain of it, about 2,000 cycles: 64 exponentials a row (700 cycles with the other
-// group's beside them 980; the special-function unit is busy 43 % of the time, the tensor cores 42), the way in and out of
+// group's beside them 980; the special-function unit and the tensor cores are each busy 44 % of the time), the way in and out of
 // tensor memory, and 100 to 200 cycles for each barrier that is passed.  So a tile has no maximum and no wait that it
-// can do without.  8,192 tokens x 32 heads of 128: 634 us with a lane for both groups' products, a maximum and a wait for the
-// accumulator in every tile, 584 now; 2,048 tokens 81 and 69; four prompts of 1,100 tokens, heads of 64, 128 and 100; 300 tokens 25 and 18.
-// (Taking turns with the exponentials, group by group: 650 us at 8,192 tokens, 82 at 2,048.)
+// can do without.  8,192 tokens x 32 heads of 128, ten launches after a pause: 646 us with a lane for both groups' products, a maximum and a
+// wait for the accumulator in every tile, 597 now (launch after launch under the power cap 648 at 1,920 MHz and 615 at 1,860); 2,048 tokens
+// launch after launch 80 and 67, heads of 64 72 and 60; four prompts of 1,100 tokens, heads of 64, 128 and 98.
+// (Taking turns with the exponentials, group by group: 650 us at 8,192 tokens where this form took 584, 82 at 2,048.)
 //
 // Tiles of at most 128 queries (short prompts, the next turn of a chat) leave the second group without queries.  It then takes
 // part in one of two ways, which every block finds from its own tile.  SPLIT (two key tiles or more): the groups share the keys,
@@ -43,7 +44,7 @@
 // key/value head see the same keys, so their queries are rows of one list, a head's behind the last head's, that its blocks take 128 at a
 // time, all of them SPLIT; and the keys of a tile may go to the blocks of a cluster, a consecutive run each, which leave their
 // accumulators in shared memory and join them there, each block some of the columns, in the blocks' order.  few_form chooses by the
-// step's lengths.
+// step's lengths, for the step as a whole: all its tiles have as many parts.
 //
 // With MAPS (differential attention) the two halves of a query and of a key are two maps over the same values: the block's
 // two groups are the two maps of ONE tile of 128 queries, whose scores are products over their half of the head; keys,
@@ -72,8 +73,9 @@ constexpr int TK = 64;       // keys per tile = one cache page
 constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;
 constexpr float LOG2E = 1.4426950408889634f;
 
-// 2^x by the special-function unit alone (float32, about 2 ulp, denormal results flushed to zero);
-// exp2f() adds range handling that the softmax does not need: its arguments are <= 0 or -inf.
+// 2^x by the special-function unit alone (float32, about 2 ulp, denormal results flushed to zero, +inf past the range);
+// exp2f() adds range handling that the softmax does not need: weights that are kept lie below 2^14, and a tile with an argument of any
+// size ahead of its maximum, or a weight that has run over, fails the bound on its sum and is worked out again.
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -585,9 +587,11 @@ __global__ void __launch_bounds__(384, 1) attn_prefill_tc_kernel(const __grid_co
     const float sc = a.scale * LOG2E;
     // A row's weights are 2^(x - M) with x = score * scale * log2 e and M a whole number that is raised (to the
     // tile's maximum, rounded up) only when a tile's weights add up to more than 2^14, so some weight is above 2^8: no weight
-    // exceeds 2^14 and the accumulator is rescaled rarely, by an exact power of two.  The common factor cancels in the final division,
-    // and rounding a weight to bfloat16 gives the same bits whatever M was: how the keys are cut into tiles or
-    // steps does not show in the rounded weights.
+    // exceeds 2^14 and the accumulator is rescaled rarely, by an exact power of two.  The common factor cancels in the final division.
+    // A weight rounded to bfloat16 has the same digits for any whole M but for the rounding of x - M itself (float32, at a magnitude that
+    // depends on M): now and then, where 2^(x - M) lies next to the middle of two bfloat16 numbers, it goes the other way.  So how the
+    // keys are cut into tiles or steps shows in a last bit of some weights and in no error: against 64 bits 2.289e-3 to 2.342e-3 at 2,048
+    // tokens and scores of standard deviation 0.3 to 8, to four digits the same under a rule that raised M by every tile's maximum.
     const float sum_bound = 16384.0f;
     const int qpos = FEW ? ti.lb + q_off_few + row_query(r) : pos0 + r;
     // positions of the warp's first and last row, for the tiles that need no mask (FEW: of the block's)
@@ -987,9 +991,13 @@ bool kv_map(const void* base, long long rows, int nkv, int hd, CUtensorMap* resu
 // multiprocessors, end soonest by the measured times below (us: a block, a key tile of a SPLIT block and of a PLAIN one, what parts add).  Parts only
 // where all clusters are resident at once: in two rounds of them a step takes longer than with whole keys (96 blocks of 1,399 to 2,813
 // keys: 39 us, in two parts 45; 16 of 810: 16 us, in four parts 13, in eight 25, as not quite sixteen clusters of eight fit).
-// Measured, heads of 128, 32 query and 8 key/value heads: 83 queries behind 4,000 keys 43 us in the other instance, 23 in four parts; 5 behind
-// 6,000 (40 heads) 58 and 18 in eight; 300 behind 6,000 119 and 69 whole, behind 1,000 39 and 25; two of 200 behind 3,000 and 2,000 73 and
-// 46; a prompt of 300 18 and 14, of 2,048 69 and 75; four prompts of 1,100 (heads of 64) 100 and 110.
+// Measured, 32 query and 8 key/value heads of 128 (of 64): 83 queries behind 4,000 keys 41 us (40) in the other instance, 21 (19) in four parts; 5
+// behind 6,000 (40 heads) 56 (54) and 16 (15) in eight; 300 behind 6,000 117 (111) and 65 (63) whole, behind 1,000 38 (35) and 24 (22); two
+// of 200 behind 3,000 and 2,000 67 (64) and 43 (40); a prompt of 300 17 (15) and 12 (11), five of 11 to 51 10.8 (9.8) and 10.1 (8.9).  Where
+// the rule stays with the other instance: a prompt of 2,048 67 us against 75, four of 1,100 (heads of 64) 98 against 110.  The times
+// of a block and of a tile are those of heads of 128; heads of 64 are 5 to 15 % faster in both instances, so the comparison stands for them.
+// Four turns of 83 queries behind 1,400 to 2,800 keys come out level by these times (33 us; 37 measured) and keep the other instance: with
+// one count of parts for the step the longest sequence's blocks are as many as the shortest's.
 struct FewForm { int parts, blocks; };
 constexpr float BLOCK_US = 7.0f, SPLIT_TILE_US = 0.57f, PLAIN_TILE_US = 1.15f, JOIN_US = 4.5f;
 FewForm few_form(const PrefillArgs& a, int sms) {
